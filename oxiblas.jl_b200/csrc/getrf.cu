@@ -127,11 +127,6 @@ static void panel_rl(LuRun<T> &R, i64 c0, i64 nc) {
     oxi_handle_s *h = R.h;
     const i64 cend = c0 + nc;
     LeafPanel pend;  // the previous step's U12, still in R.ubuf
-    // The move counter is zero at a panel's first column (k_rowmap_init), and
-    // each of these leaves zeroes it again at its end; a right half reached
-    // inside a recursive panel (tournament leaves on its left) starts from a
-    // counter those leaves left set.
-    if (c0 != R.pf) OXI_CUDA(cudaMemsetAsync(R.nmoves, 0, sizeof(int), h->stream));
     for (i64 c = c0; c < cend;) {
         const i64 mrows = R.m - c;
         if (mrows <= 0) break;
@@ -139,7 +134,6 @@ static void panel_rl(LuRun<T> &R, i64 c0, i64 nc) {
         if (lw == 0) throw CudaError{cudaErrorInvalidValue, "panel taller than the leaf capacity"};
         const i64 w = std::min<i64>(lw, cend - c);
         LeafPanel pn = leaf_panel(R, c, w);
-        pn.reset_nmoves = 1;
         pn.u_src = pend.u_src;
         pn.u_dst = pend.u_dst;
         pn.u_rows = pend.u_rows;
@@ -178,7 +172,7 @@ static void panel_leaf32(LuRun<T> &R, i64 c0, i64 nc, int w) {
         const i64 wc = std::min<i64>(w, c0 + nc - c);
         const i64 mrows = R.m - c;
         if (mrows <= 0) break;
-        OXI_CUDA(cudaMemsetAsync(R.nmoves, 0, sizeof(int), h->stream));
+        if (!R.map) OXI_CUDA(cudaMemsetAsync(R.nmoves, 0, sizeof(int), h->stream));
         maybe_stall_before_leaf(h, h->stream);
         if (R.map) {  // the leaf moves the panel's other columns itself
             launch_leaf<T>(R.W + c * R.ld + c, R.ld, mrows, (int)wc, c, R.ipiv, R.info, R.moves, R.nmoves, w,
@@ -225,7 +219,8 @@ static void panel_rec(LuRun<T> &R, i64 c0, i64 nc) {
         }
     }
     if (nc <= leafw) {
-        OXI_CUDA(cudaMemsetAsync(R.nmoves, 0, sizeof(int), h->stream));
+        // leaves that move the panel's other columns themselves use no move list
+        if (!R.map || ts) OXI_CUDA(cudaMemsetAsync(R.nmoves, 0, sizeof(int), h->stream));
         auto leaf = [&](LeafPanel pn) {
             maybe_stall_before_leaf(h, h->stream);
             if constexpr (sizeof(T) == 4) {
@@ -330,7 +325,7 @@ void getrf_rowmajor(oxi_handle_s *h, T *W, i64 ld, i64 m, i64 n, int64_t *d_ipiv
             if (compose) {
                 R.pf = f;
                 R.pl = l;
-                launch_rowmap_init(R.map, m - f, R.nmoves, listcnt, sA);
+                launch_rowmap_init(R.map, m - f, listcnt, sA);
                 panel_rec(R, f, l - f);
                 launch_rowmap_extract(R.map, m - f, list, listcnt, sA);
                 if (b_pending) {  // the previous trailing update reads L21 and writes the columns moved now

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <climits>
 #include <type_traits>
+#include "leaf.cuh"
 #include "oxi_internal.h"
 #include "tma_util.cuh"
 
@@ -77,78 +78,45 @@ template void launch_rm_to_cm<float, float>(const float *, i64, float *, i64, i6
 template void launch_rm_to_cm<float, double>(const float *, i64, double *, i64, i64, i64, cudaStream_t);
 
 // ---------------------------------------------------------------------------
-// Leaf LU: one thread-block cluster (1..16 CTAs of NT = 256 or 512 threads) holds the
-// m x W leaf in REGISTERS, R rows per thread (row position i lives in thread
-// g = i mod G, slot k = i / G, G = cluster threads).  Column by column, as the
-// leaf loop of _lu_panel! (src/lapack/factorizations.jl:116-139):
-//   pivot = first row of the largest |a_ij|, i >= j (_lu_pivot, :92-107);
-//   swap rows j and p over the leaf's W columns;
+// Leaf LU: one thread-block cluster (1..16 CTAs of NT threads) holds the m x W
+// leaf in REGISTERS, R rows per thread, with implicit pivoting: a row never
+// leaves its thread, it carries the position the interchanges have brought it
+// to and is stored there at the end.  Column by column, as the leaf loop of
+// _lu_panel! (src/lapack/factorizations.jl:116-139):
+//   pivot = first position of the largest |a_ij| among positions >= j (_lu_pivot, :92-107);
+//   positions j and p change places;
 //   zero pivot -> info (first one), skip the column;
-//   l_ij = a_ij / a_jj (a true division, as the reference);
+//   l_ij = a_ij / a_jj (correctly rounded, as the reference's division);
 //   a_ic = muladd(-l_ij, a_jc, a_ic) for c > j.
-// Per column each CTA reduces its candidate in registers/shared memory and
-// PUSHES it (|value|, position, the whole candidate row) into every CTA's
-// shared memory with st.async, one 16-byte store per thread, each completing
-// its bytes on the receiver's mbarrier; a CTA waits on its own barrier until
-// all candidates have landed and picks the same winner as every other CTA.
-// The CTA that owns position j also pushes row j, so the two swapped rows
-// never need a second exchange.  Slots are double-buffered by column parity,
-// which is what makes one exchange per column sufficient.  Each row carries
-// the index of the row it started as; at the end a position whose row changed
-// emits a (dst, src) move.  The net permutation reaches the other columns by
-// k_rowmoves, or, inside a composed panel, through the leaf itself after a
-// cluster barrier (one warp per moved row).
+// The columns go in groups of GW = 8.  A column step updates only the rest of
+// its group, so what a CTA publishes per column is its candidate's position
+// and live group values.  After the group its GW pivot rows publish their
+// multipliers and remaining columns once, every CTA solves the GW x GW unit
+// triangle for them, and each row takes the GW updates of its remaining columns
+// together.  Every element sees the same fused multiply-adds in the same order
+// as in the column-by-column form.
+//
+// Bound: latency of the column steps.  One step is a warp arg-max (one redux and
+// a ballot; ties take two more) with the winner lane's candidate into shared
+// memory, one CTA barrier, the arg-max over the warps and, across CTAs, one
+// exchange: a few warps push one 16-byte chunk each of the CTA's winner to every
+// CTA with st.async, completing on the receiver's mbarrier.  Slots are
+// double-buffered by column parity, which makes one exchange per column
+// sufficient: a slot is rewritten two columns later, after its receiver has
+// pushed the column in between, i.e. after it read the slot.  Measured forms that
+// are slower: rolled column loops (1.2-1.5 times a step), one warp reducing for
+// the others (two barriers; 1.15 times in FP64), plain stores polled by every
+// warp (1.15 times across CTAs).
+// Rows travel between global memory and the threads that own them through
+// per-warp shared memory, 128 contiguous bytes at a time: one row per lane, 16
+// bytes at a time, costs 32 cache lines an instruction.
 // ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
-// Warp arg-max for the pivot search with redux.sync: |v| >= 0 orders like its
-// bit pattern, so the warp maximum is an integer max (FP64: high word, then
-// low word), and the first row among equal maxima is an integer min of the
-// positions -- the reference's "largest |a|, first row on ties".  NaN maps to
-// the smallest key, as a NaN never wins the reference's strict '>' comparison.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t redux_max_u32(uint32_t v) {
-    uint32_t r;
-    asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(v));
-    return r;
-}
-__device__ __forceinline__ uint32_t redux_min_u32(uint32_t v) {
-    uint32_t r;
-    asm volatile("redux.sync.min.u32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(v));
-    return r;
-}
-__device__ __forceinline__ uint64_t pivot_key(float a) {
-    return (a == a) ? (uint64_t)__float_as_uint(fabsf(a)) : 0ull;
-}
-__device__ __forceinline__ uint64_t pivot_key(double a) {
-    return (a == a) ? (uint64_t)__double_as_longlong(fabs(a)) : 0ull;
-}
-// (key, pos) of the warp winner, identical in every lane; pos = INT_MAX when no lane has one.
-template <typename T>
-__device__ __forceinline__ void warp_argmax(uint64_t &key, int &pos) {
-    const uint32_t p = (uint32_t)pos;
-    if constexpr (sizeof(T) == 4) {
-        const uint32_t k = (uint32_t)key;
-        const uint32_t mk = redux_max_u32(p == (uint32_t)INT_MAX ? 0u : k);
-        const uint32_t mp = redux_min_u32(k == mk ? p : (uint32_t)INT_MAX);
-        key = mk;
-        pos = (int)mp;
-    } else {
-        const uint32_t hi = (uint32_t)(key >> 32), lo = (uint32_t)key;
-        const bool valid = p != (uint32_t)INT_MAX;
-        const uint32_t mh = redux_max_u32(valid ? hi : 0u);
-        const uint32_t ml = redux_max_u32(valid && hi == mh ? lo : 0u);
-        const uint32_t mp = redux_min_u32(hi == mh && lo == ml ? p : (uint32_t)INT_MAX);
-        key = ((uint64_t)mh << 32) | ml;
-        pos = (int)mp;
-    }
-}
-
-// A row of W elements between registers and 16-byte-aligned shared memory.
-template <typename T, int W>
-__device__ __forceinline__ void store_row(T *dst, const T (&v)[W]) {
+// N elements between registers and 16-byte-aligned shared memory.
+template <typename T, int N>
+__device__ __forceinline__ void store_row(T *dst, const T *v) {
     constexpr int VEC = 16 / sizeof(T);
 #pragma unroll
-    for (int c = 0; c < W; c += VEC) {
+    for (int c = 0; c < N; c += VEC) {
         int4 x;
         T *xx = (T *)&x;
 #pragma unroll
@@ -156,11 +124,11 @@ __device__ __forceinline__ void store_row(T *dst, const T (&v)[W]) {
         *(int4 *)(dst + c) = x;
     }
 }
-template <typename T, int W>
-__device__ __forceinline__ void load_row(T (&v)[W], const T *src) {
+template <typename T, int N>
+__device__ __forceinline__ void load_row(T *v, const T *src) {
     constexpr int VEC = 16 / sizeof(T);
 #pragma unroll
-    for (int c = 0; c < W; c += VEC) {
+    for (int c = 0; c < N; c += VEC) {
         const int4 x = *(const int4 *)(src + c);
         const T *xx = (const T *)&x;
 #pragma unroll
@@ -171,6 +139,17 @@ __device__ __forceinline__ void load_row(T (&v)[W], const T *src) {
 constexpr int LEAF_NT = 512;
 constexpr int LEAF_MAX_CS = 16;
 
+// The multiplier a / d.  FP64 divides, as the reference.  FP32 multiplies by the
+// pivot's reciprocal (taken while the arg-max picks the pivot) and corrects the
+// product by its exact remainder, which rounds as the division does but for
+// rare last bits; a pivot whose reciprocal leaves the normal range divides.
+__device__ __forceinline__ double multiplier(double a, double d, double) { return a / d; }
+__device__ __forceinline__ float multiplier(float a, float d, float y) {
+    const uint32_t u = __float_as_uint(d) & 0x7fffffffu;
+    if (u - (67u << 23) > (120u << 23)) return a / d;  // |d| outside [2^-60, 2^60]
+    const float q = a * y;
+    return fmaf(fmaf(-q, d, a), y, q);
+}
 
 template <typename T, int W, int R, int NT>
 __global__ void __launch_bounds__(NT, 1)
@@ -182,39 +161,94 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
     const int cr = (int)cl.block_rank();
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     constexpr int NW = NT / 32;
-    // in-leaf row moves: at most 2W moved rows, over at least 8 warps; at most
-    // LEAF_MAX_OTHER other panel columns, in 32-column chunks
+    constexpr int GW = W < 8 ? W : 8, NGR = W / GW;
+    constexpr int VEC = 16 / sizeof(T);               // elements per 16-byte vector
+    constexpr int CW = (VEC + GW + VEC - 1) / VEC * VEC;  // a candidate: position, live group values
+    constexpr bool STAGED = (W * sizeof(T)) % 128 == 0;   // rows of whole 128-byte segments
+    constexpr int H = STAGED ? (int)(W * sizeof(T) / 128) : 1, CC = 128 / (int)sizeof(T);
+    // in-leaf row moves: at most 2W moved rows in a CTA; at most LEAF_MAX_OTHER
+    // other panel columns
     constexpr int MOVE_PW = (2 * W + NW - 1) / NW;
-    constexpr int MOVE_CH = LEAF_MAX_OTHER / 32;
-    constexpr int VEC = 16 / sizeof(T);  // elements per 16-byte vector
-    const int G = CS * NT;  // a power of two: positions split by shift and mask
-    const int lgG = __ffs(G) - 1;
+    constexpr int MOVE_CH = LEAF_MAX_OTHER / VEC / 32 > 0 ? LEAF_MAX_OTHER / VEC / 32 : 1;
+    const int G = CS * NT;
     const int g = cr * NT + t;
-    constexpr int LG_NT = (NT == 512) ? 9 : (NT == 256 ? 8 : 10);
-    static_assert((1 << LG_NT) == NT, "NT must be 256 or 512");
 
-    __shared__ __align__(16) uint4 s_cmeta[2][LEAF_MAX_CS];  // per CTA: {key lo, key hi, position, row id}
-    __shared__ __align__(16) T s_crow[2][LEAF_MAX_CS][W];
-    __shared__ __align__(16) T s_jslot[2][W];
-    __shared__ __align__(16) uint4 s_jmeta[2];               // {row id of position j, 0, 0, 0}
-    __shared__ __align__(8) uint64_t s_xbar[2];              // exchange barriers, by column parity
-    __shared__ uint64_t s_wkey[NW];
-    __shared__ int s_wpos[NW];
-    __shared__ __align__(16) T s_myrow[W];
-    __shared__ int s_myid;
-    __shared__ __align__(16) T s_jrow[W];
-    __shared__ int s_jid;
-    __shared__ int s_piv[W];   // pivots and info stay on chip until the end: no global
-    __shared__ int s_info;     // store ahead of the per-column exchange
+    extern __shared__ __align__(16) unsigned char leaf_smem[];  // 32 rows x 144 bytes per warp (STAGED)
+    __shared__ __align__(16) T s_cand[2][NW][CW];              // this CTA's warps, by column parity
+    __shared__ __align__(16) T s_slot[2][LEAF_MAX_CS][CW];     // every CTA's winner (clusters), by column parity
+    __shared__ __align__(16) T s_right[GW][W];  // the group's pivot rows: group values, columns to the right
+    __shared__ __align__(16) T s_stage[GW][W];
+    __shared__ __align__(16) T s_u[GW][W];             // columns to the right after the unit triangle
+    __shared__ __align__(8) uint64_t s_xbar[2];        // exchange barriers, by column parity
+    __shared__ __align__(8) uint64_t s_rbar;           // pivot rows of a group
+    __shared__ int s_piv[W];   // pivots and info stay on chip until the end
+    __shared__ int s_info;
     __shared__ int s_skip;     // the call was aborted before this launch
+    __shared__ int s_mcnt;
+    __shared__ int2 s_mv[2 * W];
     if (t == 0) {
         s_info = 0;
+        s_mcnt = 0;
         s_skip = aborted(pn.abort) ? 1 : 0;
         mbar_init(&s_xbar[0], 1);
         mbar_init(&s_xbar[1], 1);
+        mbar_init(&s_rbar, 1);
         fence_barrier_init();
     }
-    // every CTA's exchange barriers exist before any CTA pushes into them
+    constexpr int PERMAX = CW / VEC;   // 16-byte chunks of a candidate
+
+    // ---- load ----
+    T r[R][W];
+    int pos[R];  // -1: no row
+    const bool vec_ok = (wact == W) && ((ld * (i64)sizeof(T)) % 16 == 0) && (((uintptr_t)P) % 16 == 0);
+    unsigned char *tr = leaf_smem + warp * (32 * 144);
+    const int trow = lane >> 3, tchk = lane & 7;       // staged transfers: four rows an instruction
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const int i = k * G + g;
+        pos[k] = i < m ? i : -1;
+#pragma unroll
+        for (int c = 0; c < W; ++c) r[k][c] = T(0);
+    }
+    if (STAGED && vec_ok) {
+        int4 x[R][H][8];
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+#pragma unroll
+            for (int hh = 0; hh < H; ++hh)
+#pragma unroll
+                for (int it = 0; it < 8; ++it) {
+                    const int i = k * G + g - lane + it * 4 + trow;
+                    x[k][hh][it] = make_int4(0, 0, 0, 0);
+                    if (i < m) x[k][hh][it] = *(const int4 *)(P + (i64)i * ld + hh * CC + tchk * VEC);
+                }
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+#pragma unroll
+            for (int hh = 0; hh < H; ++hh) {
+#pragma unroll
+                for (int it = 0; it < 8; ++it) *(int4 *)(tr + (it * 4 + trow) * 144 + tchk * 16) = x[k][hh][it];
+                __syncwarp();
+                load_row<T, W / H>(&r[k][hh * (W / H)], (const T *)(tr + lane * 144));
+                __syncwarp();
+            }
+    } else {
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            if (pos[k] >= 0) {
+                const T *src = P + (i64)pos[k] * ld;
+                if (vec_ok) {
+                    load_row<T, W>(r[k], src);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < W; ++c)
+                        if (c < wact) r[k][c] = src[c];
+                }
+            }
+        }
+    }
+    // every CTA's barriers exist before any CTA pushes into them, and
+    // every row is read before any CTA stores one at its final position
     if (CS > 1) cl.sync();
     else __syncthreads();
     // CTA 0's reading of the abort word decides for the whole cluster (the
@@ -235,297 +269,408 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
         T *ud = (T *)pn.u_dst;
         for (int e = g; e < pn.u_rows * pn.u_cols; e += G) ud[(i64)(e / pn.u_cols) * ld + e % pn.u_cols] = us[e];
     }
-
-    // ---- load: rows of W elements, 16-byte vectors when the row is whole and aligned ----
-    T r[R][W];
-    int id[R];
-    const bool vec_ok = (wact == W) && ((ld * (i64)sizeof(T)) % 16 == 0) && (((uintptr_t)P) % 16 == 0);
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-        const int i = k * G + g;
-        id[k] = i;
-#pragma unroll
-        for (int c = 0; c < W; ++c) r[k][c] = T(0);
-        if (i < m) {
-            const T *src = P + (i64)i * ld;
-            if (vec_ok) {
-#pragma unroll
-                for (int c = 0; c < W; c += VEC) {
-                    const int4 v = *(const int4 *)(src + c);
-                    const T *vv = (const T *)&v;
-#pragma unroll
-                    for (int u = 0; u < VEC; ++u) r[k][c + u] = vv[u];
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < W; ++c)
-                    if (c < wact) r[k][c] = src[c];
-            }
-        }
-    }
     const int q = m < wact ? m : wact;
+    // the same shared-memory layout in every CTA: one offset per destination
+    const int half = lane & 15;
+    const uint32_t to_cta = cluster_map_u32(&s_rbar, half < CS ? half : 0) - smem_u32(&s_rbar);
 
-    // The column loop is kept rolled (one copy of the code, resident in the
-    // instruction cache).  Each row's registers ROTATE by one slot per column:
-    // at step j the active column sits in slot 0, the unfinished columns
-    // j+1..W-1 in slots 1..W-1-j and the finished ones behind them, so every
-    // register index is static and the update is W-1 independent predicated
-    // FMAs.  After W steps the rotation has returned the row to its order.
+    // The groups are a rolled loop: the registers rotate by GW slots per group,
+    // so the active group always sits in slots 0..GW-1, the unfinished columns
+    // behind it and the finished ones last; after all groups the row is back in
+    // its order.
 #pragma unroll 1
-    for (int j = 0; j < q; ++j) {
-        const int par = j & 1;
-        // (a) this thread's best candidate in column j (slot 0)
-        uint64_t bk = 0;
-        int bp = INT_MAX;
+    for (int s = 0; s < NGR; ++s) {
+        const int j0 = s * GW;
+        uint32_t live = 0;   // columns of the group with a nonzero pivot
 #pragma unroll
-        for (int k = 0; k < R; ++k) {
-            const int i = k * G + g;
-            // _lu_pivot starts from row j with strict '>': a NaN at row j keeps
-            // row j (the largest key), a NaN below never wins (key 0)
-            const T v = r[k][0];
-            const uint64_t key = (i == j && v != v) ? ~0ull : pivot_key(v);
-            if (i >= j && i < m && (bp == INT_MAX || key > bk)) { bk = key; bp = i; }  // slots ascend in i
-        }
-        // (b) warp winner
-        warp_argmax<T>(bk, bp);
-        if (lane == 0) { s_wkey[warp] = bk; s_wpos[warp] = bp; }
-        __syncthreads();
-        // (c) CTA winner: every warp reduces the NW warp results
-        uint64_t ck = lane < NW ? s_wkey[lane] : 0ull;
-        int cp = lane < NW ? s_wpos[lane] : INT_MAX;
-        warp_argmax<T>(ck, cp);
-        if (cp != INT_MAX && (cp & (G - 1)) == g) {
-            const int kk = cp >> lgG;
+        for (int jj = 0; jj < GW; ++jj) {
+            const int j = j0 + jj;
+            if (j >= q) break;
+            const int par = jj & 1;
+            const int PER = (1 + GW - jj + VEC - 1) / VEC;  // chunks of this column's candidates
+            // (a) this thread's best candidate in column j (_lu_pivot starts from row
+            // j with strict '>')
+            uint64_t bk = step_key(r[0][jj], pos[0], j);
+            int bp = pos[0] >= j ? pos[0] : INT_MAX, bs = 0;
 #pragma unroll
-            for (int k = 0; k < R; ++k)
-                if (k == kk) {
-                    if (CS == 1) {  // a single CTA stages straight into the slots it reads
-                        store_row<T, W>(&s_crow[par][0][0], r[k]);
-                        s_cmeta[par][0] = make_uint4((uint32_t)ck, (uint32_t)(ck >> 32), (uint32_t)cp, (uint32_t)id[k]);
-                    } else {
-                        store_row<T, W>(s_myrow, r[k]);
-                        s_myid = id[k];
-                    }
+            for (int k = 1; k < R; ++k) {
+                const uint64_t key = step_key(r[k][jj], pos[k], j);
+                if (pos[k] >= j && (bp == INT_MAX || key > bk || (key == bk && pos[k] < bp))) {
+                    bk = key;
+                    bp = pos[k];
+                    bs = k;
                 }
-        }
-        if (CS == 1 && t == 0 && cp == INT_MAX) s_cmeta[par][0] = make_uint4(0u, 0u, (uint32_t)INT_MAX, 0u);
-        const bool own_j = (g == j);  // position j: slot 0 of thread j of CTA 0
-        if (own_j) {
-            if (CS == 1) {
-                store_row<T, W>(&s_jslot[par][0], r[0]);
-                s_jmeta[par] = make_uint4((uint32_t)id[0], 0u, 0u, 0u);
-            } else {
-                store_row<T, W>(s_jrow, r[0]);
-                s_jid = id[0];
             }
-        }
-        __syncthreads();
-        // (d) every CTA's candidate and, from CTA 0, row j into every CTA's slots
-        // of this parity.  Across CTAs each 16-byte store completes its bytes on
-        // the receiver's exchange barrier (st.async), and each CTA waits only on
-        // its own barrier: no cluster-wide barrier per column.  A slot is
-        // rewritten two columns later, after its receiver has pushed the column in
-        // between, i.e. after it finished reading the slot.
-        if (CS > 1 && !dead) {
-            constexpr int PER = 1 + W * (int)sizeof(T) / 16;  // stores per row: meta + 16-byte chunks
-            const int npush = CS * PER;                          // this CTA's candidate, to every CTA
-            if (t == 0) mbar_arrive_expect_tx(&s_xbar[par], (uint32_t)((CS + 1) * 16 * PER));
-            // One 16-byte store per thread, spread over the CTA's warps so that no
-            // warp issues more than one round: the candidate on threads
-            // 0..npush-1 and, in CTA 0, row j on the next npush.
-            const int nall = (cr == 0) ? 2 * npush : npush;
-            for (int e = t; e < nall; e += NT) {
-                const bool jr = e >= npush;
-                const int ee = jr ? e - npush : e;
-                const int dst = ee / PER, qq = ee - dst * PER;
-                uint4 v;
-                uint32_t raddr;
-                if (!jr) {
-                    if (qq == 0) {
-                        v = make_uint4((uint32_t)ck, (uint32_t)(ck >> 32), (uint32_t)cp, (uint32_t)s_myid);
-                        raddr = cluster_map_u32(&s_cmeta[par][cr], dst);
-                    } else {
-                        v = reinterpret_cast<const uint4 *>(s_myrow)[qq - 1];
-                        raddr = cluster_map_u32(&s_crow[par][cr][0], dst) + 16u * (qq - 1);
-                    }
-                } else {
-                    if (qq == 0) {
-                        v = make_uint4((uint32_t)s_jid, 0u, 0u, 0u);
-                        raddr = cluster_map_u32(&s_jmeta[par], dst);
-                    } else {
-                        v = reinterpret_cast<const uint4 *>(s_jrow)[qq - 1];
-                        raddr = cluster_map_u32(&s_jslot[par][0], dst) + 16u * (qq - 1);
-                    }
-                }
-                st_async_v4(raddr, v, cluster_map_u32(&s_xbar[par], dst));
-            }
-            if (!mbar_wait(&s_xbar[par], (uint32_t)((j >> 1) & 1), pn.abort, 1)) dead = true;
-        }
-        // (e) winner, identical in every CTA: lanes 0..CS-1 hold one candidate each;
-        // the winning row sits in the slot of the CTA that owns its position
-        uint64_t wk = 0ull;
-        int wp = INT_MAX;
-        if (lane < CS) {
-            const uint4 mv = s_cmeta[par][lane];
-            wk = ((uint64_t)mv.y << 32) | mv.x;
-            wp = (int)mv.z;
-        }
-        warp_argmax<T>(wk, wp);
-        const int wq = (wp == INT_MAX) ? 0 : ((wp & (G - 1)) >> LG_NT);
-        const T *prow = (wp == INT_MAX) ? &s_jslot[par][0] : &s_crow[par][wq][0];
-        const int pid = (wp == INT_MAX) ? (int)s_jmeta[par].x : (int)s_cmeta[par][wq].w;
-        if (wp == INT_MAX) wp = j;  // no comparable candidate (all NaN): keep row j
-        if (t == 0) s_piv[j] = wp;
-        const T d = prow[0];
-        if (d == T(0)) {
-            // zero pivot: info, no interchange, no elimination (the column is all zero)
-            if (t == 0 && s_info == 0) s_info = j + 1;
-        } else {
-            const int live = W - j;  // slots 1..live-1 hold the unfinished columns
-            // (f) the interchange lands in the two owner threads' registers
-            if (wp != j) {
-                if (own_j) {
+            // (b) the warp's winner into shared memory: {position, a_pj, a_p,j+1, ...}
+            {
+                const uint32_t wm = warp_winner<T>(bk, bp);
+                if (wm == 0 ? lane == 0 : ((wm >> lane) & 1)) {
+                    T row[CW];
+                    if constexpr (sizeof(T) == 4) row[0] = __int_as_float(bp);
+                    else row[0] = __longlong_as_double((long long)bp);
 #pragma unroll
-                    for (int c = 0; c < W; ++c) r[0][c] = prow[c];
-                    id[0] = pid;
-                }
-                if ((wp & (G - 1)) == g) {
-                    const int kk = wp >> lgG;
+                    for (int e = 1; e < CW; ++e) {
+                        row[e] = T(0);
+                        if (jj + e - 1 < GW) {
+                            const int c = jj + e - 1 < GW ? jj + e - 1 : 0;
+                            row[e] = r[0][c];
 #pragma unroll
-                    for (int k = 0; k < R; ++k)
-                        if (k == kk) {
-                            load_row<T, W>(r[k], &s_jslot[par][0]);
-                            id[k] = (int)s_jmeta[par].x;
+                            for (int k = 1; k < R; ++k)
+                                if (k == bs) row[e] = r[k][c];
                         }
+                    }
+#pragma unroll
+                    for (int e = 0; e < PERMAX; ++e)
+                        if (e < PER) store_row<T, VEC>(s_cand[par][warp] + e * VEC, row + e * VEC);
                 }
             }
-            // (g) scale the column and apply the rank-1 update below the pivot to
-            // the unfinished slots (the compare is uniform across the warp).  FP32
-            // multiplies finished slots by a zero instead of skipping them
-            // (fma(-l, 0, a) == a for finite l), FP64 predicates each slot: the
-            // faster form measured for each
+            __syncthreads();
+            // key, position and value of the candidate whose first chunk is h
+            auto cand_key = [&](ulonglong2 h, int &cp, T &cv) -> uint64_t {
+                if constexpr (sizeof(T) == 4) {
+                    cp = (int)(uint32_t)h.x;
+                    cv = __uint_as_float((uint32_t)(h.x >> 32));
+                } else {
+                    cp = (int)h.x;
+                    cv = __longlong_as_double((long long)h.y);
+                }
+                return step_key(cv, cp, j);
+            };
+            // the winner of n candidates, lane l looking at the first chunk h of number l
+            auto winner = [&](ulonglong2 h, int n, T &cv) -> int {
+                uint64_t ck = 0;
+                int cp = INT_MAX;
+                if (lane < n) ck = cand_key(h, cp, cv);
+                const uint32_t wm = warp_winner<T>(ck, cp);
+                return wm ? __ffs(wm) - 1 : 0;
+            };
+            T cv = T(1), v[CW];
+            int wq;
+            if (CS > 1) {
+                // (c) the CTA's winner to every CTA, warp e its chunk e
+                if (!dead) {
+                    if (t == 0) mbar_arrive_expect_tx(&s_xbar[par], (uint32_t)(CS * 16 * PER));
+                    if (warp < PER) {
+                        T w0;
+                        ulonglong2 h = make_ulonglong2(0, 0);
+                        if (lane < NW) h = *reinterpret_cast<const ulonglong2 *>(s_cand[par][lane]);
+                        const int w = winner(h, NW, w0);
+                        if (lane < CS)
+                            for (int e = warp; e < PER; e += NW)
+                                st_async_v4(smem_u32(s_slot[par][cr]) + 16u * e + to_cta,
+                                            reinterpret_cast<const uint4 *>(s_cand[par][w])[e],
+                                            smem_u32(&s_xbar[par]) + to_cta);
+                    }
+                    if (!mbar_wait(&s_xbar[par], (uint32_t)((j >> 1) & 1), pn.abort, 1)) dead = true;
+                }
+                // (d) the winner, the same in every CTA, and its row
+                ulonglong2 h = make_ulonglong2(0, 0);
+                if (lane < CS) h = *reinterpret_cast<const ulonglong2 *>(s_slot[par][lane]);
+                wq = winner(h, CS, cv);
+#pragma unroll
+                for (int e = 0; e < PERMAX; ++e)
+                    if (e < PER) load_row<T, VEC>(v + e * VEC, s_slot[par][wq] + e * VEC);
+            } else {
+                ulonglong2 h = make_ulonglong2(0, 0);
+                if (lane < NW) h = *reinterpret_cast<const ulonglong2 *>(s_cand[par][lane]);
+                wq = winner(h, NW, cv);
+#pragma unroll
+                for (int e = 0; e < PERMAX; ++e)
+                    if (e < PER) load_row<T, VEC>(v + e * VEC, s_cand[par][wq] + e * VEC);
+            }
+            T y = T(0);
+            if constexpr (sizeof(T) == 4) y = __shfl_sync(0xffffffffu, 1.0f / cv, wq);
+            int wp;
+            if constexpr (sizeof(T) == 4) wp = __float_as_int(v[0]);
+            else wp = (int)__double_as_longlong(v[0]);
+            const T d = v[1];
+            const bool ok = !is_zero(d);
+            live |= ok ? 1u << jj : 0u;
+            if (t == 0) {
+                s_piv[j] = wp;
+                // zero pivot: info, no elimination (the winner is then row j itself)
+                if (!ok && s_info == 0) s_info = j + 1;
+            }
+            // (e) interchange of positions, scaling, update inside the group
 #pragma unroll
             for (int k = 0; k < R; ++k) {
-                const int i = k * G + g;
-                if (i > j && i < m) {
-                    const T l = r[k][0] / d;
-                    r[k][0] = l;
-                    if constexpr (sizeof(T) == 4) {
+                const int p = pos[k];
+                pos[k] = p == wp ? j : (p == j ? wp : p);
+                if (ok && p >= j && p != wp) {
+                    const T l = multiplier(r[k][jj], d, y);
+                    r[k][jj] = l;
 #pragma unroll
-                        for (int c = 1; c < W; ++c) r[k][c] = fma(-l, (c < live) ? prow[c] : T(0), r[k][c]);
-                    } else {
-#pragma unroll
-                        for (int c = 1; c < W; ++c)
-                            if (c < live) r[k][c] = fma(-l, prow[c], r[k][c]);
-                    }
+                    for (int c = jj + 1; c < GW; ++c) r[k][c] = fma(-l, v[1 + c - jj], r[k][c]);
                 }
             }
         }
-        // (h) rotate: the finished column moves behind the unfinished ones
+        if constexpr (NGR > 1) {
+            const int np = min(GW, q - j0);            // pivots of this group
+            const int nblk = NGR - 1 - s;              // unfinished groups to the right
+            if (np > 0 && nblk > 0 && j0 + np < wact) {
+                const int rem = nblk * GW, nch = (GW + rem) / VEC;
+                // (f) the pivot rows' multipliers and remaining columns to every CTA
+                if (CS > 1 && t == 0 && !dead) mbar_arrive_expect_tx(&s_rbar, (uint32_t)(np * nch * 16));
 #pragma unroll
-        for (int k = 0; k < R; ++k) {
-            const T t0 = r[k][0];
+                for (int k = 0; k < R; ++k) {
+                    const int kk = pos[k] - j0;
+                    const bool own = pos[k] >= j0 && kk < np;
+                    if (own) {
+                        T *dst = (CS > 1) ? s_stage[kk] : s_right[kk];
 #pragma unroll
-            for (int c = 0; c < W - 1; ++c) r[k][c] = r[k][c + 1];
-            r[k][W - 1] = t0;
+                        for (int b = 0; b < NGR; ++b)
+                            if (b <= nblk) store_row<T, GW>(dst + b * GW, &r[k][b * GW]);
+                    }
+                    if (CS > 1) {
+                        uint32_t om = __ballot_sync(0xffffffffu, own);
+                        while (om) {
+                            const int src = __ffs(om) - 1;
+                            om &= om - 1;
+                            const int ks = __shfl_sync(0xffffffffu, kk, src);
+                            __syncwarp();
+                            if (half < CS && !dead)
+                                for (int c = lane >> 4; c < nch; c += 2)
+                                    st_async_v4(smem_u32(s_right[ks]) + 16u * c + to_cta,
+                                                reinterpret_cast<const uint4 *>(s_stage[ks])[c],
+                                                smem_u32(&s_rbar) + to_cta);
+                        }
+                    }
+                }
+                if (CS > 1) {
+                    if (warp == 0 && !dead && !mbar_wait(&s_rbar, (uint32_t)(s & 1), pn.abort, 1)) dead = true;
+                } else {
+                    __syncthreads();
+                }
+                // (g) their unit triangle, one column per lane
+                const bool full = live == (1u << GW) - 1;
+                if (warp == 0 && lane < rem) {
+                    T x[GW];
+#pragma unroll
+                    for (int k = 0; k < GW; ++k) x[k] = k < np ? s_right[k][GW + lane] : T(0);
+                    if (full) {
+#pragma unroll
+                        for (int p = 0; p < GW; ++p)
+#pragma unroll
+                            for (int k = p + 1; k < GW; ++k) x[k] = fma(-s_right[k][p], x[p], x[k]);
+                    } else {
+                        for (int p = 0; p < np; ++p) {
+                            if (!((live >> p) & 1)) continue;
+#pragma unroll
+                            for (int k = 1; k < GW; ++k) {
+                                T xp = x[0];
+#pragma unroll
+                                for (int e = 1; e < GW; ++e) xp = e == p ? x[e] : xp;
+                                if (k > p && k < np) x[k] = fma(-s_right[k][p], xp, x[k]);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < GW; ++k) s_u[k][lane] = x[k];
+                }
+                __syncthreads();
+                // (h) the group's updates of the remaining columns: the rows below the
+                // pivots take them all; a pivot row's own are its row of the triangle's
+                // solution
+                bool act[R];
+                bool any = false;
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    act[k] = pos[k] >= j0 + np;
+                    any = any || act[k];
+                }
+                const bool warp_any = __any_sync(0xffffffffu, any);
+#pragma unroll
+                for (int b = 0; b < NGR - 1; ++b) {
+                    if (b < nblk) {
+                        if (warp_any) {
+                            T nv[R][GW];
+#pragma unroll
+                            for (int k = 0; k < R; ++k)
+#pragma unroll
+                                for (int c = 0; c < GW; ++c) nv[k][c] = r[k][(b + 1) * GW + c];
+                            if (full) {
+#pragma unroll
+                                for (int p = 0; p < GW; ++p) {
+                                    T u[GW];
+                                    load_row<T, GW>(u, &s_u[p][b * GW]);
+#pragma unroll
+                                    for (int k = 0; k < R; ++k)
+#pragma unroll
+                                        for (int c = 0; c < GW; ++c) nv[k][c] = fma(-r[k][p], u[c], nv[k][c]);
+                                }
+                            } else {
+#pragma unroll
+                                for (int p = 0; p < GW; ++p) {
+                                    if (!((live >> p) & 1)) continue;
+                                    T u[GW];
+                                    load_row<T, GW>(u, &s_u[p][b * GW]);
+#pragma unroll
+                                    for (int k = 0; k < R; ++k)
+#pragma unroll
+                                        for (int c = 0; c < GW; ++c) nv[k][c] = fma(-r[k][p], u[c], nv[k][c]);
+                                }
+                            }
+#pragma unroll
+                            for (int k = 0; k < R; ++k)
+#pragma unroll
+                                for (int c = 0; c < GW; ++c)
+                                    if (act[k]) r[k][(b + 1) * GW + c] = nv[k][c];
+                        }
+#pragma unroll
+                        for (int k = 0; k < R; ++k) {
+                            const int kk = pos[k] - j0;
+                            if (pos[k] >= j0 && kk < np) load_row<T, GW>(&r[k][(b + 1) * GW], &s_u[kk][b * GW]);
+                        }
+                    }
+                }
+            }
+            // the finished group moves behind the unfinished columns
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                T f[GW];
+#pragma unroll
+                for (int c = 0; c < GW; ++c) f[c] = r[k][c];
+#pragma unroll
+                for (int c = 0; c < W - GW; ++c) r[k][c] = r[k][c + GW];
+#pragma unroll
+                for (int c = 0; c < GW; ++c) r[k][W - GW + c] = f[c];
+            }
         }
     }
     // pivots and info, written once
     dead = __syncthreads_or(dead);
     if (!dead && cr == 0 && t < q) ipiv[gofs + t] = gofs + s_piv[t] + 1;
     if (!dead && cr == 0 && t == 0 && s_info != 0 && *info == 0) *info = gofs + s_info;
-    // undo the rotation left by q < W steps (slot s holds column (s + q) mod W)
-    const int rot = q % W;
 
-    // store the leaf and emit the moves of the net permutation
+    // ---- store every row at its final position ----
+    const bool inleaf = pn.nother > 0 || pn.map;  // the moves are applied here, not by a later launch
+    if (!dead) {
 #pragma unroll
-    for (int k = 0; k < R; ++k) {
-        const int i = k * G + g;
-        if (i < m && !dead) {
-            T *dst = P + (i64)i * ld;
-            if (vec_ok && rot == 0) {
-#pragma unroll
-                for (int c = 0; c < W; c += VEC) {
-                    int4 v;
-                    T *vv = (T *)&v;
-#pragma unroll
-                    for (int u = 0; u < VEC; ++u) vv[u] = r[k][c + u];
-                    *(int4 *)(dst + c) = v;
-                }
-            } else {
-#pragma unroll
-                for (int s = 0; s < W; ++s) {
-                    int c = s + rot;
-                    if (c >= W) c -= W;
-                    if (c < wact) dst[c] = r[k][s];
+        for (int k = 0; k < R; ++k) {
+            const int i = k * G + g;
+            if (pos[k] >= 0 && pos[k] != i) {
+                if (inleaf) {
+                    const int slot = atomicAdd(&s_mcnt, 1);
+                    s_mv[slot] = make_int2(pos[k], i);
+                } else {
+                    const int slot = atomicAdd(nmoves, 1);
+                    moves[2 * slot] = pos[k];
+                    moves[2 * slot + 1] = i;
                 }
             }
-            if (id[k] != i) {
-                const int slot = atomicAdd(nmoves, 1);
-                moves[2 * slot] = i;
-                moves[2 * slot + 1] = id[k];
+            if (STAGED && vec_ok) {
+#pragma unroll
+                for (int hh = 0; hh < H; ++hh) {
+                    store_row<T, W / H>((T *)(tr + lane * 144), &r[k][hh * (W / H)]);
+                    __syncwarp();
+#pragma unroll
+                    for (int it = 0; it < 8; ++it) {
+                        const int dst = __shfl_sync(0xffffffffu, pos[k], it * 4 + trow);
+                        if (dst >= 0)
+                            *(int4 *)(P + (i64)dst * ld + hh * CC + tchk * VEC) =
+                                *(const int4 *)(tr + (it * 4 + trow) * 144 + tchk * 16);
+                    }
+                    __syncwarp();
+                }
+            } else if (pos[k] >= 0) {
+                T *dst = P + (i64)pos[k] * ld;
+                if (vec_ok) {
+                    store_row<T, W>(dst, r[k]);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < W; ++c)
+                        if (c < wact) dst[c] = r[k][c];
+                }
             }
         }
     }
-    if (pn.nother > 0 || pn.map) {
+    if (inleaf) {
         // The leaf's row interchanges on the panel's other columns, and on the
-        // panel row map, done here rather than by separate launches: read every
-        // moved row segment, meet at a cluster barrier, write.
-        __threadfence();
-        if (CS > 1) cl.sync(); else __syncthreads();
-        const int cnt = min(*(volatile int *)nmoves, 2 * W);
-        // One warp per moved row (warps of the whole cluster, in turn), one lane
-        // per column of each 32-column chunk: no division, and the leaf's rows are
-        // stored, so their registers are free for the staged values.
-        const int gw = cr * NW + warp, nwc = CS * NW;
-        const int nother = pn.nother;
-        T vals[MOVE_PW][MOVE_CH];
-        int dsts[MOVE_PW];
+        // panel row map, done here rather than by separate launches: each CTA
+        // reads the segments of its own moved rows, all CTAs meet, and each
+        // writes them at their final positions (one warp per moved row, 16 bytes
+        // a lane where the panel's column ranges allow it).
         int mapv[R];
 #pragma unroll
-        for (int mi = 0; mi < MOVE_PW; ++mi) {
-            const int mv = gw + mi * nwc;
-            dsts[mi] = -1;
-            if (mv < cnt) {
-                const int src = __ldcg(&moves[2 * mv + 1]);
-                dsts[mi] = __ldcg(&moves[2 * mv]);
-                const T *srow = P + (i64)src * ld - pn.leaf_c0;
+        for (int k = 0; k < R; ++k) {
+            const int i = k * G + g;
+            mapv[k] = (!dead && pn.map && pos[k] >= 0 && pos[k] != i) ? pn.map[pn.map_off + i] : 0;
+        }
+        __syncthreads();
+        const int cnt = s_mcnt;
+        const int nother = pn.nother;
+        T *const base = P - pn.leaf_c0;
+        const bool mvec = ((ld * (i64)sizeof(T)) % 16 == 0) && (((uintptr_t)base) % 16 == 0) &&
+                          ((pn.left_n | pn.pc_lo | pn.right_lo | nother) % VEC == 0);
+        if (mvec) {
+            const int nv = nother / VEC;
+            int off[MOVE_CH];
 #pragma unroll
-                for (int ci = 0; ci < MOVE_CH; ++ci) {
-                    const int oc = ci * 32 + lane;
-                    if (oc < nother) vals[mi][ci] = srow[oc < pn.left_n ? pn.pc_lo + oc : pn.right_lo + (oc - pn.left_n)];
+            for (int ci = 0; ci < MOVE_CH; ++ci) {
+                const int oc = (ci * 32 + lane) * VEC;
+                off[ci] = ci * 32 + lane >= nv ? -1 : (oc < pn.left_n ? pn.pc_lo + oc : pn.right_lo + (oc - pn.left_n));
+            }
+            int4 vals[MOVE_PW][MOVE_CH];
+#pragma unroll
+            for (int mi = 0; mi < MOVE_PW; ++mi) {
+                const int mv = warp + mi * NW;
+                if (mv < cnt) {
+                    const T *srow = base + (i64)s_mv[mv].y * ld;
+#pragma unroll
+                    for (int ci = 0; ci < MOVE_CH; ++ci)
+                        if (off[ci] >= 0) vals[mi][ci] = *(const int4 *)(srow + off[ci]);
+                }
+            }
+            if (CS > 1) cl.sync();
+            else __syncthreads();
+#pragma unroll
+            for (int mi = 0; mi < MOVE_PW; ++mi) {
+                const int mv = warp + mi * NW;
+                if (mv < cnt) {
+                    T *drow = base + (i64)s_mv[mv].x * ld;
+#pragma unroll
+                    for (int ci = 0; ci < MOVE_CH; ++ci)
+                        if (off[ci] >= 0) *(int4 *)(drow + off[ci]) = vals[mi][ci];
+                }
+            }
+        } else {
+            constexpr int SCH = LEAF_MAX_OTHER / 32;
+            T vals[MOVE_PW][SCH];
+#pragma unroll
+            for (int mi = 0; mi < MOVE_PW; ++mi) {
+                const int mv = warp + mi * NW;
+                if (mv < cnt) {
+                    const T *srow = base + (i64)s_mv[mv].y * ld;
+#pragma unroll
+                    for (int ci = 0; ci < SCH; ++ci) {
+                        const int oc = ci * 32 + lane;
+                        if (oc < nother) vals[mi][ci] = srow[oc < pn.left_n ? pn.pc_lo + oc : pn.right_lo + (oc - pn.left_n)];
+                    }
+                }
+            }
+            if (CS > 1) cl.sync();
+            else __syncthreads();
+#pragma unroll
+            for (int mi = 0; mi < MOVE_PW; ++mi) {
+                const int mv = warp + mi * NW;
+                if (mv < cnt) {
+                    T *drow = base + (i64)s_mv[mv].x * ld;
+#pragma unroll
+                    for (int ci = 0; ci < SCH; ++ci) {
+                        const int oc = ci * 32 + lane;
+                        if (oc < nother) drow[oc < pn.left_n ? pn.pc_lo + oc : pn.right_lo + (oc - pn.left_n)] = vals[mi][ci];
+                    }
                 }
             }
         }
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const int i = k * G + g;
-            mapv[k] = (!dead && pn.map && i < m && id[k] != i) ? pn.map[pn.map_off + id[k]] : 0;
+            if (!dead && pn.map && pos[k] >= 0 && pos[k] != i) pn.map[pn.map_off + pos[k]] = mapv[k];
         }
-        if (CS > 1) cl.sync(); else __syncthreads();
-#pragma unroll
-        for (int mi = 0; mi < MOVE_PW; ++mi) {
-            if (dsts[mi] >= 0) {
-                T *drow = P + (i64)dsts[mi] * ld - pn.leaf_c0;
-#pragma unroll
-                for (int ci = 0; ci < MOVE_CH; ++ci) {
-                    const int oc = ci * 32 + lane;
-                    if (oc < nother) drow[oc < pn.left_n ? pn.pc_lo + oc : pn.right_lo + (oc - pn.left_n)] = vals[mi][ci];
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            const int i = k * G + g;
-            if (!dead && pn.map && i < m && id[k] != i) pn.map[pn.map_off + i] = mapv[k];
-        }
-    }
-    // keep every CTA's shared memory alive until all remote pushes have landed
-    if (CS > 1) cl.sync();
-    // the move counter back to zero for the next leaf, once every CTA has read it
-    if (pn.reset_nmoves) {
-        if (CS == 1) __syncthreads();
-        if (cr == 0 && t == 0) *nmoves = 0;
+    } else if (CS > 1) {
+        // every push into a CTA that gave up has landed before its shared memory goes
+        cl.sync();
     }
 }
 
@@ -552,14 +697,15 @@ static void launch_leaf_wr(T *P, i64 ld, i64 m, int w, i64 gofs, int64_t *ipiv, 
                            int *moves, int *nmoves, cudaStream_t s, LeafPanel pn) {
     const i64 per_cta = (i64)NT * R;
     int need = (int)((m + per_cta - 1) / per_cta);
-    int cs = 1;  // cluster sizes kept to powers of two
-    while (cs < need) cs <<= 1;
+    const int cs = need;
     auto kern = k_leaf_lu<T, W, R, NT>;
     if (cs > 8) OXI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cs);
     cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = 0;
+    constexpr int smem = (W * sizeof(T)) % 128 == 0 ? (NT / 32) * 32 * 144 : 0;
+    if (smem > 0) set_max_dyn_smem((const void *)kern, smem);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -579,18 +725,16 @@ static void launch_leaf_wr(T *P, i64 ld, i64 m, int w, i64 gofs, int64_t *ipiv, 
 template <typename T>
 void launch_leaf(T *P, i64 ld, i64 m, int w, i64 gofs, int64_t *ipiv, int64_t *info, int *moves,
                  int *nmoves, int leafw, cudaStream_t s, LeafPanel pn) {
-    const i64 cap = (i64)LEAF_MAX_CS * LEAF_NT;
-    // FP32 32-wide leaves up to 8192 rows: 256 threads x 2 rows (about 15% faster per
-    // column than 512 x 1: half the warps repeat the per-column work); FP64 keeps
-    // 512 x 1 (its 2-row variant needs 254 registers and measured slower)
     if constexpr (sizeof(T) == 8) {
-        if (leafw == 32) launch_leaf_wr<T, 32, 1>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
+        if (leafw == 32 && m <= LEAF_MAX_CS * 256) launch_leaf_wr<T, 32, 1, 256>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
+        else if (leafw == 32) launch_leaf_wr<T, 32, 1>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
         else if (leafw == 16) launch_leaf_wr<T, 16, 2>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
         else if (leafw == 8) launch_leaf_wr<T, 8, 4>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
         else launch_leaf_wr<T, 4, 8>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
     } else {
         if (leafw == 32) {
-            if (m <= cap) launch_leaf_wr<T, 32, 2, 256>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
+            if (m <= LEAF_MAX_CS * 256) launch_leaf_wr<T, 32, 1, 256>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
+            else if (m <= LEAF_MAX_CS * LEAF_NT) launch_leaf_wr<T, 32, 1>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
             else launch_leaf_wr<T, 32, 2>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
         } else if (leafw == 16) {
             launch_leaf_wr<T, 16, 4>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
@@ -648,15 +792,12 @@ template void launch_rowmoves<float>(float *, i64, i64, const int *, const int *
 // leaf's moves compose into it, and at the end of the panel the positions with
 // map[p] != p form one move list for all the columns outside the panel.
 // ---------------------------------------------------------------------------
-// identity row map of a panel; also zeroes the panel's move counter and its
-// move-list count (no separate memsets on the panel's critical path)
-__global__ void k_rowmap_init(int *__restrict__ map, int len, int *__restrict__ zero0, int *__restrict__ zero1) {
+// identity row map of a panel; also zeroes the panel's move-list count (no
+// separate memset on the panel's critical path)
+__global__ void k_rowmap_init(int *__restrict__ map, int len, int *__restrict__ listcnt) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p < len) map[p] = p;
-    if (p == 0) {
-        if (zero0) *zero0 = 0;
-        if (zero1) *zero1 = 0;
-    }
+    if (p == 0) *listcnt = 0;
 }
 __global__ void k_rowmap_apply(int *__restrict__ map, int offset, const int *__restrict__ moves,
                                const int *__restrict__ nmoves) {
@@ -727,9 +868,9 @@ __global__ void __launch_bounds__(256) k_rowmoves_big(T *__restrict__ W, i64 ld,
     }
 }
 
-void launch_rowmap_init(int *map, i64 len, int *zero0, int *zero1, cudaStream_t s) {
+void launch_rowmap_init(int *map, i64 len, int *listcnt, cudaStream_t s) {
     if (len <= 0) return;
-    k_rowmap_init<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(map, (int)len, zero0, zero1);
+    k_rowmap_init<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(map, (int)len, listcnt);
     OXI_LAUNCH_CHECK();
 }
 void launch_rowmap_apply(int *map, i64 offset, const int *moves, const int *nmoves, cudaStream_t s) {

@@ -257,8 +257,6 @@ struct LeafPanel {
     const void *u_src = nullptr;
     void *u_dst = nullptr;
     int u_rows = 0, u_cols = 0;
-    // set the move counter back to zero at the end (saves the next leaf's memset)
-    int reset_nmoves = 0;
     // the call's abort word (set by launch_leaf)
     int *abort = nullptr;
 };
@@ -287,7 +285,7 @@ void launch_rowmoves(T *W, i64 ld, i64 r0, const int *moves, const int *nmoves, 
                      i64 c_hi, i64 skip_lo, i64 skip_hi, cudaStream_t s);
 
 // Per-panel composition of the leaves' row permutations (see lu_kernels.cu).
-void launch_rowmap_init(int *map, i64 len, int *zero0, int *zero1, cudaStream_t s);
+void launch_rowmap_init(int *map, i64 len, int *listcnt, cudaStream_t s);
 void launch_rowmap_apply(int *map, i64 offset, const int *moves, const int *nmoves, cudaStream_t s);
 void launch_rowmap_extract(const int *map, i64 len, int *list, int *cnt, cudaStream_t s);
 template <typename T>

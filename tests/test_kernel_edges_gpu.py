@@ -1,0 +1,127 @@
+"""The kernels at the sizes where their tiles, remainders and branches change,
+against the oracle or a 64-bit NumPy solve.
+
+FP64 LU factors are the oracle's bits.  Solves: a backward stable solve leaves
+max|b - A x| <= c n eps (|A||x| + |b|) with c of the order of the growth of the
+blocks' inverses; the bound below is 30 n eps of the normwise terms, the bar
+the reference's own solves are held to.
+"""
+import numpy as np
+import pytest
+import scipy.linalg as sl
+import torch
+
+pytestmark = pytest.mark.gpu
+EPS = np.finfo(float).eps
+
+
+def _np(t):
+    return t.detach().cpu().numpy()
+
+
+def _backward(A, x, b):
+    r = np.abs(b - A @ x).max()
+    return r / (np.abs(A).sum(1).max() * np.abs(x).max() + np.abs(b).max()) / (A.shape[0] * EPS)
+
+
+@pytest.mark.parametrize("m", [5, 31, 33, 255, 256, 257, 513, 4095, 4096, 4097, 8191, 8193])
+def test_leaf_heights_bit_identical(pkg, oracle, m):
+    """Rows per CTA and cluster sizes of the leaf change with the height; 40
+    columns leave a whole leaf and a narrow one.  Values of equal magnitude make
+    the arg-max resolve ties by position."""
+    rng = np.random.default_rng(m)
+    for A in (rng.standard_normal((m, 40)), rng.integers(-2, 3, (m, 40)).astype(float)):
+        F = pkg.lu(A, check=False)
+        Fo, ipo, info = oracle.getrf(A, check=False)
+        assert F.info == info
+        assert np.array_equal(_np(F.ipiv), ipo)
+        assert np.array_equal(_np(F.factors), Fo)
+
+
+def test_leaf_zero_nan_and_extreme_pivots(pkg, oracle):
+    rng = np.random.default_rng(7)
+    A = rng.standard_normal((300, 64))
+    A[:, 11] = 0.0                       # a zero pivot inside a group
+    A[:, 20] = A[:, 3] * 2.0             # rank deficiency found by elimination
+    A[40:, 33] = np.nan                  # a NaN below never wins
+    B = rng.standard_normal((300, 64)) * 10.0 ** rng.uniform(-250, 250, (300, 1))
+    C = rng.standard_normal((300, 64))
+    C[rng.uniform(size=C.shape) < 0.3] = -0.0
+    for M in (A, B, C):
+        F = pkg.lu(M, check=False)
+        Fo, ipo, info = oracle.getrf(M, check=False)
+        assert F.info == info
+        assert np.array_equal(_np(F.ipiv), ipo)
+        assert np.array_equal(_np(F.factors), Fo, equal_nan=True)
+
+
+@pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 511, 513, 1100])
+@pytest.mark.parametrize("nrhs", [1, 2, 3, 7, 8, 17])
+def test_superblock_solves(pkg, n, nrhs):
+    rng = np.random.default_rng(1000 * n + nrhs)
+    A = rng.standard_normal((n, n)) + 2 * np.sqrt(n) * np.eye(n)
+    B = rng.standard_normal((n, nrhs))
+    F = pkg.lu(A)
+    assert _backward(A, _np(F.solve(B)), B) <= 30
+    assert _backward(A.T, _np(F.T.solve(B)), B) <= 30
+    S = A @ A.T / n + np.eye(n)
+    S = (S + S.T) / 2
+    assert _backward(S, _np(pkg.cholesky(S).solve(torch.from_numpy(B))), B) <= 30
+
+
+@pytest.mark.parametrize("n", [1, 33, 127, 128, 129, 300])
+@pytest.mark.parametrize("nrhs", [1, 2, 5])
+def test_superblock_solves_complex(pkg, n, nrhs):
+    rng = np.random.default_rng(1000 * n + nrhs)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 2 * np.sqrt(n) * np.eye(n)
+    B = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    F = pkg.lu(A)
+    assert _backward(A, _np(F.solve(B)), B) <= 30
+    assert _backward(A.T, _np(F.T.solve(B)), B) <= 30
+    assert _backward(A.conj().T, _np(F.H.solve(B)), B) <= 30
+
+
+@pytest.mark.parametrize("m", [15, 16, 17, 255, 257, 4096, 4097, 8193])
+def test_complex_leaf_heights(pkg, oracle, m):
+    """Pivots as the oracle's; the overflow rule (abs2 not finite) inside a group."""
+    rng = np.random.default_rng(m)
+    A = rng.standard_normal((m, 20)) + 1j * rng.standard_normal((m, 20))
+    A[m // 2, 2] = 1e200 + 1e200j
+    A[m // 3, 2] = 2e200
+    F = pkg.lu(A, check=False)
+    Fo, ipo, info = oracle.zgetrf(A)
+    assert F.info == info
+    assert np.array_equal(_np(F.ipiv), ipo)
+    assert np.linalg.norm(_np(F.factors) - Fo) <= 1e-11 * np.linalg.norm(Fo)
+
+
+@pytest.mark.parametrize("n", [8, 9, 31, 121, 127, 129, 136, 257, 385])
+def test_cholesky_blocks_and_first_failing_column(pkg, oracle, n):
+    rng = np.random.default_rng(n)
+    G = rng.standard_normal((n, n))
+    A = G @ G.T + n * np.eye(n)
+    Lo, _ = oracle.potrf(A)
+    assert np.linalg.norm(_np(pkg.cholesky(A).L) - Lo) <= 1e-13 * np.linalg.norm(Lo)
+    for bad in sorted({0, 7, 8, n // 2, n - 1}):
+        if bad >= n:
+            continue
+        M = A.copy()
+        M[bad, bad] = -1.0
+        assert pkg.cholesky(M, check=False).info == oracle.potrf(M)[1] == bad + 1
+
+
+@pytest.mark.parametrize("nrhs", [4, 5, 8, 9, 16])
+@pytest.mark.parametrize("n", [130, 300, 1027])
+def test_mixed_solve_right_hand_sides(pkg, n, nrhs):
+    """The residual's tensor-core pass (more than four right-hand sides) and the
+    narrow block solve of the FP32 panels, whole and ragged."""
+    rng = np.random.default_rng(n + nrhs)
+    A = rng.standard_normal((n, n)) + 2 * np.sqrt(n) * np.eye(n)
+    B = rng.standard_normal((n, nrhs))
+    r = pkg.mixed_solve(A, B, maxiter=20, rtol=1e-14, precision="fp16x3", refine="auto", normwise=True)
+    x = _np(r["x"])
+    assert r["converged"]
+    res = np.abs(B - A @ x).max(0) / (np.abs(A).sum(1).max() * np.abs(x).max(0) + np.abs(B).max(0))
+    assert res.max() <= 1e-14 + 4 * n * EPS  # the report's value up to the rounding of this residual
+    xe = sl.solve(A, B)
+    assert np.linalg.norm(x - xe) <= 1e-10 * np.linalg.norm(xe)
