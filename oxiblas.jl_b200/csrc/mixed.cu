@@ -421,7 +421,7 @@ struct MixedRun {
     int64_t *perm, *ipiv;
     void *W;  // float (low) or double (fallback) row-major factors
     i64 ldw;
-    void *dinvL, *dinvU;  // inverses of the 64 x 64 diagonal blocks of L and U
+    void *dinvL, *dinvU;  // superblock inverses of L and U (tri_inverses)
     bool fallback = false;
     bool chol = false;  // Cholesky family: W holds the column-major lower factor L
     double *scal;  // device scalars (cw/rmax/xmax/bmax per rhs, r^2)
@@ -497,21 +497,21 @@ static void precond(MixedRun &M, const double *Rin, i64 ldr, double *Z, i64 ldz,
         k_to_low<float><<<gb, 256, 0, s>>>(Rin, ldr, n, nr, M.rows, M.perm, M.mag, M.low32, M.err);
         OXI_LAUNCH_CHECK();
         if (M.chol)
-            chol_solve_ops<float>(M.h, (const float *)M.W, M.ldw, n, M.low32, n, nr, M.err,
-                                  (const float *)M.dinvL, (const float *)M.dinvU);
+            tri_solves<float>(M.h, TriForm::CHOLESKY, (const float *)M.W, M.ldw, n, M.low32, n, nr, M.err,
+                              (const float *)M.dinvL, (const float *)M.dinvU);
         else
-            lu_solve_rowmajor<float>(M.h, (const float *)M.W, M.ldw, n, M.low32, n, nr, M.err,
-                                     (const float *)M.dinvL, (const float *)M.dinvU);
+            tri_solves<float>(M.h, TriForm::LU_ROWMAJOR, (const float *)M.W, M.ldw, n, M.low32, n, nr, M.err,
+                              (const float *)M.dinvL, (const float *)M.dinvU);
         k_apply_corr<float><<<gb, 256, 0, s>>>(Z, ldz, n, nr, M.low32, M.mag, M.cols, 0);
     } else {
         k_to_low<double><<<gb, 256, 0, s>>>(Rin, ldr, n, nr, M.rows, M.perm, M.mag, M.low64, M.err);
         OXI_LAUNCH_CHECK();
         if (M.chol)
-            chol_solve_ops<double>(M.h, (const double *)M.W, M.ldw, n, M.low64, n, nr, M.err,
-                                   (const double *)M.dinvL, (const double *)M.dinvU);
+            tri_solves<double>(M.h, TriForm::CHOLESKY, (const double *)M.W, M.ldw, n, M.low64, n, nr, M.err,
+                              (const double *)M.dinvL, (const double *)M.dinvU);
         else
-            lu_solve_rowmajor<double>(M.h, (const double *)M.W, M.ldw, n, M.low64, n, nr, M.err,
-                                      (const double *)M.dinvL, (const double *)M.dinvU);
+            tri_solves<double>(M.h, TriForm::LU_ROWMAJOR, (const double *)M.W, M.ldw, n, M.low64, n, nr, M.err,
+                              (const double *)M.dinvL, (const double *)M.dinvU);
         k_apply_corr<double><<<gb, 256, 0, s>>>(Z, ldz, n, nr, M.low64, M.mag, M.cols, 0);
     }
     OXI_LAUNCH_CHECK();
@@ -666,7 +666,7 @@ static int dgesv_mixed(oxi_handle_s *h, int prec, int refine, i64 n, i64 nrhs, c
                  o_perm = take(8 * n), o_ipiv = take(8 * n), o_V = take(8 * n * GM_MAXV),
                  o_gw = take(8 * n), o_gt = take(8 * n), o_gpart = take(8 * 120 * GM_MAXV),
                  o_gh = take(8 * GM_MAXV), o_gz = take(8 * n),
-                 o_dinv = take(2 * 8 * (size_t)lu_block_inverse_elems(n)),
+                 o_dinv = take(2 * 8 * (size_t)tri_inverse_elems<double>(n)),
                  o_pwork = chol ? take(8 * potrf_work_elems(n)) : take(0);
     char *ws = (char *)h->mixed_ws.get(off);
     M.rows = (double *)(ws + o_rows); M.cols = (double *)(ws + o_cols);
@@ -677,7 +677,7 @@ static int dgesv_mixed(oxi_handle_s *h, int prec, int refine, i64 n, i64 nrhs, c
     M.perm = (int64_t *)(ws + o_perm); M.ipiv = (int64_t *)(ws + o_ipiv);
     M.V = (double *)(ws + o_V); M.gw = (double *)(ws + o_gw); M.gt = (double *)(ws + o_gt);
     M.gpart = (double *)(ws + o_gpart); M.gh = (double *)(ws + o_gh); M.gz = (double *)(ws + o_gz);
-    const i64 inv_elems = lu_block_inverse_elems(n);
+    const i64 inv_elems = tri_inverse_elems<double>(n);
     char *sc = (char *)h->scratch.get(kScratchBytes);
     M.err = (int *)(sc + kScratchErrOff);
     int *nonfinite = M.err + 1;
@@ -761,7 +761,7 @@ static int dgesv_mixed(oxi_handle_s *h, int prec, int refine, i64 n, i64 nrhs, c
             }
             h->trailing = saved_tr;
             M.dinvU = (float *)M.dinvL + inv_elems;
-            chol_block_ops<float>(h, W, ldw, n, (float *)M.dinvL, (float *)M.dinvU);
+            tri_inverses<float>(h, TriForm::CHOLESKY, W, ldw, n, (float *)M.dinvL, (float *)M.dinvU);
         } else {
             double *W = (double *)h->work.get((size_t)n * ldw * sizeof(double));
             M.W = W;
@@ -769,7 +769,7 @@ static int dgesv_mixed(oxi_handle_s *h, int prec, int refine, i64 n, i64 nrhs, c
             OXI_LAUNCH_CHECK();
             potrf_rowmajor<double>(h, W, ldw, n, d_info, (double *)(ws + o_pwork));
             M.dinvU = (double *)M.dinvL + inv_elems;
-            chol_block_ops<double>(h, W, ldw, n, (double *)M.dinvL, (double *)M.dinvU);
+            tri_inverses<double>(h, TriForm::CHOLESKY, W, ldw, n, (double *)M.dinvL, (double *)M.dinvU);
         }
         OXI_CUDA(cudaMemcpyAsync(M.hpiv, d_info, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
         OXI_CUDA(cudaStreamSynchronize(s));
@@ -813,11 +813,11 @@ static int dgesv_mixed(oxi_handle_s *h, int prec, int refine, i64 n, i64 nrhs, c
         if (!fp64) {
             M.dinvL = ws + o_dinv;
             M.dinvU = (float *)M.dinvL + inv_elems;
-            lu_block_inverses_rowmajor<float>(h, (const float *)M.W, ldw, n, (float *)M.dinvL, (float *)M.dinvU);
+            tri_inverses<float>(h, TriForm::LU_ROWMAJOR, (const float *)M.W, ldw, n, (float *)M.dinvL, (float *)M.dinvU);
         } else {
             M.dinvL = ws + o_dinv;
             M.dinvU = (double *)M.dinvL + inv_elems;
-            lu_block_inverses_rowmajor<double>(h, (const double *)M.W, ldw, n, (double *)M.dinvL, (double *)M.dinvU);
+            tri_inverses<double>(h, TriForm::LU_ROWMAJOR, (const double *)M.W, ldw, n, (double *)M.dinvL, (double *)M.dinvU);
         }
         OXI_CUDA(cudaMemcpyAsync(M.hpiv, d_info, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
         OXI_CUDA(cudaMemcpyAsync(M.hpiv + 8, M.ipiv, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, s));

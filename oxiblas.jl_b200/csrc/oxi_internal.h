@@ -39,8 +39,6 @@ constexpr size_t kScratchBytes = 65536;
 constexpr size_t kScratchErrOff = 1024;     // the abort block (16 bytes), then other int error words
 constexpr size_t kScratchStallOff = 1984;   // flag of the missing-producer test hook (never set)
 constexpr size_t kScratchScalOff = 2048;    // double scalars of the mixed path
-constexpr size_t kScratchTrsvOff = 8192;    // triangular-solve tickets and flags
-constexpr int kTrsvCtlInts = (int)((kScratchBytes - kScratchTrsvOff) / sizeof(int));
 
 // Device workspace owned by a handle; grows monotonically.
 struct DeviceBuffer {
@@ -133,8 +131,8 @@ struct oxi_handle_s {
     cudaStream_t la_main = nullptr;          // lookahead: the panels' stream (highest priority)
     cudaEvent_t la_in = nullptr, la_out = nullptr;  // caller's stream -> la_main -> caller's stream
     cudaEvent_t la_fork = nullptr, la_join = nullptr;
-    oxi::DeviceBuffer xtag_ws;   // tagged solution words of the triangular solves
-    oxi::DeviceBuffer trsv_ws;   // per-block solve operators of getrs (inverse + two coupling blocks)
+    oxi::DeviceBuffer xtag_ws;   // tickets and exchange words of the triangular solves
+    oxi::DeviceBuffer trsv_ws;   // superblock inverses of getrs / potrs
     oxi::DeviceBuffer rowmap_ws; // per-panel row map and composite move list
     oxi::DeviceBuffer tslu_ws;   // tournament-pivoting tree of the FP32 leaves
     int tslu = 0;                // 1 inside the mixed solve's FP32 factor: tournament leaves
@@ -343,14 +341,42 @@ size_t potrf_work_elems(i64 n);
 void ensure_lookahead_streams(oxi_handle_s *h);
 template <typename T>
 void potrf_rowmajor(oxi_handle_s *h, T *U, i64 ld, i64 n, int64_t *d_info, T *work);
-// Solves with a column-major lower Cholesky factor L: the block operators of L
-// and of L^T (lu_block_inverse_elems(n) elements each), then L L^T X = B in
-// place with them (solve.cu).
+// Triangular solves in superblocks (trsv.cu).  tri_inverses: the superblock
+// inverses of both triangles of a factor, tri_inverse_elems(n) elements each;
+// tri_solves: the two solves in the form's order, X (column-major n x nrhs) in
+// place.  *err is the call's abort block.
+enum class TriForm {
+    LU_N,         // column-major LU: L, then U
+    LU_T,         // column-major LU: U^T, then L^T
+    LU_C,         // the same with the conjugates (complex elements)
+    LU_ROWMAJOR,  // row-major LU: L, then U
+    CHOLESKY,     // column-major lower L: L, then L^T
+};
+// A complex element as the solves compute with it: the layout of double2.
+struct __align__(16) zc64 {
+    double x, y;
+    zc64() = default;
+    __host__ __device__ explicit zc64(double re, double im = 0.0) : x(re), y(im) {}
+};
+__host__ __device__ inline zc64 operator+(zc64 a, zc64 b) { return zc64(a.x + b.x, a.y + b.y); }
+__host__ __device__ inline zc64 operator-(zc64 a, zc64 b) { return zc64(a.x - b.x, a.y - b.y); }
+__host__ __device__ inline zc64 operator-(zc64 a) { return zc64(-a.x, -a.y); }
+__host__ __device__ inline zc64 &operator+=(zc64 &a, zc64 b) { return a = a + b; }
+// a / b, scaled by the larger of |b.x|, |b.y| (no spurious overflow)
+__host__ __device__ inline zc64 operator/(zc64 a, zc64 b) {
+    double s = fmax(fabs(b.x), fabs(b.y));
+    if (s == 0.0) s = 1.0;  // a zero divisor: the quotients below become infinite or NaN
+    const double br = b.x / s, bi = b.y / s, ar = a.x / s, ai = a.y / s;
+    const double den = br * br + bi * bi;
+    return zc64((ar * br + ai * bi) / den, (ai * br - ar * bi) / den);
+}
 template <typename T>
-void chol_block_ops(oxi_handle_s *h, const T *L, i64 ldl, i64 n, T *P1, T *P2);
+i64 tri_inverse_elems(i64 n);
 template <typename T>
-void chol_solve_ops(oxi_handle_s *h, const T *L, i64 ldl, i64 n, T *X, i64 ldx, i64 nrhs, int *d_err,
-                    const T *P1, const T *P2);
+void tri_inverses(oxi_handle_s *h, TriForm form, const T *A, i64 lda, i64 n, T *P0, T *P1);
+template <typename T>
+void tri_solves(oxi_handle_s *h, TriForm form, const T *A, i64 lda, i64 n, T *X, i64 ldx, i64 nrhs, int *err,
+                const T *P0, const T *P1);
 
 // getrf_rowmajor through the handle's graph cache (same shape, buffers and
 // options: replay; second occurrence: capture; otherwise direct launches).
@@ -377,13 +403,5 @@ template <typename T>
 void getrs_perm(oxi_handle_s *h, char trans, i64 n, i64 nrhs, const T *LU, i64 lda,
                 const int64_t *d_perm, T *B, i64 ldb, int *d_err);
 void perm_from_ipiv(const int64_t *ipiv, i64 q, i64 m, int64_t *perm);
-// L then U solves with ROW-major factors (W, ld), X column-major n x nrhs, in place.
-template <typename T>
-void lu_solve_rowmajor(oxi_handle_s *h, const T *W, i64 ld, i64 n, T *X, i64 ldx, i64 nrhs,
-                       int *d_err, const T *DinvL = nullptr, const T *DinvU = nullptr);
-// Inverses of the 64 x 64 diagonal blocks of L (unit) and U of row-major factors.
-template <typename T>
-void lu_block_inverses_rowmajor(oxi_handle_s *h, const T *W, i64 ld, i64 n, T *DinvL, T *DinvU);
-i64 lu_block_inverse_elems(i64 n);
 
 }  // namespace oxi

@@ -1,0 +1,702 @@
+// Triangular solves with up to 16 right-hand sides per launch (ldiv!, the
+// refinement's corrections, Cholesky's two solves).
+//
+// A triangle is taken in solve order: M(i, j) = a[i rs + j cs] is lower
+// triangular, an upper one being read from its last row and column with
+// negated strides.  Its rows form superblocks of SP = 256, each of NS = 8 strips
+// of ST = 32 rows.  For superblock B
+//     x_B = Inv_B (b_B - sum_{C < B} M(B, C) x_C),   Inv_B = M(B, B)^-1,
+// the inverses computed once per factor (k_tri_inv).  k_tri_solve is ONE launch
+// per triangle: a cluster of NS CTAs takes the next superblock from a ticket
+// (everything it waits on is already running), one strip per CTA.  Each CTA
+// accumulates its strip's products with the solved superblocks as they
+// appear, the strips meet at a cluster barrier and read each other's
+// right-hand sides through distributed shared memory, and each multiplies by
+// its strip of Inv_B and publishes its 32 rows.
+//
+// Bound: for one right-hand side of a large system the single pass over the
+// factor, otherwise the chain of superblocks: one hop through L2, one cluster
+// barrier and two 32 x SP products per SP rows.  Measured on one B200 against
+// the form it replaces (64-row blocks, a hop through L2 per block): see the
+// figures at trsv_pair.
+//
+// A solved value is its own flag: the exchange buffer starts as all-ones words
+// (one memset per launch pair, the tickets included), which no published value
+// equals, and a reader polls the data itself.
+#include <cooperative_groups.h>
+#include <algorithm>
+#include "oxi_internal.h"
+#include "tma_util.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace oxi {
+
+namespace {
+constexpr int ST = 32;
+// rows of a superblock: half as many for complex elements, whose inverse's strip
+// would not fit shared memory otherwise
+template <typename T> constexpr int SP_ = sizeof(T) == 16 ? 128 : 256;
+constexpr int INV_NT = 256;
+
+// One effective triangle in solve order.
+template <typename T>
+struct TriView {
+    const T *a;
+    i64 rs, cs;
+    int n;
+    int unit;  // unit diagonal, not stored
+    int rev;   // solve order runs from the last row to the first
+    int conj;  // complex elements conjugated
+};
+
+// c + a b
+__device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ zc64 mad(zc64 a, zc64 b, zc64 c) {
+    return zc64(fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y)));
+}
+__device__ __forceinline__ float shfl_xor(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ double shfl_xor(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ zc64 shfl_xor(zc64 v, int o) {
+    return zc64(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+__device__ __forceinline__ float conj_if(float v, int) { return v; }
+__device__ __forceinline__ double conj_if(double v, int) { return v; }
+__device__ __forceinline__ zc64 conj_if(zc64 v, int c) { return zc64(v.x, c ? -v.y : v.y); }
+
+template <typename T>
+TriView<T> tri_view(const T *A, i64 lda, i64 n, bool lower, bool unit, bool rowacc, bool conj = false) {
+    TriView<T> v{A, rowacc ? lda : 1, rowacc ? 1 : lda, (int)n, unit ? 1 : 0, lower ? 0 : 1, conj ? 1 : 0};
+    if (!lower) {
+        v.a = A + (n - 1) * (v.rs + v.cs);
+        v.rs = -v.rs;
+        v.cs = -v.cs;
+    }
+    return v;
+}
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// Strip s of every superblock's inverse, one CTA per strip and triangle: the
+// row strip Y of L^-1 solves Y L = E_s, from the diagonal to the left:
+// Y_s = L_ss^-1, Y_t = -(sum_{t < u <= s} Y_u L_ut) L_tt^-1, with the 32 x 32
+// diagonal inverses by substitution, one warp each, the column of a lane in its
+// registers.  Each block column's elements are requested before the products
+// of the one before it.  FP64 products run on the tensor cores, a 16 x 8 tile
+// per warp.  Written column by column, P[(strip * SP + c) * ST + r], zero to the
+// right of the diagonal; rows past n are those of the identity.  Bound: latency
+// of the block columns' steps (up to seven, each two barriers and a chain of
+// up to 64 DMMAs); both triangles of a factor are one launch.
+// ---------------------------------------------------------------------------
+template <typename T>
+struct TriInvSmem {
+    static constexpr int SP = SP_<T>, NS = SP / ST;
+    static constexpr int DP = ST + 4, YP = SP + 4;  // FP64: 4 modulo 16, no conflicts of a DMMA fragment's loads
+    T D[NS][ST][DP];
+    T L[(NS - 1) * ST][DP];
+    T Z[ST][DP];
+    T Y[ST][YP];
+};
+
+// out (32 x 32, this thread's four elements of row `row`, columns c4..) =
+// A (32 x K, pitch ap) B (K x 32, pitch bp)
+template <typename T>
+__device__ __forceinline__ void inv_product(const T *A, int ap, const T *B, int bp, int K, T *out, int op) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if constexpr (sizeof(T) == 8) {
+        const int m0 = (warp & 1) * 16, n0 = (warp >> 1) * 8, gid = lane >> 2, tig = lane & 3;
+        double c[2][4] = {};  // two chains of products
+#pragma unroll 4
+        for (int k = 0; k < K; k += 8) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int kc = k + 4 * h + tig;
+                const double a0 = A[(m0 + gid) * ap + kc], a1 = A[(m0 + gid + 8) * ap + kc], b = B[kc * bp + n0 + gid];
+                asm volatile(
+                    "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                    : "+d"(c[h][0]), "+d"(c[h][1]), "+d"(c[h][2]), "+d"(c[h][3])
+                    : "d"(a0), "d"(a1), "d"(b));
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            out[(m0 + gid + 8 * (e >> 1)) * op + n0 + 2 * tig + (e & 1)] = c[0][e] + c[1][e];
+    } else {
+        const int row = t >> 3, c4 = (t & 7) * 4;
+        T z[4] = {T(0), T(0), T(0), T(0)};
+        const T *y = A + row * ap;
+#pragma unroll 8
+        for (int k = 0; k < K; ++k) {
+            const T yv = y[k];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) z[u] = mad(yv, B[k * bp + c4 + u], z[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) out[row * op + c4 + u] = z[u];
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(INV_NT) k_tri_inv(const TriView<T> v0, const TriView<T> v1, T *__restrict__ P0,
+                                                    T *__restrict__ P1) {
+    constexpr int SP = SP_<T>, NS = SP / ST, DP = TriInvSmem<T>::DP, YP = TriInvSmem<T>::YP;
+    constexpr int PRE = (NS - 1) * ST * ST / INV_NT;
+    extern __shared__ __align__(16) unsigned char tri_smem[];
+    TriInvSmem<T> &S = *reinterpret_cast<TriInvSmem<T> *>(tri_smem);
+    const TriView<T> &v = blockIdx.y ? v1 : v0;
+    T *P = blockIdx.y ? P1 : P0;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int g = blockIdx.x, s = g % NS;
+    const i64 r0 = (i64)(g / NS) * SP;  // the superblock's first row
+    const bool rowacc = v.cs == 1 || v.cs == -1;
+    const T *base = v.a + r0 * (v.rs + v.cs);
+    const int nrow = (int)(v.n - r0 < SP ? v.n - r0 : SP);
+    // the elements below diagonal block b: K = (s - b) ST rows, ST columns
+    T pre[PRE];
+    auto place = [&](int q, int &i, int &j) {  // element q of this thread
+        const int e = t + INV_NT * q;
+        i = rowacc ? e / ST : (e / (ST * ST)) * ST + e % ST;
+        j = rowacc ? e % ST : (e / ST) % ST;
+    };
+    auto fetch = [&](int b) {
+#pragma unroll
+        for (int q = 0; q < PRE; ++q) {
+            int i, j;
+            place(q, i, j);
+            const int gi = (b + 1) * ST + i;
+            pre[q] = (i < (s - b) * ST && gi < nrow) ? base[gi * v.rs + (b * ST + j) * v.cs] : T(0);
+        }
+    };
+    if (s > 0) fetch(s - 1);
+    if (warp <= s) {
+        T(*D)[DP] = S.D[warp];
+        const int d0 = warp * ST;
+#pragma unroll
+        for (int e = 0; e < ST; ++e) {
+            const int i = rowacc ? e : lane, j = rowacc ? lane : e;
+            T x = i == j ? T(1) : T(0);
+            if (d0 + i < nrow && (j < i || (j == i && !v.unit))) x = conj_if(base[(d0 + i) * v.rs + (d0 + j) * v.cs], v.conj);
+            D[i][j] = x;
+        }
+        __syncwarp();
+        T x[ST];
+#pragma unroll
+        for (int i = 0; i < ST; ++i) x[i] = (i == lane) ? T(1) : T(0);
+#pragma unroll
+        for (int p = 0; p < ST; ++p) {
+            if (!v.unit) x[p] = x[p] / D[p][p];
+#pragma unroll
+            for (int i = p + 1; i < ST; ++i) x[i] = mad(-D[i][p], x[p], x[i]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < ST; ++i) D[i][lane] = x[i];
+    }
+    __syncthreads();
+    for (int e = t; e < ST * SP; e += INV_NT) {
+        const int r = e / SP, c = e % SP;
+        S.Y[r][c] = (c / ST == s) ? S.D[s][r][c % ST] : T(0);
+    }
+    for (int b = s - 1; b >= 0; --b) {
+        const int K = (s - b) * ST;  // rows of the block column below its diagonal block
+#pragma unroll
+        for (int q = 0; q < PRE; ++q) {
+            int i, j;
+            place(q, i, j);
+            if (i < K) S.L[i][j] = conj_if(pre[q], v.conj);
+        }
+        __syncthreads();
+        if (b > 0) fetch(b - 1);
+        inv_product<T>(&S.Y[0][(b + 1) * ST], YP, &S.L[0][0], DP, K, &S.Z[0][0], DP);
+        __syncthreads();
+        inv_product<T>(&S.Z[0][0], DP, &S.D[b][0][0], DP, ST, &S.Y[0][b * ST], YP);
+        __syncthreads();
+        for (int e = t; e < ST * ST; e += INV_NT) {
+            T &y = S.Y[e / ST][b * ST + e % ST];
+            y = -y;
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    T *Pg = P + (i64)g * SP * ST;
+#pragma unroll 4
+    for (int e = t; e < SP * ST; e += INV_NT) Pg[e] = S.Y[e % ST][e / ST];
+}
+
+// ---------------------------------------------------------------------------
+// The solve.  ROWACC: the factor's unit stride runs along M's rows.
+// ---------------------------------------------------------------------------
+// An exchange word: the value's bits; all ones means "not there yet", and a
+// value that has those bits (a NaN) is published as another NaN.
+template <typename T>
+struct ExchWord {  // double, and complex as two words
+    using U = unsigned long long;
+    static constexpr int W = (int)(sizeof(T) / sizeof(U));
+    static __device__ __forceinline__ U load(const U *p) {
+        U v;
+        asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+        return v;
+    }
+    static __device__ __forceinline__ void load2(const U *p, U &a, U &b) {
+        asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+    }
+    static __device__ __forceinline__ U bits1(double v) {
+        const U u = (U)__double_as_longlong(v);
+        return u == ~U(0) ? u ^ 1u : u;
+    }
+    static __device__ __forceinline__ T value(const U *u) {
+        if constexpr (W == 2) return T(__longlong_as_double((long long)u[0]), __longlong_as_double((long long)u[1]));
+        else return __longlong_as_double((long long)u[0]);
+    }
+    static __device__ __forceinline__ void publish(U *p, T v) {
+        if constexpr (W == 2) {
+            *(volatile U *)p = bits1(v.x);
+            *(volatile U *)(p + 1) = bits1(v.y);
+        } else {
+            *(volatile U *)p = bits1(v);
+        }
+    }
+};
+template <> struct ExchWord<float> {
+    using U = unsigned int;
+    static constexpr int W = 1;
+    static __device__ __forceinline__ U load(const U *p) {
+        U v;
+        asm volatile("ld.volatile.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+        return v;
+    }
+    static __device__ __forceinline__ void load2(const U *p, U &a, U &b) {
+        asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "l"(p) : "memory");
+    }
+    static __device__ __forceinline__ float value(const U *u) { return __uint_as_float(u[0]); }
+    static __device__ __forceinline__ void publish(U *p, float v) {
+        const U u = __float_as_uint(v);
+        *(volatile U *)p = u == ~U(0) ? u ^ 1u : u;
+    }
+};
+
+// Sum V values over the 32 lanes by halving: V - 1 exchanges for V <= 32, and
+// lane l ends with the sums of value indexes lane_value(l) .. + max(V / 32, 1).
+template <typename T, int V, int OFF>
+__device__ __forceinline__ void lane_sums(T (&a)[V], int lane) {
+    if constexpr (OFF > 0) {
+        if constexpr (V > 1) {
+            constexpr int HV = V / 2;
+            const bool up = lane & OFF;
+            T h[HV];
+#pragma unroll
+            for (int i = 0; i < HV; ++i) {
+                const T send = up ? a[i] : a[i + HV], keep = up ? a[i + HV] : a[i];
+                h[i] = keep + shfl_xor(send, OFF);
+            }
+            lane_sums<T, HV, OFF / 2>(h, lane);
+#pragma unroll
+            for (int i = 0; i < HV; ++i) a[i] = h[i];
+        } else {
+            a[0] += shfl_xor(a[0], OFF);
+            lane_sums<T, 1, OFF / 2>(a, lane);
+        }
+    }
+}
+template <int V>
+__device__ __forceinline__ int lane_value(int lane) {
+    int idx = 0;
+#pragma unroll
+    for (int h = V / 2, off = 16; h >= 1 && off > 0; h /= 2, off /= 2) idx += (lane & off) ? h : 0;
+    return idx;
+}
+
+// NR values of one row: 16-byte accesses where they fill one
+template <typename T, int NR>
+__device__ __forceinline__ void get_row(T (&v)[NR], const T *p) {
+    constexpr int VEC = 16 / (int)sizeof(T);
+    if constexpr (NR % VEC == 0 && VEC > 1) {
+#pragma unroll
+        for (int k = 0; k < NR; k += VEC) {
+            const int4 x = *reinterpret_cast<const int4 *>(p + k);
+            const T *xx = reinterpret_cast<const T *>(&x);
+#pragma unroll
+            for (int u = 0; u < VEC; ++u) v[k + u] = xx[u];
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < NR; ++k) v[k] = p[k];
+    }
+}
+template <typename T, int NR>
+__device__ __forceinline__ void put_row(T *p, const T (&v)[NR]) {
+    constexpr int VEC = 16 / (int)sizeof(T);
+    if constexpr (NR % VEC == 0 && VEC > 1) {
+#pragma unroll
+        for (int k = 0; k < NR; k += VEC) {
+            int4 x;
+            T *xx = reinterpret_cast<T *>(&x);
+#pragma unroll
+            for (int u = 0; u < VEC; ++u) xx[u] = v[k + u];
+            *reinterpret_cast<int4 *>(p + k) = x;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < NR; ++k) p[k] = v[k];
+    }
+}
+
+template <typename T, int NR>
+struct TriSolveSmem {
+    static constexpr int SP = SP_<T>, NS = SP / ST;
+    // pitch of a row's values: 16 bytes more keep eight lanes' 16-byte reads of
+    // eight rows free of bank conflicts
+    static constexpr int XP = NR * (int)sizeof(T) >= 32 ? NR + 16 / (int)sizeof(T) : NR;
+    T inv[SP][ST];       // this strip of the superblock's inverse, by columns
+    T xs[2][SP * XP];    // solved values being multiplied, double-buffered
+    T part[NS][NR][ST];  // per-warp partial sums
+    T r[ST][NR];         // the strip's right-hand side, read by the other strips
+};
+
+template <typename T, bool ROWACC, int NR>
+__global__ void __cluster_dims__(SP_<T> / ST, 1, 1) __launch_bounds__(SP_<T>, 1)
+k_tri_solve(const TriView<T> v, const T *__restrict__ P, T *__restrict__ X, i64 ldx, int *__restrict__ ticket,
+            typename ExchWord<T>::U *__restrict__ exch, int *__restrict__ err) {
+    using EW = ExchWord<T>;
+    using U = typename EW::U;
+    constexpr int SP = SP_<T>, NS = SP / ST, TRI_NT = SP, TW = EW::W;
+    constexpr int RPW = ST / NS, CPL = SP / 32;  // ROWACC: rows per warp, columns per lane
+    // the next tile is loaded ahead where two fit the registers
+    constexpr bool AHEAD = sizeof(T) <= 8;
+    constexpr int XP = TriSolveSmem<T, NR>::XP;
+    extern __shared__ __align__(16) unsigned char tri_smem[];
+    TriSolveSmem<T, NR> &S = *reinterpret_cast<TriSolveSmem<T, NR> *>(tri_smem);
+    __shared__ int s_blk;
+    cg::cluster_group cl = cg::this_cluster();
+    const int s = (int)cl.block_rank();
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int n = v.n, nsb = (n + SP - 1) / SP;
+    // the ticket counts from -1 (cleared with the exchange words); an aborted call takes no block
+    if (s == 0 && t == 0) s_blk = aborted(err) ? nsb : atomicAdd(ticket, 1) + 1;
+    cl.sync();
+    const int B = *cl.map_shared_rank(&s_blk, 0);
+    if (B >= nsb) {
+        cl.sync();
+        return;
+    }
+    const int g = B * NS + s;
+    const i64 r0 = (i64)B * SP + s * ST;
+    const int rows = (int)(n - r0 < 0 ? 0 : (n - r0 < ST ? n - r0 : ST));
+
+    // ---- no dependency on other superblocks: the inverse's strip, the right-hand side ----
+    if (warp <= s && rows > 0) {
+        const T *Pg = P + (i64)g * SP * ST;
+#pragma unroll
+        for (int c = 0; c < ST; ++c) S.inv[warp * ST + c][lane] = Pg[(warp * ST + c) * ST + lane];
+    }
+    constexpr int V = ROWACC ? RPW * NR : NR;             // accumulators per lane
+    constexpr int OUT = (ST * NR + TRI_NT - 1) / TRI_NT;  // outputs per thread
+    // outputs of the first product: (row, rhs) of thread t's q-th value
+    auto r_out = [&](int q, int &row, int &k) -> bool {
+        if constexpr (ROWACC) {
+            const int idx = lane_value<V>(lane) + q;
+            row = warp * RPW + idx / NR;
+            k = idx % NR;
+            return V >= 32 || (lane & (32 / (V < 32 ? V : 32) - 1)) == 0;
+        } else {
+            const int o = t + TRI_NT * q;
+            row = o % ST;
+            k = o / ST;
+            return o < ST * NR;
+        }
+    };
+    auto xrow = [&](i64 i) -> i64 { return v.rev ? n - 1 - i : i; };
+    T bv[OUT];
+#pragma unroll
+    for (int q = 0; q < OUT; ++q) {
+        int row, k;
+        bv[q] = T(0);
+        if (r_out(q, row, k) && row < rows) bv[q] = X[xrow(r0 + row) + (i64)k * ldx];
+    }
+
+    // ---- products with the superblocks before this one ----
+    T acc[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[i] = T(0);
+    auto load_tile = [&](int C, T (&a)[32]) {
+        const i64 c0 = (i64)C * SP;
+        if constexpr (ROWACC) {
+#pragma unroll
+            for (int i = 0; i < RPW; ++i) {
+                const int row = warp * RPW + i;
+                const T *p = v.a + (r0 + row) * v.rs + (c0 + lane) * v.cs;
+#pragma unroll
+                for (int u = 0; u < CPL; ++u) a[i * CPL + u] = row < rows ? conj_if(p[32 * u * v.cs], v.conj) : T(0);
+            }
+        } else {
+            const T *p = v.a + (r0 + lane) * v.rs + (c0 + warp * ST) * v.cs;
+#pragma unroll
+            for (int c = 0; c < 32; ++c) a[c] = lane < rows ? conj_if(p[c * v.cs], v.conj) : T(0);
+        }
+    };
+    U xw[NR * TW];
+    const U *myx = exch + (i64)t * (NR * TW);
+    auto load_x = [&](int C) {
+        const U *p = myx + (i64)C * SP * (NR * TW);
+        if constexpr (NR * TW == 1) {
+            xw[0] = EW::load(p);
+        } else {
+#pragma unroll
+            for (int k = 0; k < NR * TW; k += 2) EW::load2(p + k, xw[k], xw[k + 1]);
+        }
+    };
+    auto x_ready = [&]() -> bool {
+        bool ok = true;
+#pragma unroll
+        for (int k = 0; k < NR * TW; ++k) ok = ok && xw[k] != ~U(0);
+        return ok;
+    };
+    auto step = [&](int C, T (&a)[32], T (&next)[32]) {
+        if (!AHEAD) {
+            load_tile(C, a);
+            load_x(C);
+        }
+        if (!x_ready()) {
+            const uint64_t t0 = global_ns();
+            uint32_t it = 0;
+            for (;;) {
+                load_x(C);
+                if (x_ready()) break;
+                if (spin_give_up<256>(it, t0, err, 3)) break;
+            }
+        }
+        T *xs = S.xs[C & 1];
+        {
+            T x[NR];
+#pragma unroll
+            for (int k = 0; k < NR; ++k) x[k] = EW::value(xw + k * TW);
+            put_row<T, NR>(xs + t * XP, x);
+        }
+        if (AHEAD && C + 1 < B) {
+            load_tile(C + 1, next);
+            load_x(C + 1);
+        }
+        if constexpr (ROWACC) {
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < CPL; ++u) {
+                T x[NR];
+                get_row<T, NR>(x, xs + (lane + 32 * u) * XP);
+#pragma unroll
+                for (int k = 0; k < NR; ++k)
+#pragma unroll
+                    for (int i = 0; i < RPW; ++i) acc[i * NR + k] = mad(a[i * CPL + u], x[k], acc[i * NR + k]);
+            }
+        } else {
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 32; ++c) {
+                T x[NR];
+                get_row<T, NR>(x, xs + (warp * ST + c) * XP);
+#pragma unroll
+                for (int k = 0; k < NR; ++k) acc[k] = mad(a[c], x[k], acc[k]);
+            }
+            __syncwarp();
+        }
+    };
+    if (B > 0 && rows > 0) {
+        T a0[32];
+        if constexpr (AHEAD) {
+            T a1[32];
+            load_tile(0, a0);
+            load_x(0);
+            for (int C = 0; C < B; C += 2) {
+                step(C, a0, a1);
+                if (C + 1 < B) step(C + 1, a1, a0);
+            }
+        } else {
+            for (int C = 0; C < B; ++C) step(C, a0, a0);
+        }
+    }
+    // ---- the strip's right-hand side, to the whole superblock ----
+    if constexpr (ROWACC) {
+        lane_sums<T, V, 16>(acc, lane);
+    } else {
+#pragma unroll
+        for (int k = 0; k < NR; ++k) S.part[warp][k][lane] = acc[k];
+        __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < OUT; ++q) {
+        int row, k;
+        if (r_out(q, row, k)) {
+            T sum;
+            if constexpr (ROWACC) {
+                sum = acc[q < V ? q : 0];
+            } else {
+                sum = T(0);
+#pragma unroll
+                for (int w = 0; w < NS; ++w) sum += S.part[w][k][row];
+            }
+            S.r[row][k] = bv[q] - sum;
+        }
+    }
+    cl.sync();
+
+    // ---- x = Inv r: warp w takes strip w's 32 columns, a lane one row ----
+    T o[NR];
+#pragma unroll
+    for (int k = 0; k < NR; ++k) o[k] = T(0);
+    if (warp <= s && rows > 0) {
+        const T *rr = cl.map_shared_rank(&S.r[0][0], warp) + lane * NR;
+        T *xs = S.xs[0];
+        {
+            T x[NR];
+            get_row<T, NR>(x, rr);
+            put_row<T, NR>(xs + t * XP, x);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < ST; ++c) {
+            const T iv = S.inv[warp * ST + c][lane];
+            T x[NR];
+            get_row<T, NR>(x, xs + (warp * ST + c) * XP);
+#pragma unroll
+            for (int k = 0; k < NR; ++k) o[k] = mad(iv, x[k], o[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NR; ++k) S.part[warp][k][lane] = o[k];
+    __syncthreads();
+    for (int e = t; e < ST * NR; e += TRI_NT) {
+        const int row = e / NR, k = e % NR;
+        T x = T(0);
+#pragma unroll
+        for (int w = 0; w < NS; ++w) x += S.part[w][k][row];
+        if (row < rows) {
+            EW::publish(exch + ((r0 + row) * NR + k) * TW, x);
+            X[xrow(r0 + row) + (i64)k * ldx] = x;
+        }
+    }
+    cl.sync();  // the other strips have read this one's right-hand side
+}
+
+template <typename T>
+i64 tri_inverse_elems(i64 n) {
+    return (n + SP_<T> - 1) / SP_<T> * SP_<T> * (i64)SP_<T>;
+}
+template i64 tri_inverse_elems<float>(i64);
+template i64 tri_inverse_elems<double>(i64);
+template i64 tri_inverse_elems<zc64>(i64);
+
+// Exchange words and tickets of one launch pair: a ticket per triangle, then
+// their words.
+template <typename T>
+static i64 exch_words(i64 n, int nr) {
+    return (n + SP_<T> - 1) / SP_<T> * SP_<T> * (i64)nr * ExchWord<T>::W;
+}
+
+template <typename T>
+static void tri_inv_launch(const TriView<T> &v0, const TriView<T> &v1, T *P0, T *P1, cudaStream_t s) {
+    const int smem = (int)sizeof(TriInvSmem<T>);
+    set_max_dyn_smem((const void *)k_tri_inv<T>, smem);
+    const unsigned strips = (unsigned)((v0.n + ST - 1) / ST);
+    constexpr double SP = SP_<T>;
+    ProfScope ps(KC_TRSV, s, 2.0 * 2.0 * v0.n * SP * SP / 3.0, 2.0 * (double)v0.n * SP * 1.5 * sizeof(T));
+    k_tri_inv<T><<<dim3(strips, 2), INV_NT, smem, s>>>(v0, v1, P0, P1);
+    OXI_LAUNCH_CHECK();
+}
+
+// First triangle, then the second, on X (n x nrhs, in place), by chunks of right-hand
+// sides.  Measured on one B200 (us for the pair of solves, before -> now):
+template <typename T, bool ROWACC0, bool ROWACC1>
+static void trsv_pair(oxi_handle_s *h, const TriView<T> &v0, const TriView<T> &v1, const T *P0, const T *P1, T *X,
+                      i64 ldx, i64 nrhs, int *err) {
+    using U = typename ExchWord<T>::U;
+    cudaStream_t s = h->stream;
+    const i64 n = v0.n;
+    constexpr int SP = SP_<T>, TRI_NT = SP;
+    const unsigned grid = (unsigned)((n + SP - 1) / SP * (SP / ST));
+    constexpr int NRX = sizeof(T) == 4 ? 16 : (sizeof(T) == 8 ? 8 : 4);
+    for (i64 k0 = 0; k0 < nrhs;) {
+        const i64 left = nrhs - k0;
+        const int nr = left >= 16 && NRX == 16 ? 16 : left >= 8 && NRX >= 8 ? 8 : left >= 4 ? 4 : left >= 2 ? 2 : 1;
+        const size_t words = (size_t)exch_words<T>(n, nr);
+        const size_t bytes = 256 + 2 * words * sizeof(U);
+        char *ws = (char *)h->xtag_ws.get(256 + 2 * (size_t)exch_words<T>(n, NRX) * sizeof(U));
+        int *tickets = (int *)ws;
+        U *e0 = (U *)(ws + 256), *e1 = e0 + words;
+        ProfScope ps(KC_TRSV, s, 2.0 * (double)n * n * nr, (double)n * n * sizeof(T));
+        OXI_CUDA(cudaMemsetAsync(ws, 0xff, bytes, s));
+        T *Xk = X + k0 * ldx;
+#define OXI_TRI_GO(NRV)                                                                                   \
+    do {                                                                                                  \
+        const int smem = (int)sizeof(TriSolveSmem<T, NRV>);                                               \
+        set_max_dyn_smem((const void *)k_tri_solve<T, ROWACC0, NRV>, smem);                               \
+        set_max_dyn_smem((const void *)k_tri_solve<T, ROWACC1, NRV>, smem);                               \
+        k_tri_solve<T, ROWACC0, NRV><<<grid, TRI_NT, smem, s>>>(v0, P0, Xk, ldx, tickets, e0, err);       \
+        OXI_LAUNCH_CHECK();                                                                               \
+        k_tri_solve<T, ROWACC1, NRV><<<grid, TRI_NT, smem, s>>>(v1, P1, Xk, ldx, tickets + 1, e1, err);   \
+        OXI_LAUNCH_CHECK();                                                                               \
+    } while (0)
+        if constexpr (NRX == 16) {
+            if (nr == 16) OXI_TRI_GO(16);
+        }
+        if constexpr (NRX >= 8) {
+            if (nr == 8) OXI_TRI_GO(8);
+        }
+        if (nr == 4) OXI_TRI_GO(4);
+        else if (nr == 2) OXI_TRI_GO(2);
+        else if (nr == 1) OXI_TRI_GO(1);
+#undef OXI_TRI_GO
+        k0 += nr;
+    }
+}
+
+// The four forms: LU solves with a column-major factor (N: L, U; T: U^T, L^T),
+// with a row-major one, and the two solves of a column-major lower Cholesky factor.
+template <typename T>
+static void tri_views(TriForm form, const T *A, i64 lda, i64 n, TriView<T> &v0, TriView<T> &v1) {
+    switch (form) {
+    case TriForm::LU_N:
+        v0 = tri_view(A, lda, n, true, true, false);
+        v1 = tri_view(A, lda, n, false, false, false);
+        break;
+    case TriForm::LU_T:
+    case TriForm::LU_C:
+        v0 = tri_view(A, lda, n, true, false, true, form == TriForm::LU_C);
+        v1 = tri_view(A, lda, n, false, true, true, form == TriForm::LU_C);
+        break;
+    case TriForm::LU_ROWMAJOR:
+        v0 = tri_view(A, lda, n, true, true, true);
+        v1 = tri_view(A, lda, n, false, false, true);
+        break;
+    case TriForm::CHOLESKY:
+        v0 = tri_view(A, lda, n, true, false, false);
+        v1 = tri_view(A, lda, n, false, false, true);
+        break;
+    }
+}
+
+template <typename T>
+void tri_inverses(oxi_handle_s *h, TriForm form, const T *A, i64 lda, i64 n, T *P0, T *P1) {
+    TriView<T> v0, v1;
+    tri_views(form, A, lda, n, v0, v1);
+    tri_inv_launch<T>(v0, v1, P0, P1, h->stream);
+}
+template <typename T>
+void tri_solves(oxi_handle_s *h, TriForm form, const T *A, i64 lda, i64 n, T *X, i64 ldx, i64 nrhs, int *err,
+                const T *P0, const T *P1) {
+    TriView<T> v0, v1;
+    tri_views(form, A, lda, n, v0, v1);
+    if (form == TriForm::LU_N) trsv_pair<T, false, false>(h, v0, v1, P0, P1, X, ldx, nrhs, err);
+    else if (form == TriForm::CHOLESKY) trsv_pair<T, false, true>(h, v0, v1, P0, P1, X, ldx, nrhs, err);
+    else trsv_pair<T, true, true>(h, v0, v1, P0, P1, X, ldx, nrhs, err);
+}
+template void tri_inverses<zc64>(oxi_handle_s *, TriForm, const zc64 *, i64, i64, zc64 *, zc64 *);
+template void tri_solves<zc64>(oxi_handle_s *, TriForm, const zc64 *, i64, i64, zc64 *, i64, i64, int *, const zc64 *,
+                               const zc64 *);
+template void tri_inverses<float>(oxi_handle_s *, TriForm, const float *, i64, i64, float *, float *);
+template void tri_inverses<double>(oxi_handle_s *, TriForm, const double *, i64, i64, double *, double *);
+template void tri_solves<float>(oxi_handle_s *, TriForm, const float *, i64, i64, float *, i64, i64, int *,
+                                const float *, const float *);
+template void tri_solves<double>(oxi_handle_s *, TriForm, const double *, i64, i64, double *, i64, i64, int *,
+                                 const double *, const double *);
+
+}  // namespace oxi

@@ -40,15 +40,6 @@ __device__ __forceinline__ zd zmul(zd a, zd b) { return {a.r * b.r - a.i * b.i, 
 __device__ __forceinline__ zd zmsub(zd c, zd a, zd b) {
     return {c.r - (a.r * b.r - a.i * b.i), c.i - (a.r * b.i + a.i * b.r)};
 }
-// a / b, scaled by the larger of |b.r|, |b.i| (no spurious overflow)
-__device__ __forceinline__ zd zdivd(zd a, zd b) {
-    double s = fmax(fabs(b.r), fabs(b.i));
-    if (s == 0.0) s = 1.0;  // a zero divisor: the quotients below become infinite or NaN
-    const double br = b.r / s, bi = b.i / s, ar = a.r / s, ai = a.i / s;
-    const double den = br * br + bi * bi;
-    return {(ar * br + ai * bi) / den, (ai * br - ar * bi) / den};
-}
-
 // 1 / b, scaled by the larger of |b.r|, |b.i| (no spurious overflow)
 __device__ __forceinline__ zd zrecip(zd b) {
     double s = fmax(fabs(b.r), fabs(b.i));
@@ -550,142 +541,6 @@ static void zgetrf_planes(ZRun &R) {
     }
 }
 
-// ---- solves: one CTA per right-hand side, the substitutions row by row with
-// a CTA-wide dot product per row (factor rows are contiguous in column-major
-// only along columns, so each dot product reads one row of the triangle) ----
-__device__ __forceinline__ zd cta_sum(zd v, zd *s_buf) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int off = 16; off > 0; off >>= 1) {
-        v.r += __shfl_xor_sync(0xffffffffu, v.r, off);
-        v.i += __shfl_xor_sync(0xffffffffu, v.i, off);
-    }
-    if (lane == 0) s_buf[warp] = v;
-    __syncthreads();
-    zd t = {0.0, 0.0};
-    if (threadIdx.x == 0)
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { t.r += s_buf[w].r; t.i += s_buf[w].i; }
-    __syncthreads();
-    return t;  // valid in thread 0
-}
-
-// x <- op(T)^-1 x for the n x n factor LU (interleaved column-major):
-// lower (unit L) or upper (U), op = none / transpose / conjugate transpose.
-__global__ void __launch_bounds__(256) k_ztrsv(const double2 *__restrict__ LU, i64 lda, double2 *__restrict__ X,
-                                               i64 ldx, int n, int lower_solve, int unit, int transposed,
-                                               int conjugate) {
-    __shared__ zd s_buf[8];
-    double2 *x = X + (i64)blockIdx.x * ldx;
-    for (int step = 0; step < n; ++step) {
-        const int i = lower_solve ? step : n - 1 - step;
-        zd acc = {0.0, 0.0};
-        const int p0 = lower_solve ? 0 : i + 1, p1 = lower_solve ? i : n;
-        for (int p = p0 + threadIdx.x; p < p1; p += 256) {
-            const double2 a2 = transposed ? LU[p + (i64)i * lda] : LU[i + (i64)p * lda];
-            const zd a = {a2.x, conjugate ? -a2.y : a2.y};
-            const double2 xp = x[p];
-            const zd pr = zmul(a, {xp.x, xp.y});
-            acc.r += pr.r;
-            acc.i += pr.i;
-        }
-        acc = cta_sum(acc, s_buf);
-        if (threadIdx.x == 0) {
-            const double2 b = x[i];
-            zd v = {b.x - acc.r, b.y - acc.i};
-            if (!unit) {
-                const double2 d2 = LU[i + (i64)i * lda];
-                v = zdivd(v, {d2.x, conjugate ? -d2.y : d2.y});
-            }
-            x[i] = make_double2(v.r, v.i);
-        }
-        __syncthreads();
-    }
-}
-
-// x <- T^-1 x for the untransposed factors, column by column with x in shared
-// memory: the forward unit-lower solve (x_i -= l_ij x_j for i > j once x_j is
-// final) or the backward upper one (x_j /= u_jj, then x_i -= u_ij x_j for
-// i < j).  Each step reads one column of the factor, contiguous in memory.
-// One CTA per right-hand side; n <= ZCOLS_MAXN.
-constexpr int ZCOLS_NT = 512;
-constexpr int ZCOLS_MAXN = 12288;
-__global__ void __launch_bounds__(ZCOLS_NT) k_ztrsv_cols(const double2 *__restrict__ LU, i64 lda,
-                                                         double2 *__restrict__ X, i64 ldx, int n, int lower) {
-    // a step's column entries for this thread are loaded together into
-    // registers before any is used: one global latency per step, not one per row
-    constexpr int PER = ZCOLS_MAXN / ZCOLS_NT;
-    extern __shared__ double2 zx[];
-    double2 *x = X + (i64)blockIdx.x * ldx;
-    const int tid = threadIdx.x;
-    for (int i = tid; i < n; i += ZCOLS_NT) zx[i] = x[i];
-    __syncthreads();
-    double2 cv[PER];
-    if (lower) {
-        for (int j = 0; j < n - 1; ++j) {
-            const double2 *col = LU + (i64)j * lda;
-#pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int i = j + 1 + tid + q * ZCOLS_NT;
-                if (i < n) cv[q] = col[i];
-            }
-            const double2 xv = zx[j];
-            const zd xj = {xv.x, xv.y};
-#pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int i = j + 1 + tid + q * ZCOLS_NT;
-                if (i < n) {
-                    const double2 b = zx[i];
-                    const zd v = zmsub({b.x, b.y}, {cv[q].x, cv[q].y}, xj);
-                    zx[i] = make_double2(v.r, v.i);
-                }
-            }
-            __syncthreads();
-        }
-        for (int i = tid; i < n; i += ZCOLS_NT) x[i] = zx[i];
-    } else {
-        // zx[j] is not written in step j (every thread divides it for itself),
-        // and not read after it: the solution goes straight to x[j]
-        for (int j = n - 1; j >= 0; --j) {
-            const double2 *col = LU + (i64)j * lda;
-#pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int i = tid + q * ZCOLS_NT;
-                if (i < j) cv[q] = col[i];
-            }
-            const double2 xv = zx[j], d = col[j];
-            const zd xj = zdivd({xv.x, xv.y}, {d.x, d.y});
-#pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int i = tid + q * ZCOLS_NT;
-                if (i < j) {
-                    const double2 b = zx[i];
-                    const zd v = zmsub({b.x, b.y}, {cv[q].x, cv[q].y}, xj);
-                    zx[i] = make_double2(v.r, v.i);
-                }
-            }
-            if (tid == 0) x[j] = make_double2(xj.r, xj.i);
-            __syncthreads();
-        }
-    }
-}
-
-// the interchanges on the columns of X: forward (before the 'N' solves) or in
-// reverse (after the 'T' / 'C' solves), one thread per right-hand side
-__global__ void k_zperm(double2 *__restrict__ X, i64 ldx, int n, int nrhs, const int64_t *__restrict__ ipiv,
-                        int reverse) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nrhs) return;
-    double2 *x = X + (i64)c * ldx;
-    for (int s = 0; s < n; ++s) {
-        const int j = reverse ? n - 1 - s : s;
-        const int p = (int)ipiv[j] - 1;
-        if (p != j) {
-            const double2 t = x[j];
-            x[j] = x[p];
-            x[p] = t;
-        }
-    }
-}
-
 }  // namespace oxi
 
 extern "C" int oxi_zgetrf(oxi_handle_t h, int64_t m, int64_t n, void *dA, int64_t lda, int64_t *d_ipiv,
@@ -721,65 +576,6 @@ extern "C" int oxi_zgetrf(oxi_handle_t h, int64_t m, int64_t n, void *dA, int64_
         const int we = check_abort(h, (const int *)(hi + 2));
         if (we != OXI_OK) return we;
         return hi[0] > 0 ? OXI_ESINGULAR : OXI_OK;
-    } catch (const CudaError &e) {
-        h->last_error = std::string(e.what) + ": " + cudaGetErrorString(e.code);
-        return OXI_ECUDA;
-    }
-}
-
-extern "C" int oxi_zgetrs(oxi_handle_t h, char trans, int64_t n, int64_t nrhs, const void *dLU, int64_t lda,
-                          const int64_t *d_ipiv, void *dB, int64_t ldb) {
-    using namespace oxi;
-    if (!h) return OXI_EINVAL;
-    if (trans != 'N' && trans != 'T' && trans != 'C') return OXI_EINVAL;
-    if (n < 0 || nrhs < 0 || lda < std::max<int64_t>(1, n) || ldb < std::max<int64_t>(1, n)) return OXI_EINVAL;
-    if (n == 0 || nrhs == 0) return OXI_OK;
-    if (!dLU || !d_ipiv || !dB || n >= (1ll << 31) || nrhs >= (1ll << 31)) return OXI_EINVAL;
-    if ((uintptr_t)dLU % 16 || (uintptr_t)dB % 16) return OXI_EINVAL;
-    try {
-        ProfGuard pg(&h->prof);
-        OXI_CUDA(cudaSetDevice(h->device));
-        AbortScope ab(h);
-        // the pivots are validated on the host (one copy of n entries)
-        std::vector<int64_t> ip(n);
-        OXI_CUDA(cudaMemcpyAsync(ip.data(), d_ipiv, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, h->stream));
-        OXI_CUDA(cudaStreamSynchronize(h->stream));
-        for (i64 j = 0; j < n; ++j)
-            if (ip[j] < 1 || ip[j] > n) return OXI_EINVAL;
-        cudaStream_t s = h->stream;
-        const double2 *LU = (const double2 *)dLU;
-        double2 *X = (double2 *)dB;
-        const unsigned gp = (unsigned)((nrhs + 127) / 128);
-        if (trans == 'N') {
-            k_zperm<<<gp, 128, 0, s>>>(X, ldb, (int)n, (int)nrhs, d_ipiv, 0);
-            OXI_LAUNCH_CHECK();
-            if (n <= ZCOLS_MAXN) {
-                const int smem = (int)(sizeof(double2) * n);
-                set_max_dyn_smem((const void *)k_ztrsv_cols, (int)(sizeof(double2) * ZCOLS_MAXN));
-                k_ztrsv_cols<<<(unsigned)nrhs, ZCOLS_NT, smem, s>>>(LU, lda, X, ldb, (int)n, 1);
-                OXI_LAUNCH_CHECK();
-                k_ztrsv_cols<<<(unsigned)nrhs, ZCOLS_NT, smem, s>>>(LU, lda, X, ldb, (int)n, 0);
-                OXI_LAUNCH_CHECK();
-            } else {
-                k_ztrsv<<<(unsigned)nrhs, 256, 0, s>>>(LU, lda, X, ldb, (int)n, 1, 1, 0, 0);
-                OXI_LAUNCH_CHECK();
-                k_ztrsv<<<(unsigned)nrhs, 256, 0, s>>>(LU, lda, X, ldb, (int)n, 0, 0, 0, 0);
-                OXI_LAUNCH_CHECK();
-            }
-        } else {
-            const int cj = trans == 'C';
-            // U^T (U^H) is lower, non-unit; L^T (L^H) upper, unit
-            k_ztrsv<<<(unsigned)nrhs, 256, 0, s>>>(LU, lda, X, ldb, (int)n, 1, 0, 1, cj);
-            OXI_LAUNCH_CHECK();
-            k_ztrsv<<<(unsigned)nrhs, 256, 0, s>>>(LU, lda, X, ldb, (int)n, 0, 1, 1, cj);
-            OXI_LAUNCH_CHECK();
-            k_zperm<<<gp, 128, 0, s>>>(X, ldb, (int)n, (int)nrhs, d_ipiv, 1);
-            OXI_LAUNCH_CHECK();
-        }
-        int *he = (int *)h->host_ws.get(64);
-        queue_abort_read(h, he);
-        OXI_CUDA(cudaStreamSynchronize(s));
-        return check_abort(h, he);
     } catch (const CudaError &e) {
         h->last_error = std::string(e.what) + ": " + cudaGetErrorString(e.code);
         return OXI_ECUDA;
