@@ -1127,81 +1127,93 @@ static void trsm_steps_rec(int a, int b, TrsmSteps &st) {
 }
 
 constexpr int TR_TMAX = 128;
+constexpr int TR_LP = TR_TMAX + 1;  // row pitch of the staged triangle
 
-template <int CW>
+// Bound: latency of the steps, each a barrier, the operands' shared-memory
+// loads and one chain of up to 64 dependent FP64 FMAs (31 steps, about 7000
+// cycles at t = 128).  The strict lower triangle of L is therefore staged in
+// shared memory once per CTA, with everything in flight at once, instead of
+// being fetched through L1 in every step.
+template <int CW, int CPT>
 __global__ void __launch_bounds__(256) k_trsm_refo(const double *__restrict__ L, i64 ldl, double *__restrict__ B,
                                                    i64 ldb, int t, i64 N, const __grid_constant__ TrsmSteps st) {
-    // L is read through the L1 cache (threads of a warp that share a row read
-    // the same element: one broadcast load), the CTA's columns stay in shared
-    // memory: t x (CW + 1) doubles, several CTAs per SM.
     extern __shared__ __align__(16) double tr_smem[];
-    double *X = tr_smem;
-    constexpr int XP = CW + 1;
-    const int tid = threadIdx.x;
+    double *X = tr_smem;                          // t x CW
+    double *Ls = tr_smem + (size_t)t * CW;        // t x TR_LP, strict lower triangle
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const i64 c0 = (i64)blockIdx.x * CW;
     const int cols = (int)((N - c0) < CW ? (N - c0) : CW);
+    for (int i = warp; i < t; i += 8)
+        for (int p = lane; p < i; p += 32) {
+            const uint32_t dst = smem_u32(&Ls[i * TR_LP + p]);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(L + (i64)i * ldl + p) : "memory");
+        }
+#pragma unroll 4
     for (int e = tid; e < t * CW; e += 256) {
         const int i = e / CW, c = e - i * CW;
-        X[i * XP + c] = (c < cols) ? B[(i64)i * ldb + c0 + c] : 0.0;
+        X[i * CW + c] = (c < cols) ? B[(i64)i * ldb + c0 + c] : 0.0;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     for (int k = 0; k < st.count; ++k) {
         const int4 o = st.step[k];
         if (o.x == 0) {
-            // leaf of nl <= 8 rows: the column in registers, the triangle's
-            // loads all issued up front (fully unrolled, predicated)
+            // leaf of nl <= 8 rows, a column per thread: the triangle's loads all
+            // issued up front (fully unrolled, predicated)
             if (tid < CW) {
                 const int nl = o.z - o.y;
                 double xv[8], lv[8][8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    xv[u] = (u < nl) ? X[(o.y + u) * XP + tid] : 0.0;
+                    xv[u] = (u < nl) ? X[(o.y + u) * CW + tid] : 0.0;
 #pragma unroll
-                    for (int pp = 0; pp < u; ++pp)
-                        lv[u][pp] = (u < nl) ? __ldg(L + (i64)(o.y + u) * ldl + o.y + pp) : 0.0;
+                    for (int pp = 0; pp < u; ++pp) lv[u][pp] = (u < nl) ? Ls[(o.y + u) * TR_LP + o.y + pp] : 0.0;
                 }
 #pragma unroll
                 for (int u = 1; u < 8; ++u)
 #pragma unroll
                     for (int pp = 0; pp < u; ++pp) xv[u] = fma(-lv[u][pp], xv[pp], xv[u]);
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (u < nl) X[(o.y + u) * XP + tid] = xv[u];
+                for (int u = 1; u < 8; ++u)
+                    if (u < nl) X[(o.y + u) * CW + tid] = xv[u];
             }
         } else {
-            // rows [o.z, o.w) -= L[rows, o.y:o.z] X[o.y:o.z]: a thread takes four
-            // columns of up to two rows (register blocking; each element is
-            // still one fma chain in pp order, then the subtraction)
-            constexpr int NG = CW / 4, RGS = 256 / NG;
-            const int cq = (tid % NG) * 4, rg = tid / NG;
-            for (int r0 = o.z + rg; r0 < o.w; r0 += 2 * RGS) {
-                const int r1 = r0 + RGS;
-                const bool has1 = r1 < o.w;
-                const double *L0 = L + (i64)r0 * ldl, *L1 = L + (i64)(has1 ? r1 : r0) * ldl;
-                double a0[4] = {0.0, 0.0, 0.0, 0.0}, a1[4] = {0.0, 0.0, 0.0, 0.0};
+            // rows [o.z, o.w) -= L[rows, o.y:o.z] X[o.y:o.z]: a thread takes CPT
+            // columns of one row at a time (each element is one fma chain in pp
+            // order, then the subtraction)
+            constexpr int NG = CW / CPT, RGS = 256 / NG;
+            const int cq = (tid % NG) * CPT;
+            for (int r = o.z + tid / NG; r < o.w; r += RGS) {
+                const double *Lr = Ls + r * TR_LP;
+                double a[CPT];
+#pragma unroll
+                for (int u = 0; u < CPT; ++u) a[u] = 0.0;
 #pragma unroll 8
                 for (int pp = o.y; pp < o.z; ++pp) {
-                    const double l0 = __ldg(L0 + pp), l1 = __ldg(L1 + pp);
-                    const double *xr = X + pp * XP + cq;
+                    const double l = Lr[pp];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        a0[u] = fma(l0, xr[u], a0[u]);
-                        a1[u] = fma(l1, xr[u], a1[u]);
+                    for (int u = 0; u < CPT; u += 2) {
+                        const double2 x2 = *(const double2 *)(X + pp * CW + cq + u);
+                        a[u] = fma(l, x2.x, a[u]);
+                        a[u + 1] = fma(l, x2.y, a[u + 1]);
                     }
                 }
+                double *xr = X + r * CW + cq;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) X[r0 * XP + cq + u] -= a0[u];
-                if (has1) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) X[r1 * XP + cq + u] -= a1[u];
+                for (int u = 0; u < CPT; u += 2) {
+                    double2 x2 = *(double2 *)(xr + u);
+                    x2.x -= a[u];
+                    x2.y -= a[u + 1];
+                    *(double2 *)(xr + u) = x2;
                 }
             }
         }
         __syncthreads();
     }
+#pragma unroll 4
     for (int e = tid; e < t * CW; e += 256) {
         const int i = e / CW, c = e - i * CW;
-        if (c < cols) B[(i64)i * ldb + c0 + c] = X[i * XP + c];
+        if (c < cols) B[(i64)i * ldb + c0 + c] = X[i * CW + c];
     }
 }
 
@@ -1213,15 +1225,15 @@ void launch_trsm_refo(const double *L, i64 ldl, double *B, i64 ldb, int t, i64 N
     TrsmSteps st{};
     trsm_steps_rec(0, t, st);
     ProfScope ps(KC_TRSM_LEAF, s, (double)t * t * N, 2.0 * (double)t * N * 8);
-    if (N <= 2048) {
-        constexpr int CW = 8;
-        const size_t smem = sizeof(double) * (size_t)t * (CW + 1);
-        k_trsm_refo<CW><<<(unsigned)((N + CW - 1) / CW), 256, smem, s>>>(L, ldl, B, ldb, t, N, st);
-    } else {
-        constexpr int CW = 32;
-        const size_t smem = sizeof(double) * (size_t)t * (CW + 1);
-        k_trsm_refo<CW><<<(unsigned)((N + CW - 1) / CW), 256, smem, s>>>(L, ldl, B, ldb, t, N, st);
-    }
+    // Narrow strips while they fit one wave (a strip's time is its chain of
+    // steps), then wider ones, which read the triangle less often.
+    auto go = [&](auto kern, int cw) {
+        set_max_dyn_smem((const void *)kern, (int)(sizeof(double) * TR_TMAX * (cw + TR_LP)));
+        kern<<<(unsigned)((N + cw - 1) / cw), 256, sizeof(double) * (size_t)t * (cw + TR_LP), s>>>(L, ldl, B, ldb, t, N,
+                                                                                                  st);
+    };
+    if (N <= 8 * 148) go(k_trsm_refo<8, 2>, 8);
+    else go(k_trsm_refo<32, 4>, 32);
     OXI_LAUNCH_CHECK();
 }
 
