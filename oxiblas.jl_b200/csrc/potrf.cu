@@ -10,22 +10,23 @@
 // matrix, and L (column-major, lower) is U = L^T (row-major, upper) in the same
 // memory.  So the factorization runs in place, row-oriented, with no copy:
 // blocks of NB rows of U, each
-//   1. U_kk = chol(A_kk) and W = U_kk^-1, one CTA, the block in shared memory;
-//   2. U_k,right = W^T A_k,right on the FP64 tensor cores (the block-row solve
-//      as a product with the inverted diagonal block, into a scratch block row
-//      X, then copied into place);
+//   1. U_kk = chol(A_kk) and the inverses of its four 32 x 32 diagonal blocks,
+//      one CTA, the block in shared memory;
+//   2. U_k,right = U_kk^-T A_k,right by blocks of 32 rows (products with the
+//      diagonal blocks' inverses), into place, into an aligned block row X and
+//      into its transpose, one launch;
 //   3. A_right,right -= X^T X on the FP64 tensor cores, upper triangle only
 //      (tiles wholly below the diagonal skipped, crossing tiles write only on
-//      and above it), its left operand a transposed copy of X so that both
+//      and above it), its left operand the transposed copy so that both
 //      operands are K-contiguous.
 // The reference solves the block row by substitution (trsm!); the product with
-// the inverted 128 x 128 block is the same solve with another association of
-// the sums (the diagonal blocks of a positive definite matrix's factor are
-// well conditioned: cond(U_kk)^2 <= cond(A)).
+// the inverted 32 x 32 diagonal blocks is the same solve with another
+// association of the sums (the diagonal blocks of a positive definite matrix's
+// factor are well conditioned: cond(U_kk)^2 <= cond(A)).
 // A pivot that is not finite and positive stops the factorization there: info
-// is its 1-based column (PosDefException(info)); the inverse of that block and
-// of every later one is written as zero, so the later products change nothing,
-// and the block rows are not copied back.
+// is its 1-based column (PosDefException(info)); every later block row X is
+// written as zero, so the later updates change nothing, and no block row
+// reaches the matrix.
 #include <algorithm>
 #include <cmath>
 #include "oxi_internal.h"
@@ -35,130 +36,315 @@ namespace oxi {
 
 namespace {
 constexpr int PO_NB = 128;          // block rows per step
-constexpr int PO_NT = 512;          // threads of the diagonal-block kernel (4 per column of the inverse)
+constexpr int PO_SB = 32;           // blocks inside a diagonal block
+constexpr int PO_NT = 256;
+constexpr int PO_GB = 8;            // rows factored between two updates of the block
+// row pitches in shared memory: 4 modulo 16, no conflicts of a DMMA fragment's loads
+constexpr int PO_LP = PO_NB + 4, PO_CP = PO_SB + 4;
 }  // namespace
 
-// Cholesky of the t x t diagonal block (row-major upper, ld) in shared memory:
-// for each row c, d = sqrt(a_cc), the row scaled by d, then the rank-1 update
-// of the upper triangle below it, a_ij = fma(-u_ci, u_cj, a_ij) for c < i <= j
-// (the reference leaf's column updates, src/lapack/factorizations.jl:266-282,
-// read through the transposition).  Then W = U^-1 by 32 x 32 diagonal blocks
-// and the off-diagonal blocks of the 64 and 128 levels, W^T kept in the
-// block's unused strict lower triangle, and
-// Wneg = -W^T (t x t, row-major, lower) written for the block-row product.
+// d = sqrt(a) and y = 1 / d for a finite a > 0: the approximate reciprocal
+// root, one cubic Newton step, and a fused correction of each result (the
+// latency of one chain instead of a square root followed by a division); the
+// library functions where an exponent could over- or underflow on the way.
+__device__ __forceinline__ void root_recip(double a, double &d, double &y) {
+    if (a > 0x1p-900 && a < 0x1p900) {
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+        const double e = fma(-(a * y), y, 1.0);
+        y = fma(y * e, fma(0.375, e, 0.5), y);
+        const double g = a * y;
+        d = fma(fma(-g, g, a), 0.5 * y, g);
+        y = fma(fma(-d, y, 1.0), y, y);
+    } else {
+        d = sqrt(a);
+        y = 1.0 / d;
+    }
+}
+__device__ __forceinline__ void root_recip(float a, float &d, float &y) {
+    d = sqrtf(a);
+    y = 1.0f / d;
+}
+__device__ __forceinline__ bool exp_all_ones(double a) { return (__double2hiint(a) & 0x7ff00000) == 0x7ff00000; }
+__device__ __forceinline__ bool exp_all_ones(float a) { return (__float_as_uint(a) & 0x7f800000u) == 0x7f800000u; }
+// a / d with the reciprocal's rounding corrected by the remainder
+template <typename T>
+__device__ __forceinline__ T scaled(T a, T d, T y) {
+    const T q = a * y;
+    const T r = fma(fma(-q, d, a), y, q);
+    return exp_all_ones(r) ? a / d : r;
+}
+
+// four neighbours in shared memory, 16-byte aligned
+__device__ __forceinline__ void load4(double (&v)[4], const double *p) {
+    const double2 a = *(const double2 *)p, b = *(const double2 *)(p + 2);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void load4(float (&v)[4], const float *p) {
+    const float4 a = *(const float4 *)p;
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void store4(double *p, const double (&v)[4]) {
+    *(double2 *)p = make_double2(v[0], v[1]);
+    *(double2 *)(p + 2) = make_double2(v[2], v[3]);
+}
+__device__ __forceinline__ void store4(float *p, const float (&v)[4]) { *(float4 *)p = make_float4(v[0], v[1], v[2], v[3]); }
+
+// Cholesky of the t x t diagonal block (row-major upper, ld) in shared memory, by
+// groups of 8 rows: warp 0 factors the group's 8 x 8 diagonal block in
+// registers, the columns to the right are solved by substitution, one per
+// thread, and the rest takes the rank-8 update in 4 x 4 tiles.  Element for
+// element these are the operations of the reference leaf's column updates
+// (src/lapack/factorizations.jl:266-282), read through the transposition.
+// Winv: the inverses of a full block's 32 x 32 diagonal blocks, PO_SB x PO_SB
+// row-major each (upper), one warp each at the end.
+// Bound: latency of the 16 groups (eight dependent roots, reciprocals and scaled
+// rows in one warp, then two phases of the CTA).
 template <typename T>
 __global__ void __launch_bounds__(PO_NT) k_potrf_diag(T *__restrict__ U, i64 ld, int t, i64 g0,
-                                                      int64_t *__restrict__ info, T *__restrict__ Wneg) {
+                                                      int64_t *__restrict__ info, T *__restrict__ Winv) {
     extern __shared__ __align__(16) unsigned char po_smem_raw[];
-    const int lp = t + 1;
     T *S = (T *)po_smem_raw;
-    T *s_inv = S + (size_t)t * lp;  // 1 / u_ii
+    __shared__ T s_y[PO_NB];  // 1 / u_ii
     __shared__ int s_fail;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_fail = (*(volatile int64_t *)info != 0) ? 1 : 0;
     __syncthreads();
-    if (s_fail) {  // an earlier block failed: later products change nothing
-        for (int e = tid; e < t * t; e += PO_NT) Wneg[e] = T(0);
-        return;
-    }
-    for (int e = tid; e < t * t; e += PO_NT) {
-        const int i = e / t, j = e - i * t;
-        S[i * lp + j] = (j >= i) ? U[(i64)i * ld + j] : T(0);
+    if (s_fail) return;  // an earlier block failed
+#pragma unroll 16
+    for (int e = tid; e < PO_NB * PO_NB; e += PO_NT) {
+        const int i = e / PO_NB, j = e % PO_NB;
+        S[i * PO_LP + j] = (i < t && j < t) ? ((j >= i) ? U[(i64)i * ld + j] : T(0)) : (i == j ? T(1) : T(0));
     }
     __syncthreads();
-    for (int c = 0; c < t; ++c) {
-        T d = S[c * lp + c];
-        if (!(d > T(0)) || !isfinite(d)) {  // not positive definite at global column g0 + c + 1
-            if (tid == 0) {
-                s_fail = 1;
-                if (*info == 0) *info = g0 + c + 1;
+#pragma unroll 1
+    for (int b0 = 0; b0 < t; b0 += PO_GB) {
+        if (warp == 0) {
+            const int col = lane & (PO_GB - 1);  // lanes 0..7 hold the columns (the others repeat them)
+            T x[PO_GB];
+#pragma unroll
+            for (int i = 0; i < PO_GB; ++i) x[i] = S[(b0 + i) * PO_LP + b0 + col];
+            bool fail = false;
+#pragma unroll
+            for (int c = 0; c < PO_GB; ++c) {
+                const T a = __shfl_sync(0xffffffffu, x[c], c);
+                if (!(a > T(0)) || exp_all_ones(a)) {  // not positive definite at global column g0 + b0 + c + 1
+                    if (!fail && lane == 0) {
+                        s_fail = 1;
+                        if (*info == 0) *info = g0 + b0 + c + 1;
+                    }
+                    fail = true;
+                }
+                if (!fail) {
+                    T d, y;
+                    root_recip(a, d, y);
+                    x[c] = (col == c) ? d : scaled(x[c], d, y);
+                    if (lane == c) s_y[b0 + c] = y;
+#pragma unroll
+                    for (int i = c + 1; i < PO_GB; ++i) x[i] = fma(-__shfl_sync(0xffffffffu, x[c], i), x[c], x[i]);
+                }
             }
-            break;
+#pragma unroll
+            for (int i = 0; i < PO_GB; ++i)
+                if (lane < PO_GB && i <= col) S[(b0 + i) * PO_LP + b0 + col] = x[i];
         }
-        d = sqrt(d);
-        // the row right of the pivot (the pivot itself is written after the
-        // barrier: every thread has read it by then)
-        for (int j = c + 1 + tid; j < t; j += PO_NT) S[c * lp + j] = S[c * lp + j] / d;
         __syncthreads();
-        if (tid == 0) S[c * lp + c] = d;
-        // rows i below c, columns j >= i: 16 row groups x 32 columns of threads
-        const int tx = tid & 31, ty = tid >> 5;
-        for (int i = c + 1 + ty; i < t; i += PO_NT / 32) {
-            const T ui = S[c * lp + i];
-            for (int j = i + tx; j < t; j += 32) S[i * lp + j] = fma(-ui, S[c * lp + j], S[i * lp + j]);
+        if (s_fail) break;
+        const int r0 = b0 + PO_GB;  // the columns to the right
+        if (tid < PO_NB - r0) {
+            // x_i = (a_i - sum_{p<i} u_pi x_p) / u_ii
+            const int j = r0 + tid;
+            T x[PO_GB];
+#pragma unroll
+            for (int i = 0; i < PO_GB; ++i) x[i] = S[(b0 + i) * PO_LP + j];
+#pragma unroll
+            for (int p = 0; p < PO_GB; ++p) {
+                const T *row = S + (b0 + p) * PO_LP + b0;
+                x[p] = scaled(x[p], row[p], s_y[b0 + p]);
+#pragma unroll
+                for (int i = p + 1; i < PO_GB; ++i) x[i] = fma(-row[i], x[p], x[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < PO_GB; ++i) S[(b0 + i) * PO_LP + j] = x[i];
+        }
+        __syncthreads();
+        // a_ij -= sum_p u_pi u_pj (r0 <= i <= j), 4 x 4 tiles of the upper triangle
+        const int nt4 = (PO_NB - r0) / 4, tasks = nt4 * (nt4 + 1) / 2;
+        for (int q = tid; q < tasks; q += PO_NT) {
+            int bj = (int)((sqrtf(8.0f * q + 1.0f) - 1.0f) * 0.5f);
+            while ((bj + 1) * (bj + 2) / 2 <= q) ++bj;
+            while (bj * (bj + 1) / 2 > q) --bj;
+            const int bi = q - bj * (bj + 1) / 2;
+            const int i = r0 + 4 * bi, j = r0 + 4 * bj;
+            T acc[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) load4(acc[u], S + (i + u) * PO_LP + j);
+#pragma unroll
+            for (int p = 0; p < PO_GB; ++p) {
+                const T *row = S + (b0 + p) * PO_LP;
+                T ui[4], uj[4];
+                load4(ui, row + i);
+                load4(uj, row + j);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) acc[u][w] = fma(-ui[u], uj[w], acc[u][w]);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) store4(S + (i + u) * PO_LP + j, acc[u]);
         }
         __syncthreads();
     }
     __syncthreads();
-    for (int e = tid; e < t * t; e += PO_NT) {
-        const int i = e / t, j = e - i * t;
-        if (j >= i) U[(i64)i * ld + j] = S[i * lp + j];
-    }
-    if (s_fail) {
-        for (int e = tid; e < t * t; e += PO_NT) Wneg[e] = T(0);
-        return;
-    }
-    // W = U^-1 by blocks (only the full 128-row blocks have a block row to the
-    // right; a shorter last block needs no inverse): the four 32 x 32 diagonal
-    // blocks column by column (a thread per column, the columns independent),
-    // then the off-diagonal block of each 64 x 64 and of the 128 x 128 level,
-    //   W[A, C] = -W[A, A] (U[A, C] W[C, C]),
-    // as two products in shared memory.  W (upper) is kept transposed in the
-    // strict lower part of S (w_rc at S[c * lp + r], r < c), its diagonal in s_inv.
-    if (t != PO_NB) {
-        for (int e = tid; e < t * t; e += PO_NT) Wneg[e] = T(0);
-        return;
-    }
-    for (int i = tid; i < t; i += PO_NT) s_inv[i] = T(1) / S[i * lp + i];
-    __syncthreads();
-    if (tid < t) {
-        const int c = tid, b0 = c & ~31;
-        for (int i = c - 1; i >= b0; --i) {
-            T part = T(0);
-            for (int p = i + 1; p <= c; ++p) part = fma(S[i * lp + p], (p == c) ? s_inv[c] : S[c * lp + p], part);
-            S[c * lp + i] = -part * s_inv[i];
+    if (warp < PO_NB / PO_SB && t == PO_NB && !s_fail) {
+        // column `lane` of this warp's diagonal block's inverse, eight rows at a time
+        const int b0 = warp * PO_SB;
+        T w[PO_SB];
+#pragma unroll
+        for (int i = 0; i < PO_SB; ++i) w[i] = (i == lane) ? T(1) : T(0);
+#pragma unroll
+        for (int p = PO_SB - 1; p >= 0; --p) {
+            w[p] = w[p] * s_y[b0 + p];
+#pragma unroll
+            for (int i = 0; i < p; ++i) w[i] = fma(-S[(b0 + i) * PO_LP + b0 + p], w[p], w[i]);
         }
+#pragma unroll
+        for (int i = 0; i < PO_SB; ++i) Winv[(b0 + i) * PO_SB + lane] = w[i];
     }
-    __syncthreads();
-    T *Tm = s_inv + t;  // (t / 2h) blocks of h x h: U[A, C] W[C, C]
-    for (int hh = 32; hh < t; hh *= 2) {
-        const int nel = (t / (2 * hh)) * hh * hh;
-        for (int e = tid; e < nel; e += PO_NT) {
-            const int blk = e / (hh * hh), rc = e - blk * hh * hh, r = rc / hh, c = rc - r * hh;
-            const int a0 = blk * 2 * hh, c0 = a0 + hh;
-            T acc = T(0);
-            for (int p = 0; p <= c; ++p)
-                acc = fma(S[(a0 + r) * lp + c0 + p], (p == c) ? s_inv[c0 + c] : S[(c0 + c) * lp + c0 + p], acc);
-            Tm[e] = acc;
-        }
-        __syncthreads();
-        for (int e = tid; e < nel; e += PO_NT) {
-            const int blk = e / (hh * hh), rc = e - blk * hh * hh, r = rc / hh, c = rc - r * hh;
-            const int a0 = blk * 2 * hh, c0 = a0 + hh;
-            const T *tcol = Tm + blk * hh * hh + c;
-            T acc = T(0);
-            for (int q = r; q < hh; ++q) acc = fma((q == r) ? s_inv[a0 + r] : S[(a0 + q) * lp + a0 + r], tcol[q * hh], acc);
-            S[(c0 + c) * lp + a0 + r] = -acc;
-        }
-        __syncthreads();
-    }
-    // Wneg = -W^T: row i holds -w_pi for p <= i
-    for (int e = tid; e < t * t; e += PO_NT) {
-        const int i = e / t, p = e - i * t;
-        Wneg[e] = (p < i) ? -S[i * lp + p] : (p == i ? -s_inv[i] : T(0));
+#pragma unroll 16
+    for (int e = tid; e < PO_NB * PO_NB; e += PO_NT) {
+        const int i = e / PO_NB, j = e % PO_NB;
+        if (j >= i && j < t) U[(i64)i * ld + j] = S[i * PO_LP + j];
     }
 }
 
-// The solved block row back into place (row-major t x N), unless the
-// factorization failed.
+// The block row right of a full diagonal block: X = U_kk^-T A (128 x N), 32
+// columns per CTA, row block by row block: T_k = A_k - sum_{p<k} U_pk^T X_p,
+// X_k = W_kk^T T_k with the diagonal block's inverse.  X goes into place (A), into
+// the aligned block row X and, transposed, into Xt (N x 128); zeros instead, and
+// A untouched, once the factorization has failed.  One launch instead of a
+// cleared block row, a product, a copy and a transpose.  FP64 products run on the
+// tensor cores.  Bound: latency (the staging, then up to 20 chained DMMAs and
+// three barriers per row block).
 template <typename T>
-__global__ void k_copy_block_row(const T *__restrict__ X, i64 ldx, T *__restrict__ B, i64 ldb, int t,
-                                 i64 N, const int64_t *__restrict__ info) {
-    if (*(volatile const int64_t *)info != 0) return;
-    const i64 idx = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (i64)t * N) return;
-    const i64 i = idx / N, c = idx - i * N;
-    B[i * ldb + c] = X[i * ldx + c];
+struct PoRowSmem {
+    T U[PO_NB][PO_LP];
+    T W[PO_NB][PO_CP];
+    T A[PO_NB][PO_CP];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(PO_NT) k_potrf_row(const T *__restrict__ Ukk, const T *__restrict__ Winv,
+                                                     T *__restrict__ A, i64 ld, i64 N, T *__restrict__ X, i64 ldx,
+                                                     T *__restrict__ Xt, const int64_t *__restrict__ info) {
+    extern __shared__ __align__(16) unsigned char po_smem_raw[];
+    PoRowSmem<T> &S = *reinterpret_cast<PoRowSmem<T> *>(po_smem_raw);
+    const int tid = threadIdx.x;
+    const i64 c0 = (i64)blockIdx.x * PO_SB;
+    const int cols = (int)((N - c0) < PO_SB ? (N - c0) : PO_SB);
+    const bool failed = *(volatile const int64_t *)info != 0;
+    if (failed) {
+        for (int e = tid; e < PO_NB * PO_SB; e += PO_NT) {
+            const int i = e / PO_SB, c = e % PO_SB;
+            if (c < cols) {
+                X[(i64)i * ldx + c0 + c] = T(0);
+                Xt[(c0 + c) * PO_NB + i] = T(0);
+            }
+        }
+        return;
+    }
+auto copy_async = [](T *dst, const T *src) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"((int)sizeof(T)) : "memory");
+    };
+    for (int e = tid; e < PO_NB * PO_NB; e += PO_NT) {
+        const int i = e / PO_NB, j = e % PO_NB;
+        if (j / PO_SB > i / PO_SB) copy_async(&S.U[i][j], Ukk + (i64)i * ld + j);
+    }
+    for (int e = tid; e < PO_NB * PO_SB; e += PO_NT) {
+        const int i = e / PO_SB, c = e % PO_SB;
+        copy_async(&S.W[i][c], Winv + e);
+        if (c < cols) copy_async(&S.A[i][c], A + (i64)i * ld + c0 + c);
+        else S.A[i][c] = T(0);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if constexpr (sizeof(T) == 8) {
+        // a 16 x 8 tile of the row block per warp on the tensor cores
+        const int lane = tid & 31, warp = tid >> 5, gid = lane >> 2, tig = lane & 3;
+        const int m0 = (warp & 1) * 16 + gid, n0 = (warp >> 1) * 8;
+        auto products = [&](double (&c)[2][4], const double *Am, int ap, const double *Bm, int K) {  // Am^T Bm
+#pragma unroll 4
+            for (int k = 0; k < K; k += 8)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int kc = k + 4 * h + tig;
+                    asm volatile(
+                        "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                        : "+d"(c[h][0]), "+d"(c[h][1]), "+d"(c[h][2]), "+d"(c[h][3])
+                        : "d"(Am[kc * ap + m0]), "d"(Am[kc * ap + m0 + 8]), "d"(Bm[kc * PO_CP + n0 + gid]));
+                }
+        };
+        for (int b = 0; b < PO_NB; b += PO_SB) {
+            if (b > 0) {
+                double c[2][4] = {};
+                products(c, &S.U[0][b], PO_LP, &S.A[0][0], b);
+                // each thread rewrites elements that only it has read in this block
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S.A[b + m0 + 8 * (e >> 1)][n0 + 2 * tig + (e & 1)] -= c[0][e] + c[1][e];
+                __syncthreads();
+            }
+            double c[2][4] = {};
+            products(c, &S.W[b][0], PO_CP, &S.A[b][0], PO_SB);  // W is zero below its diagonal
+            __syncthreads();
+#pragma unroll
+            for (int e = 0; e < 4; ++e) S.A[b + m0 + 8 * (e >> 1)][n0 + 2 * tig + (e & 1)] = c[0][e] + c[1][e];
+            __syncthreads();
+        }
+    } else {
+        const int ri = tid >> 3, c4 = (tid & 7) * 4;  // a row, four columns
+        for (int b = 0; b < PO_NB; b += PO_SB) {
+            T v[4];
+            load4(v, &S.A[b + ri][c4]);
+            if (b > 0) {
+#pragma unroll 8
+                for (int p = 0; p < b; ++p) {
+                    const T u = S.U[p][b + ri];
+                    T x[4];
+                    load4(x, &S.A[p][c4]);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) v[q] = fma(-u, x[q], v[q]);
+                }
+                store4(&S.A[b + ri][c4], v);
+                __syncthreads();
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = T(0);
+#pragma unroll 8
+            for (int p = 0; p < PO_SB; ++p) {
+                const T w = S.W[b + p][ri];  // zero below the diagonal
+                T x[4];
+                load4(x, &S.A[b + p][c4]);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = fma(w, x[q], v[q]);
+            }
+            __syncthreads();
+            store4(&S.A[b + ri][c4], v);
+            __syncthreads();
+        }
+    }
+#pragma unroll 4
+    for (int e = tid; e < PO_NB * PO_SB; e += PO_NT) {
+        const int i = e / PO_SB, c = e % PO_SB;
+        if (c < cols) {
+            const T x = S.A[i][c];
+            A[(i64)i * ld + c0 + c] = x;
+            X[(i64)i * ldx + c0 + c] = x;
+        }
+    }
+#pragma unroll 4
+    for (int e = tid; e < PO_NB * PO_SB; e += PO_NT) {
+        const int c = e / PO_NB, i = e % PO_NB;
+        if (c < cols) Xt[(c0 + c) * PO_NB + i] = S.A[i][c];
+    }
 }
 
 // The strict lower triangle of the row-major view (the strict upper triangle
@@ -172,27 +358,18 @@ __global__ void k_zero_strict_lower(T *__restrict__ U, i64 ld, int n, const int6
     if (j < i) U[(i64)i * ld + j] = T(0);
 }
 
-// Workspace of one factorization, in elements: T (n x NB) and X (NB x ldx),
-// two of each (the lookahead's update of block k reads them while block k + 1
-// writes the other pair), Bc (NB x ldx), Wneg (NB x NB).
+// Workspace of one factorization, in elements: Xt (n x NB) and X (NB x ldx), two
+// of each (the lookahead's update of block k reads them while block k + 1 writes
+// the other pair), and the diagonal blocks' inverses.
 size_t potrf_work_elems(i64 n) {
     const i64 ldx = (n + 3) / 4 * 4;
-    return 2 * (size_t)n * PO_NB + 3 * (size_t)PO_NB * ldx + (size_t)PO_NB * PO_NB + 64;
+    return 2 * (size_t)n * PO_NB + 2 * (size_t)PO_NB * ldx + (size_t)PO_NB * PO_SB + 64;
 }
 
-// X (t x N) = 0 - Wneg B and the symmetric update A22 -= T X (T = X^T), upper
-// triangle of the row-major view: FP64 on the DMMA tensor-core GEMM; FP32 (the
-// mixed solve's low-precision factor, a private copy) with the product on the
-// CUDA cores and the update in the handle's trailing precision (tcgen05 for the
-// 16-bit kinds; the whole square, the other triangle being scratch there).
-static void po_block_row(oxi_handle_s *h, double *X, i64 ldx, const double *Wneg, int t, const double *B, i64 ldb,
-                         i64 N, cudaStream_t s) {
-    launch_gemm_dmma(X, ldx, Wneg, t, B, ldb, t, N, t, s);
-}
-static void po_block_row(oxi_handle_s *, float *X, i64 ldx, const float *Wneg, int t, const float *B, i64 ldb,
-                         i64 N, cudaStream_t s) {
-    launch_gemm_simt<float>(X, ldx, Wneg, t, B, ldb, t, N, t, s);
-}
+// The symmetric update A22 -= Xt X, upper triangle of the row-major view: FP64
+// on the DMMA tensor-core GEMM; FP32 (the mixed solve's low-precision factor, a
+// private copy) in the handle's trailing precision (tcgen05 for the 16-bit
+// kinds; the whole square, the other triangle being scratch there).
 // rows x N block of the symmetric update whose (0, 0) is on the diagonal
 // (M <= N): FP64 only on and above the diagonal
 static void po_sym_update(oxi_handle_s *, double *A22, i64 ld, const double *T, int t, const double *X, i64 ldx,
@@ -219,8 +396,7 @@ void potrf_rowmajor(oxi_handle_s *h, T *U, i64 ld, i64 n, int64_t *d_info, T *wo
     const i64 ldx = (n + 3) / 4 * 4;  // 16-byte rows for the TMA-fed GEMMs
     T *Tt2[2] = {work, work + (size_t)n * PO_NB};
     T *X2[2] = {work + 2 * (size_t)n * PO_NB, work + 2 * (size_t)n * PO_NB + (size_t)PO_NB * ldx};
-    T *Bc = X2[1] + (size_t)PO_NB * ldx;
-    T *Wneg = Bc + (size_t)PO_NB * ldx;
+    T *Winv = X2[1] + (size_t)PO_NB * ldx;
     if (la) {
         ensure_lookahead_streams(h);
         OXI_CUDA(cudaEventRecord(h->la_in, caller));
@@ -235,35 +411,22 @@ void potrf_rowmajor(oxi_handle_s *h, T *U, i64 ld, i64 n, int64_t *d_info, T *wo
             T *Ukk = U + k0 * ld + k0;
             T *Tt = Tt2[kb & 1], *X = X2[kb & 1];
             {
-                // the block, 1 / u_ii, and the inverse's product scratch (h x h at the top level)
-                const size_t smem = sizeof(T) * ((size_t)t * (t + 1) + t + (size_t)(PO_NB / 2) * (PO_NB / 2));
-                set_max_dyn_smem((const void *)k_potrf_diag<T>,
-                                 (int)(sizeof(T) * (PO_NB * (PO_NB + 1) + PO_NB + (PO_NB / 2) * (PO_NB / 2))));
+                const int smem = (int)(sizeof(T) * PO_NB * PO_LP);
+                set_max_dyn_smem((const void *)k_potrf_diag<T>, smem);
                 ProfScope ps(KC_LEAF, s, (double)t * t * t * (2.0 / 3.0), 2.0 * sizeof(T) * t * t);
-                k_potrf_diag<T><<<1, PO_NT, smem, s>>>(Ukk, ld, t, k0, d_info, Wneg);
+                k_potrf_diag<T><<<1, PO_NT, smem, s>>>(Ukk, ld, t, k0, d_info, Winv);
                 OXI_LAUNCH_CHECK();
             }
             const i64 right = n - k0 - t;
             if (right <= 0) break;
-            T *Bk = Ukk + t;  // rows k0..k0+t, columns k0+t..n
-            // the tensor-core GEMM reads its operands through TMA (16-byte aligned
-            // rows); a block row at an odd offset or pitch is copied first
-            const T *Bop = Bk;
-            i64 ldb_op = ld;
-            if ((uintptr_t)Bk % 16 != 0 || (ld * (i64)sizeof(T)) % 16 != 0) {
-                OXI_CUDA(cudaMemcpy2DAsync(Bc, sizeof(T) * ldx, Bk, sizeof(T) * ld, sizeof(T) * right, (size_t)t,
-                                           cudaMemcpyDeviceToDevice, s));
-                Bop = Bc;
-                ldb_op = ldx;
+            {
+                const int smem = (int)sizeof(PoRowSmem<T>);
+                set_max_dyn_smem((const void *)k_potrf_row<T>, smem);
+                ProfScope ps(KC_TRSM_LEAF, s, (double)t * t * right, 4.0 * (double)t * right * sizeof(T));
+                k_potrf_row<T><<<(unsigned)((right + PO_SB - 1) / PO_SB), PO_NT, smem, s>>>(Ukk, Winv, Ukk + t, ld, right,
+                                                                                           X, ldx, Tt, d_info);
+                OXI_LAUNCH_CHECK();
             }
-            // X = 0 - (-W^T) A_k,right = U_kk^-T A_k,right
-            OXI_CUDA(cudaMemsetAsync(X, 0, sizeof(T) * (size_t)t * ldx, s));
-            po_block_row(h, X, ldx, Wneg, t, Bop, ldb_op, right, s);
-            k_copy_block_row<T><<<(unsigned)(((i64)t * right + 255) / 256), 256, 0, s>>>(X, ldx, Bk, ld, t, right,
-                                                                                        d_info);
-            OXI_LAUNCH_CHECK();
-            // Tt = X^T (right x t, row-major): X read as a column-major right x t matrix
-            launch_cm_to_rm<T, T>(X, ldx, Tt, t, right, t, s);
             T *A22 = U + (k0 + t) * ld + (k0 + t);
             if (!la) {
                 po_sym_update(h, A22, ld, Tt, t, X, ldx, right, right, s);
