@@ -211,4 +211,157 @@ void launch_gemm_dmma(double *C, i64 ldc, const double *A, i64 lda, const double
     OXI_LAUNCH_CHECK();
 }
 
+// ---------------------------------------------------------------------------
+// The complex update C -= A B on real and imaginary planes (row-major, one ld),
+// one launch: 64 x 64 tile, k slab 16, 3 stages of the four operand planes, the
+// two accumulators of a C element in registers, four DMMAs per fragment pair
+// (Cr: Ar Br, then (-Ai) Bi; Ci: Ar Bi, then Ai Br; the negation is a sign bit
+// of the fragment).  Against four launches of k_gemm_dmma and a negated copy
+// of Ai it loads each fragment once for two products and moves C once.
+// ---------------------------------------------------------------------------
+namespace {
+constexpr int ZM = 64, ZN = 64, ZST = 3;
+constexpr int ZPLANE = ZM * BK * 8;            // 8 KB: a plane of A or of B
+constexpr int ZSTAGE = 4 * ZPLANE;
+constexpr int ZSMEM = ZST * ZSTAGE + 1024 + 256;
+}  // namespace
+
+__device__ __forceinline__ void dmma_16x8x4(double (&c)[4], double a0, double a1, double b) {
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+                 : "d"(a0), "d"(a1), "d"(b));
+}
+
+__global__ void __launch_bounds__(NTHREADS, 2)
+k_zgemm_dmma(const __grid_constant__ CUtensorMap tmAr, const __grid_constant__ CUtensorMap tmAi,
+             const __grid_constant__ CUtensorMap tmBr, const __grid_constant__ CUtensorMap tmBi,
+             double *__restrict__ Cr, double *__restrict__ Ci, i64 ldc, int M, int N, int K, int *__restrict__ ab) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~uintptr_t(1023));
+    uint64_t *full = (uint64_t *)(smem + ZST * ZSTAGE);
+    uint64_t *empty = full + ZST;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m0 = blockIdx.y * ZM, n0 = blockIdx.x * ZN;
+    const int KT = (K + BK - 1) / BK;
+    __shared__ int s_skip;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < ZST; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], NCONSUMER_WARPS);
+        }
+        s_skip = aborted(ab) ? 1 : 0;  // one reading for the whole CTA
+        fence_barrier_init();
+    }
+    __syncthreads();
+    if (s_skip) return;
+
+    if (warp == NCONSUMER_WARPS) {
+        if (lane == 0) {
+            for (int kt = 0; kt < KT; ++kt) {
+                const int s = kt % ZST;
+                if (kt >= ZST && !mbar_wait<false>(&empty[s], ((kt / ZST) + 1) & 1, ab, 2)) break;
+                uint8_t *sa = smem + s * ZSTAGE;
+                mbar_arrive_expect_tx(&full[s], ZSTAGE);
+                tma_load_2d(sa, &tmAr, &full[s], kt * BK, m0);
+                tma_load_2d(sa + ZPLANE, &tmAi, &full[s], kt * BK, m0);
+#pragma unroll
+                for (int g = 0; g < ZN / 8; ++g) {
+                    tma_load_2d(sa + 2 * ZPLANE + g * (BK * 64), &tmBr, &full[s], n0 + 8 * g, kt * BK);
+                    tma_load_2d(sa + 3 * ZPLANE + g * (BK * 64), &tmBi, &full[s], n0 + 8 * g, kt * BK);
+                }
+            }
+        }
+        return;
+    }
+
+    const int wm = warp & 3, wn = warp >> 2;  // 4 x 2 warps: 16 rows x 32 columns each
+    const int gid = lane >> 2, tig = lane & 3;
+    double cr[4][4], ci[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) cr[b][c] = ci[b][c] = 0.0;
+    for (int kt = 0; kt < KT; ++kt) {
+        const int s = kt % ZST;
+        if (!mbar_wait<false>(&full[s], (kt / ZST) & 1, ab, 2)) return;
+        const uint8_t *sa = smem + s * ZSTAGE;
+#pragma unroll
+        for (int k4 = 0; k4 < BK / 4; ++k4) {
+            const int kc = k4 * 4 + tig;
+            double ar[2], ai[2];
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int r = wm * 16 + gid + 8 * hh;
+                const int off = r * 128 + ((((kc * 8) >> 4) ^ (r & 7)) << 4) + ((kc * 8) & 15);
+                ar[hh] = *(const double *)(sa + off);
+                ai[hh] = *(const double *)(sa + ZPLANE + off);
+            }
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const int off = (wn * 4 + nt) * (BK * 64) + kc * 64 + gid * 8;
+                const double br = *(const double *)(sa + 2 * ZPLANE + off);
+                const double bi = *(const double *)(sa + 3 * ZPLANE + off);
+                dmma_16x8x4(cr[nt], ar[0], ar[1], br);
+                dmma_16x8x4(ci[nt], ar[0], ar[1], bi);
+                dmma_16x8x4(cr[nt], -ai[0], -ai[1], bi);
+                dmma_16x8x4(ci[nt], ai[0], ai[1], br);
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
+    }
+
+    const bool vec2 = ((ldc & 1) == 0) && ((((uintptr_t)Cr) & 15) == 0) && ((((uintptr_t)Ci) & 15) == 0);
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+        const int r = m0 + wm * 16 + gid + 8 * hh;
+        if (r >= M) continue;
+#pragma unroll
+        for (int pl = 0; pl < 2; ++pl) {
+            double *crow = (pl ? Ci : Cr) + (i64)r * ldc;
+            double2 cv[4];
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const int c = n0 + wn * 32 + nt * 8 + 2 * tig;
+                if (c + 1 < N && vec2) cv[nt] = *(const double2 *)(crow + c);
+                else {
+                    cv[nt].x = c < N ? crow[c] : 0.0;
+                    cv[nt].y = c + 1 < N ? crow[c + 1] : 0.0;
+                }
+            }
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const int c = n0 + wn * 32 + nt * 8 + 2 * tig;
+                double2 v;
+                v.x = cv[nt].x - (pl ? ci[nt][2 * hh] : cr[nt][2 * hh]);
+                v.y = cv[nt].y - (pl ? ci[nt][2 * hh + 1] : cr[nt][2 * hh + 1]);
+                if (c + 1 < N && vec2) *(double2 *)(crow + c) = v;
+                else {
+                    if (c < N) crow[c] = v.x;
+                    if (c + 1 < N) crow[c + 1] = v.y;
+                }
+            }
+        }
+    }
+}
+
+bool zgemm_dmma_applicable(const double *Ar, const double *Ai, const double *Br, const double *Bi, i64 ld) {
+    return (((uintptr_t)Ar | (uintptr_t)Ai | (uintptr_t)Br | (uintptr_t)Bi) % 16 == 0) && ld % 2 == 0;
+}
+void launch_zgemm_dmma(double *Cr, double *Ci, const double *Ar, const double *Ai, const double *Br, const double *Bi,
+                       i64 ld, i64 M, i64 N, i64 K, cudaStream_t s) {
+    if (M <= 0 || N <= 0 || K <= 0) return;
+    CUtensorMap tm[4];
+    make_tmap_2d(&tm[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, Ar, K, M, ld, BK, ZM, CU_TENSOR_MAP_SWIZZLE_128B);
+    make_tmap_2d(&tm[1], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, Ai, K, M, ld, BK, ZM, CU_TENSOR_MAP_SWIZZLE_128B);
+    make_tmap_2d(&tm[2], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, Br, N, K, ld, 8, BK, CU_TENSOR_MAP_SWIZZLE_NONE);
+    make_tmap_2d(&tm[3], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, Bi, N, K, ld, 8, BK, CU_TENSOR_MAP_SWIZZLE_NONE);
+    set_max_dyn_smem((const void *)k_zgemm_dmma, ZSMEM);
+    dim3 grid((unsigned)((N + ZN - 1) / ZN), (unsigned)((M + ZM - 1) / ZM));
+    ProfScope ps(KC_GEMM_DMMA, s, 8.0 * M * N * K, 16.0 * (2.0 * M * N + M * K + K * N));
+    k_zgemm_dmma<<<grid, NTHREADS, ZSMEM, s>>>(tm[0], tm[1], tm[2], tm[3], Cr, Ci, ld, (int)M, (int)N, (int)K,
+                                               cur_abort());
+    OXI_LAUNCH_CHECK();
+}
+
 }  // namespace oxi

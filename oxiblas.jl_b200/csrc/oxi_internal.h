@@ -320,6 +320,12 @@ void launch_gemm_ref(T *C, i64 ldc, const T *A, i64 lda, const T *B, i64 ldb, i6
 void launch_gemm_dmma(double *C, i64 ldc, const double *A, i64 lda, const double *B, i64 ldb,
                       i64 M, i64 N, i64 K, cudaStream_t s, bool upper_only = false);
 
+// The complex form on real and imaginary planes (one leading dimension) when
+// the operand planes are aligned for TMA.
+bool zgemm_dmma_applicable(const double *Ar, const double *Ai, const double *Br, const double *Bi, i64 ld);
+void launch_zgemm_dmma(double *Cr, double *Ci, const double *Ar, const double *Ai, const double *Br, const double *Bi,
+                       i64 ld, i64 M, i64 N, i64 K, cudaStream_t s);
+
 // tcgen05 GEMM: C (FP32 row-major) -= scale * A16 * B16^T, 16-bit K-major operands.
 void launch_gemm_tc(int fmt, float *C, i64 ldc, const void *A16, i64 lda16, const void *B16,
                     i64 ldb16, i64 M, i64 N, i64 K, float scale, const float *d_scale,

@@ -22,7 +22,9 @@
 #include <cmath>
 #include <cstring>
 #include <vector>
+#include "leaf.cuh"
 #include "oxi_internal.h"
+#include "tma_util.cuh"
 
 namespace oxi {
 
@@ -40,6 +42,11 @@ __device__ __forceinline__ zd zmul(zd a, zd b) { return {a.r * b.r - a.i * b.i, 
 __device__ __forceinline__ zd zmsub(zd c, zd a, zd b) {
     return {c.r - (a.r * b.r - a.i * b.i), c.i - (a.r * b.i + a.i * b.r)};
 }
+// c - a b on double2
+__device__ __forceinline__ double2 zmsub2(double2 c, double2 a, double2 b) {
+    return make_double2(fma(a.y, b.y, fma(-a.x, b.x, c.x)), fma(-a.y, b.x, fma(-a.x, b.y, c.y)));
+}
+
 // 1 / b, scaled by the larger of |b.r|, |b.i| (no spurious overflow)
 __device__ __forceinline__ zd zrecip(zd b) {
     double s = fmax(fabs(b.r), fabs(b.i));
@@ -291,6 +298,324 @@ __global__ void __launch_bounds__(ZCL_NT, 1) k_zleaf_cl(double *__restrict__ Wr,
     }
 }
 
+// The leaf of up to 8192 rows, in the form of the real one (leaf.cuh, lu_kernels.cu):
+// a cluster holds the rows in registers, one per thread, with implicit
+// pivoting; columns in groups of ZGW = 4, whose pivot rows publish their other
+// columns once per group.  A candidate is {position, key}, a_pj, a_p,j+1, ...
+// with the key abs2; a column whose largest abs2 is not finite repeats its search
+// with abs (_lu_pivot, src/lapack/factorizations.jl:92-107).  Bound: latency of
+// the column steps, as the real leaf.
+constexpr int ZGW = 4, ZNG = ZLEAF / ZGW;
+template <int NT>
+__global__ void __launch_bounds__(NT, 1)
+k_zleaf_reg(double *__restrict__ Wr, double *__restrict__ Wi, i64 ld, int m, int w, i64 gofs,
+            int64_t *__restrict__ ipiv, int64_t *__restrict__ info, LeafPanel pn) {
+    cgz::cluster_group cl = cgz::this_cluster();
+    const int CS = (int)cl.num_blocks(), cr = (int)cl.block_rank();
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, half = lane & 15;
+    constexpr int NW = NT / 32, PERMAX = 1 + ZGW;
+    constexpr int MOVE_PW = (2 * ZLEAF + NW - 1) / NW, MOVE_CH = LEAF_MAX_OTHER / 32;
+    extern __shared__ __align__(16) unsigned char zl_smem[];  // 32 rows x 144 bytes per warp
+    __shared__ double2 s_cand[2][NW][PERMAX];
+    __shared__ double2 s_slot[2][16][PERMAX];
+    __shared__ double2 s_right[ZGW][ZLEAF], s_stage[ZGW][ZLEAF], s_u[ZGW][ZLEAF];
+    __shared__ __align__(8) uint64_t s_xbar[2], s_rbar;
+    __shared__ int s_piv[ZLEAF], s_info, s_skip, s_mcnt;
+    __shared__ int2 s_mv[2 * ZLEAF];
+    if (t == 0) {
+        s_info = 0;
+        s_mcnt = 0;
+        s_skip = aborted(pn.abort) ? 1 : 0;
+        mbar_init(&s_xbar[0], 1);
+        mbar_init(&s_xbar[1], 1);
+        mbar_init(&s_rbar, 1);
+        fence_barrier_init();
+    }
+    const int G = CS * NT, i0 = cr * NT + t;
+    int pos = i0 < m ? i0 : -1;
+    double2 r[ZLEAF];
+#pragma unroll
+    for (int c = 0; c < ZLEAF; ++c) r[c] = make_double2(0.0, 0.0);
+    const bool vec_ok = w == ZLEAF && ld % 2 == 0 && (((uintptr_t)Wr | (uintptr_t)Wi) % 16 == 0);
+    unsigned char *tr = zl_smem + warp * (32 * 144);
+    const int trow = lane >> 3, tchk = lane & 7;
+    if (vec_ok) {
+        double2 x[2][8];
+#pragma unroll
+        for (int pl = 0; pl < 2; ++pl)
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+                const int i = i0 - lane + it * 4 + trow;
+                x[pl][it] = make_double2(0.0, 0.0);
+                if (i < m) x[pl][it] = *(const double2 *)((pl ? Wi : Wr) + (i64)i * ld + 2 * tchk);
+            }
+#pragma unroll
+        for (int pl = 0; pl < 2; ++pl) {
+#pragma unroll
+            for (int it = 0; it < 8; ++it) *(double2 *)(tr + (it * 4 + trow) * 144 + tchk * 16) = x[pl][it];
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < ZLEAF; c += 2) {
+                const double2 v = *(const double2 *)(tr + lane * 144 + c * 8);
+                if (pl == 0) { r[c].x = v.x; r[c + 1].x = v.y; }
+                else { r[c].y = v.x; r[c + 1].y = v.y; }
+            }
+            __syncwarp();
+        }
+    } else if (pos >= 0) {
+#pragma unroll
+        for (int c = 0; c < ZLEAF; ++c)
+            if (c < w) r[c] = make_double2(Wr[(i64)i0 * ld + c], Wi[(i64)i0 * ld + c]);
+    }
+    // barriers exist, and every row is read, before any CTA pushes or stores
+    if (CS > 1) cl.sync();
+    else __syncthreads();
+    const int skip = (CS > 1) ? *cl.map_shared_rank(&s_skip, 0) : s_skip;
+    if (skip) {
+        if (CS > 1) cl.sync();
+        return;
+    }
+    bool dead = false;  // an exchange wait gave up: nothing is stored, every cluster barrier still met
+    const int q = m < w ? m : w;
+    const uint32_t to_cta = cluster_map_u32(&s_xbar[0], half < CS ? half : 0) - smem_u32(&s_xbar[0]);
+    int xc = 0;         // exchanges so far
+#pragma unroll 1
+    for (int s = 0; s < ZNG; ++s) {
+        const int j0 = s * ZGW;
+        uint32_t live = 0;
+#pragma unroll
+        for (int jj = 0; jj < ZGW; ++jj) {
+            const int j = j0 + jj;
+            if (j >= q) break;
+            const int PER = 1 + ZGW - jj;
+            const double2(*cand)[PERMAX] = nullptr;
+            int wq = 0;
+            double2 cy;   // this lane's candidate's reciprocal
+#pragma unroll 1
+            for (int round = 0; round < 2; ++round, ++xc) {
+                const int par = xc & 1;
+                const double2 a = r[jj];
+                const double key = round == 0 ? a.x * a.x + a.y * a.y : hypot(a.x, a.y);
+                const uint64_t kb = step_key(key, pos, j);
+                {
+                    const uint32_t wm = warp_winner<double>(kb, pos >= j ? pos : INT_MAX);
+                    if (wm == 0 ? lane == 0 : ((wm >> lane) & 1)) {
+                        double2 *c = s_cand[par][warp];
+                        c[0] = make_double2(__hiloint2double(0, wm ? pos : INT_MAX), __longlong_as_double((long long)kb));
+#pragma unroll
+                        for (int e = jj; e < ZGW; ++e) c[1 + e - jj] = r[e];
+                    }
+                }
+                __syncthreads();
+                auto list_winner = [&](const double2(*l)[PERMAX], int n, uint64_t &ck) -> int {
+                    int cp = INT_MAX;
+                    ck = 0;
+                    if (lane < n) {
+                        const double2 h = l[lane][0];
+                        cp = __double2loint(h.x);
+                        ck = (uint64_t)__double_as_longlong(h.y);
+                    }
+                    const uint32_t wm = warp_winner<double>(ck, cp);
+                    return wm ? __ffs(wm) - 1 : 0;
+                };
+                uint64_t ck;
+                if (CS > 1 && !dead) {
+                    if (t == 0) mbar_arrive_expect_tx(&s_xbar[par], (uint32_t)(CS * 16 * PER));
+                    if (warp < PER) {
+                        const int wn = list_winner(s_cand[par], NW, ck);
+                        if (lane < CS)
+                            st_async_v4(smem_u32(s_slot[par][cr]) + 16u * warp + to_cta,
+                                        reinterpret_cast<const uint4 *>(s_cand[par][wn])[warp],
+                                        smem_u32(&s_xbar[par]) + to_cta);
+                    }
+                    if (!mbar_wait(&s_xbar[par], (uint32_t)((xc >> 1) & 1), pn.abort, 1)) dead = true;
+                }
+                cand = (CS > 1) ? s_slot[par] : s_cand[par];
+                const int nc = CS > 1 ? CS : NW;
+                zd rec = zrecip(lane < nc ? zd{cand[lane][1].x, cand[lane][1].y} : zd{1.0, 0.0});
+                cy = make_double2(rec.r, rec.i);
+                wq = list_winner(cand, nc, ck);
+                const uint64_t best = (uint64_t)__double_as_longlong(cand[wq][0].y);
+                // the CTA decides together: after a wait that gave up its warps may
+                // have read different slots
+                if (!__syncthreads_or(round == 0 && best >= 0x7ff0000000000000ull)) {
+                    ++xc;
+                    break;
+                }
+            }
+            const double2 dinv = make_double2(__shfl_sync(0xffffffffu, cy.x, wq), __shfl_sync(0xffffffffu, cy.y, wq));
+            const int wp = __double2loint(cand[wq][0].x);
+            double2 v[ZGW];
+#pragma unroll
+            for (int c = jj; c < ZGW; ++c) v[c] = cand[wq][1 + c - jj];
+            const bool ok = !(is_zero(v[jj].x) && is_zero(v[jj].y));
+            if (ok) live |= 1u << jj;
+            if (t == 0) {
+                s_piv[j] = wp;
+                if (!ok && s_info == 0) s_info = j + 1;
+            }
+            const int p = pos;
+            pos = p == wp ? j : (p == j ? wp : p);
+            if (ok && p >= j && p != wp) {
+                const zd l = zmul({r[jj].x, r[jj].y}, {dinv.x, dinv.y});
+                r[jj] = make_double2(l.r, l.i);
+#pragma unroll
+                for (int c = jj + 1; c < ZGW; ++c) r[c] = zmsub2(r[c], r[jj], v[c]);
+            }
+        }
+        const int np = min(ZGW, q - j0), nblk = ZNG - 1 - s;
+        if (np > 0 && nblk > 0 && j0 + np < w) {
+            const int rem = nblk * ZGW, nch = ZGW + rem;
+            if (CS > 1 && t == 0 && !dead) mbar_arrive_expect_tx(&s_rbar, (uint32_t)(np * nch * 16));
+            const int kk = pos - j0;
+            const bool own = pos >= j0 && kk < np;
+            if (own) {
+                double2 *dst = (CS > 1) ? s_stage[kk] : s_right[kk];
+#pragma unroll
+                for (int b = 0; b < ZNG; ++b)
+                    if (b <= nblk)
+#pragma unroll
+                        for (int c = 0; c < ZGW; ++c) dst[b * ZGW + c] = r[b * ZGW + c];
+            }
+            if (CS > 1) {
+                uint32_t om = __ballot_sync(0xffffffffu, own);
+                while (om) {
+                    const int src = __ffs(om) - 1;
+                    om &= om - 1;
+                    const int ks = __shfl_sync(0xffffffffu, kk, src);
+                    __syncwarp();
+                    if (half < CS && !dead)
+                        for (int c = lane >> 4; c < nch; c += 2)
+                            st_async_v4(smem_u32(s_right[ks]) + 16u * c + to_cta,
+                                        reinterpret_cast<const uint4 *>(s_stage[ks])[c], smem_u32(&s_rbar) + to_cta);
+                }
+                if (warp == 0 && !dead && !mbar_wait(&s_rbar, (uint32_t)(s & 1), pn.abort, 1)) dead = true;
+            } else {
+                __syncthreads();
+            }
+            const bool full = live == (1u << ZGW) - 1;
+            if (warp == 0 && lane < rem) {
+                double2 x[ZGW];
+#pragma unroll
+                for (int k = 0; k < ZGW; ++k) x[k] = k < np ? s_right[k][ZGW + lane] : make_double2(0.0, 0.0);
+#pragma unroll
+                for (int p = 0; p < ZGW; ++p)
+#pragma unroll
+                    for (int k = p + 1; k < ZGW; ++k)
+                        if (full || (((live >> p) & 1) && k < np)) x[k] = zmsub2(x[k], s_right[k][p], x[p]);
+#pragma unroll
+                for (int k = 0; k < ZGW; ++k) s_u[k][lane] = x[k];
+            }
+            __syncthreads();
+            const bool act = pos >= j0 + np;
+#pragma unroll
+            for (int b = 0; b < ZNG - 1; ++b) {
+                if (b < nblk) {
+                    if (act) {
+#pragma unroll
+                        for (int p = 0; p < ZGW; ++p)
+                            if ((live >> p) & 1)
+#pragma unroll
+                                for (int c = 0; c < ZGW; ++c)
+                                    r[(b + 1) * ZGW + c] = zmsub2(r[(b + 1) * ZGW + c], r[p], s_u[p][b * ZGW + c]);
+                    } else if (own) {
+#pragma unroll
+                        for (int c = 0; c < ZGW; ++c) r[(b + 1) * ZGW + c] = s_u[kk][b * ZGW + c];
+                    }
+                }
+            }
+        }
+        // the finished group moves behind the unfinished columns
+        double2 f[ZGW];
+#pragma unroll
+        for (int c = 0; c < ZGW; ++c) f[c] = r[c];
+#pragma unroll
+        for (int c = 0; c < ZLEAF - ZGW; ++c) r[c] = r[c + ZGW];
+#pragma unroll
+        for (int c = 0; c < ZGW; ++c) r[ZLEAF - ZGW + c] = f[c];
+    }
+    dead = __syncthreads_or(dead);
+    if (!dead && cr == 0) {
+        if (t < q) ipiv[gofs + t] = gofs + s_piv[t] + 1;
+        if (t == 0 && s_info != 0 && *info == 0) *info = gofs + s_info;
+    }
+    const bool moved = !dead && pos >= 0 && pos != i0;
+    if (!dead) {
+        if (moved && pn.map) {
+            const int slot = atomicAdd(&s_mcnt, 1);
+            s_mv[slot] = make_int2(pos, i0);
+        }
+        if (vec_ok) {
+#pragma unroll
+            for (int pl = 0; pl < 2; ++pl) {
+#pragma unroll
+                for (int c = 0; c < ZLEAF; c += 2)
+                    *(double2 *)(tr + lane * 144 + c * 8) =
+                        pl == 0 ? make_double2(r[c].x, r[c + 1].x) : make_double2(r[c].y, r[c + 1].y);
+                __syncwarp();
+#pragma unroll
+                for (int it = 0; it < 8; ++it) {
+                    const int dst = __shfl_sync(0xffffffffu, pos, it * 4 + trow);
+                    if (dst >= 0)
+                        *(double2 *)((pl ? Wi : Wr) + (i64)dst * ld + 2 * tchk) =
+                            *(const double2 *)(tr + (it * 4 + trow) * 144 + tchk * 16);
+                }
+                __syncwarp();
+            }
+        } else if (pos >= 0) {
+#pragma unroll
+            for (int c = 0; c < ZLEAF; ++c)
+                if (c < w) {
+                    Wr[(i64)pos * ld + c] = r[c].x;
+                    Wi[(i64)pos * ld + c] = r[c].y;
+                }
+        }
+    }
+    if (pn.map) {
+        // the interchanges on the panel's other columns and on its row map, as
+        // the real leaf: read, meet, write
+        const int mapv = moved ? pn.map[pn.map_off + i0] : 0;
+        __syncthreads();
+        const int cnt = s_mcnt, nother = pn.nother;
+        double *const br = Wr - pn.leaf_c0, *const bi = Wi - pn.leaf_c0;
+        int off[MOVE_CH];
+#pragma unroll
+        for (int ci = 0; ci < MOVE_CH; ++ci) {
+            const int oc = ci * 32 + lane;
+            off[ci] = oc >= nother ? -1 : (oc < pn.left_n ? pn.pc_lo + oc : pn.right_lo + (oc - pn.left_n));
+        }
+        double2 vals[MOVE_PW][MOVE_CH];
+#pragma unroll
+        for (int mi = 0; mi < MOVE_PW; ++mi) {
+            const int mv = warp + mi * NW;
+            if (mv < cnt) {
+                const i64 src = (i64)s_mv[mv].y * ld;
+#pragma unroll
+                for (int ci = 0; ci < MOVE_CH; ++ci)
+                    if (off[ci] >= 0) vals[mi][ci] = make_double2(br[src + off[ci]], bi[src + off[ci]]);
+            }
+        }
+        if (CS > 1) cl.sync();
+        else __syncthreads();
+#pragma unroll
+        for (int mi = 0; mi < MOVE_PW; ++mi) {
+            const int mv = warp + mi * NW;
+            if (mv < cnt) {
+                const i64 dst = (i64)s_mv[mv].x * ld;
+#pragma unroll
+                for (int ci = 0; ci < MOVE_CH; ++ci)
+                    if (off[ci] >= 0) {
+                        br[dst + off[ci]] = vals[mi][ci].x;
+                        bi[dst + off[ci]] = vals[mi][ci].y;
+                    }
+            }
+        }
+        if (moved) pn.map[pn.map_off + pos] = mapv;
+    } else if (CS > 1) {
+        cl.sync();  // every push into a CTA that gave up has landed before its shared memory goes
+    }
+}
+
 // laswp: the interchanges ipiv[k0 .. k0+cnt) (global 1-based rows, cnt <= 16)
 // on columns [c_lo, c_hi) of both planes.  Their net effect is at most 2 cnt
 // row moves (dst <- src); thread 0 of each CTA folds the sequence into that
@@ -348,30 +673,51 @@ __global__ void k_zlaswp(double *__restrict__ Wr, double *__restrict__ Wi, i64 l
 }
 
 // B (t x N at (Br, Bi), ld) <- L^-1 B, L the unit lower t x t block at (Lr, Li),
-// t <= ZT_MAXT: a CTA per 32 columns, the t x 32 tile in shared memory; once
-// row i is final every later row r is updated, x_r -= l_ri x_i (8 row groups of
-// a warp each, its lanes across the columns: l_ri is one broadcast load).
-constexpr int ZT_NT = 256, ZT_CW = 32, ZT_MAXT = 128;
+// t <= ZT_MAXT: a CTA per ZT_CW columns, its columns and L's strict lower
+// triangle in shared memory (loaded once, everything in flight together).  By
+// blocks of 8 rows: the block by substitution, a column per thread, then its
+// products subtracted from the rows below.  Bound: latency of the 2 t / 8 steps.
+constexpr int ZT_NT = 256, ZT_CW = 16, ZT_MAXT = 64, ZT_RB = 8;
 __global__ void __launch_bounds__(ZT_NT) k_ztrsm_lunit(const double *__restrict__ Lr, const double *__restrict__ Li,
                                                        double *__restrict__ Br, double *__restrict__ Bi, i64 ld,
                                                        int t, i64 N) {
-    extern __shared__ double2 zt[];  // [t][ZT_CW]
-    const int tid = threadIdx.x, cl = tid & (ZT_CW - 1), rg = tid / ZT_CW;
+    extern __shared__ double2 zt[];  // [t][ZT_CW], then L [t][ZT_MAXT + 1]
+    double2 *Ls = zt + t * ZT_CW;
+    constexpr int LP = ZT_MAXT + 1;
+    const int tid = threadIdx.x, cl = tid % ZT_CW, rg = tid / ZT_CW;
     constexpr int RG = ZT_NT / ZT_CW;
     const i64 c0 = (i64)blockIdx.x * ZT_CW;
     const bool live = c0 + cl < N;
+#pragma unroll 8
+    for (int e = tid; e < t * ZT_MAXT; e += ZT_NT) {
+        const int i = e / ZT_MAXT, p = e % ZT_MAXT;
+        if (p < i) Ls[i * LP + p] = make_double2(Lr[(i64)i * ld + p], Li[(i64)i * ld + p]);
+    }
+#pragma unroll 4
     for (int r = rg; r < t; r += RG)
         zt[r * ZT_CW + cl] = live ? make_double2(Br[(i64)r * ld + c0 + cl], Bi[(i64)r * ld + c0 + cl])
                                   : make_double2(0.0, 0.0);
     __syncthreads();
-    for (int i = 0; i < t - 1; ++i) {
-        const double2 xv = zt[i * ZT_CW + cl];
-        const zd xi = {xv.x, xv.y};
-        for (int r = i + 1 + rg; r < t; r += RG) {
-            const zd l = {__ldg(Lr + (i64)r * ld + i), __ldg(Li + (i64)r * ld + i)};
-            const double2 bv = zt[r * ZT_CW + cl];
-            const zd v = zmsub({bv.x, bv.y}, l, xi);
-            zt[r * ZT_CW + cl] = make_double2(v.r, v.i);
+    for (int b = 0; b < t; b += ZT_RB) {
+        if (tid < ZT_CW) {
+            double2 x[ZT_RB];
+#pragma unroll
+            for (int i = 0; i < ZT_RB; ++i) x[i] = b + i < t ? zt[(b + i) * ZT_CW + tid] : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int p = 0; p < ZT_RB; ++p)
+#pragma unroll
+                for (int i = p + 1; i < ZT_RB; ++i)
+                    if (b + i < t) x[i] = zmsub2(x[i], Ls[(b + i) * LP + b + p], x[p]);
+#pragma unroll
+            for (int i = 1; i < ZT_RB; ++i)
+                if (b + i < t) zt[(b + i) * ZT_CW + tid] = x[i];
+        }
+        __syncthreads();
+        for (int r = b + ZT_RB + rg; r < t; r += RG) {
+            double2 v = zt[r * ZT_CW + cl];
+#pragma unroll
+            for (int p = 0; p < ZT_RB; ++p) v = zmsub2(v, Ls[r * LP + b + p], zt[(b + p) * ZT_CW + cl]);
+            zt[r * ZT_CW + cl] = v;
         }
         __syncthreads();
     }
@@ -435,10 +781,13 @@ struct ZRun {
     int64_t *ipiv, *info;
     double *neg;  // -Ai scratch (m x (nb + 2))
     i64 nb;       // panel width (lu_factor's blocksize, 128 by default)
+    // the current panel [pf, pl) and its row map (null: every leaf's interchanges
+    // go to all other columns at once)
+    i64 pf = 0, pl = 0;
+    int *map = nullptr, *list = nullptr, *listcnt = nullptr;
 };
 
-// C -= A B on complex planes (row-major, common ld): four FP64 tensor-core
-// products, the imaginary part of A negated once into scratch.
+// C -= A B on complex planes (row-major, common ld).
 static void zgemm_minus(ZRun &R, i64 cr, i64 cc, i64 ar, i64 ac, i64 br, i64 bc, i64 M, i64 N, i64 K) {
     if (M <= 0 || N <= 0 || K <= 0) return;
     cudaStream_t s = R.h->stream;
@@ -446,6 +795,11 @@ static void zgemm_minus(ZRun &R, i64 cr, i64 cc, i64 ar, i64 ac, i64 br, i64 bc,
     double *Cr = R.Wr + cr * ld + cc, *Ci = R.Wi + cr * ld + cc;
     const double *Ar = R.Wr + ar * ld + ac, *Ai = R.Wi + ar * ld + ac;
     const double *Bre = R.Wr + br * ld + bc, *Bim = R.Wi + br * ld + bc;
+    if (zgemm_dmma_applicable(Ar, Ai, Bre, Bim, ld)) {
+        launch_zgemm_dmma(Cr, Ci, Ar, Ai, Bre, Bim, ld, M, N, K, s);
+        return;
+    }
+    // an odd column offset (an odd panel width): the plain kernel, plane by plane
     const i64 ldn = zrup(K, 2);
     k_negate<<<(unsigned)((M * K + 255) / 256), 256, 0, s>>>(Ai, ld, R.neg, ldn, M, K);
     OXI_LAUNCH_CHECK();
@@ -458,15 +812,15 @@ static void zgemm_minus(ZRun &R, i64 cr, i64 cc, i64 ar, i64 ac, i64 br, i64 bc,
 static void ztrsm(ZRun &R, i64 r0, i64 c0, int t, i64 bc, i64 N) {
     if (t <= 1 || N <= 0) return;
     const i64 ld = R.ld;
-    if (t > ZT_MAXT) {  // a wider block (blocksize > 128): the top rows, their update of the rest, the rest
+    if (t > ZT_MAXT) {  // a wider block: the top rows, their update of the rest, the rest
         const int h = ZT_MAXT;
         ztrsm(R, r0, c0, h, bc, N);
         zgemm_minus(R, r0 + h, bc, r0 + h, c0, r0, bc, t - h, N, h);
         ztrsm(R, r0 + h, c0 + h, t - h, bc, N);
         return;
     }
-    const int smem = (int)(sizeof(double2) * t * ZT_CW);
-    set_max_dyn_smem((const void *)k_ztrsm_lunit, (int)(sizeof(double2) * ZT_MAXT * ZT_CW));
+    const int smem = (int)(sizeof(double2) * t * (ZT_CW + ZT_MAXT + 1));
+    set_max_dyn_smem((const void *)k_ztrsm_lunit, (int)(sizeof(double2) * ZT_MAXT * (ZT_CW + ZT_MAXT + 1)));
     k_ztrsm_lunit<<<(unsigned)((N + ZT_CW - 1) / ZT_CW), ZT_NT, smem, R.h->stream>>>(
         R.Wr + r0 * ld + c0, R.Wi + r0 * ld + c0, R.Wr + r0 * ld + bc, R.Wi + r0 * ld + bc, ld, t, N);
     OXI_LAUNCH_CHECK();
@@ -481,6 +835,32 @@ static void zlaswp(ZRun &R, i64 k0, int cnt, i64 c_lo, i64 c_hi, i64 skip_lo, i6
     OXI_LAUNCH_CHECK();
 }
 
+constexpr i64 ZREG_MAXM = 16 * 512;  // rows of the register leaf
+template <int NT>
+static void launch_zleaf_reg(ZRun &R, i64 c0, i64 mrows, int nc, LeafPanel pn) {
+    const int cs = (int)((mrows + NT - 1) / NT);
+    auto kern = k_zleaf_reg<NT>;
+    constexpr int smem = (NT / 32) * 32 * 144;
+    set_max_dyn_smem((const void *)kern, smem);
+    if (cs > 8) OXI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cs);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = R.h->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    ProfScope ps(KC_LEAF, R.h->stream, 0.0, 32.0 * (double)mrows * nc);
+    OXI_CUDA(cudaLaunchKernelEx(&cfg, kern, R.Wr + c0 * R.ld + c0, R.Wi + c0 * R.ld + c0, R.ld, (int)mrows, nc, c0, R.ipiv,
+                                R.info, pn));
+    count_launch();
+}
+
 // _lu_panel! on columns [c0, c0+nc), rows [c0, m): the leaf's interchanges go
 // to every other column of the matrix right after it (the reference applies
 // them to the panel's columns in the recursion and to the rest per panel; each
@@ -488,6 +868,23 @@ static void zlaswp(ZRun &R, i64 k0, int cnt, i64 c_lo, i64 c_hi, i64 skip_lo, i6
 static void zpanel(ZRun &R, i64 c0, i64 nc) {
     const i64 mrows = R.m - c0;
     if (mrows <= 0 || nc <= 0) return;
+    if (nc <= ZLEAF && mrows <= ZREG_MAXM) {
+        LeafPanel pn;
+        if (R.map) {
+            pn.left_n = (int)(c0 - R.pf);
+            pn.nother = (int)((c0 - R.pf) + (R.pl - c0 - nc));
+            pn.pc_lo = (int)R.pf;
+            pn.right_lo = (int)(c0 + nc);
+            pn.leaf_c0 = (int)c0;
+            pn.map = R.map;
+            pn.map_off = (int)(c0 - R.pf);
+        }
+        pn.abort = cur_abort();
+        if (mrows <= 16 * 256) launch_zleaf_reg<256>(R, c0, mrows, (int)nc, pn);
+        else launch_zleaf_reg<512>(R, c0, mrows, (int)nc, pn);
+        if (!R.map) zlaswp(R, c0, (int)std::min<i64>(nc, mrows), 0, R.n, c0, c0 + nc);
+        return;
+    }
     if (nc <= ZLEAF) {
         if (mrows <= (i64)ZCL_MAXRP * 16) {
             // rows over a cluster of up to 16 CTAs, in shared memory
@@ -531,9 +928,30 @@ static void zpanel(ZRun &R, i64 c0, i64 nc) {
 
 static void zgetrf_planes(ZRun &R) {
     const i64 q = std::min(R.m, R.n);
+    int *map0 = nullptr;
+    if (R.nb <= LEAF_MAX_OTHER) {
+        map0 = (int *)R.h->rowmap_ws.get(sizeof(int) * (size_t)(R.m + 4 * R.nb + 64));
+        R.list = map0 + R.m;
+        R.listcnt = R.list + 4 * R.nb;
+    }
     for (i64 f = 0; f < q; f += R.nb) {
         const i64 l = std::min(q, f + R.nb);
+        // a panel of register leaves applies its interchanges to the columns
+        // outside it once, composed
+        int *const map = R.m - f <= ZREG_MAXM ? map0 : nullptr;
+        R.map = map;
+        R.pf = f;
+        R.pl = l;
+        if (map) launch_rowmap_init(map, R.m - f, R.listcnt, R.h->stream);
         zpanel(R, f, l - f);
+        if (map) {
+            launch_rowmap_extract(map, R.m - f, R.list, R.listcnt, R.h->stream);
+            const int maxcnt = (int)std::min<i64>(2 * (l - f), R.m - f);
+            for (double *W : {R.Wr, R.Wi}) {
+                launch_rowmoves_big<double>(W, R.ld, f, R.list, R.listcnt, maxcnt, 0, f, R.h->stream);
+                launch_rowmoves_big<double>(W, R.ld, f, R.list, R.listcnt, maxcnt, l, R.n, R.h->stream);
+            }
+        }
         if (l >= R.n) continue;
         ztrsm(R, f, f, (int)(l - f), l, R.n - l);
         if (l >= R.m) continue;
