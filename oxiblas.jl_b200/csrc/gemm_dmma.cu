@@ -2,9 +2,12 @@
 //
 // sm_100a has no FP64 kind for tcgen05.mma; the FP64 tensor path is DMMA
 // (mma.sync.aligned.m16n8k4 .f64), which this kernel feeds from TMA.
-// CTA tile 128 x 64, k slab 16, 4-stage mbarrier pipeline:
-//   warp 8      producer: one lane issues the TMA loads of each stage;
-//   warps 0..7  consumers: 4 x 2 warp grid, 32 x 32 per warp (2 x 4 MMAs per k4).
+// CTA tile 128 x 64, k slab 16, 4-stage mbarrier pipeline, 8 warps in a 4 x 2 grid,
+// 32 x 32 per warp (2 x 4 MMAs per k4).  Thread 0 issues the TMA loads: a slot is
+// refilled one slab after its own, when every warp has left it.  (A producer warp
+// of its own costs the others registers: nine warps a CTA, two CTAs an SM,
+// leave 96 a thread, eight leave 128, which the epilogue's loads in flight need.)
+// The C tile is prefetched into L2 while the slabs run, and read in two batches.
 // A stage holds A[128 x 16] with the 128-byte swizzle (conflict-free fragment
 // loads) and B[16 x 64] as eight 16 x 8 boxes laid side by side (each k row of a
 // box is 64 contiguous bytes, so a fragment load reads 256 contiguous bytes).
@@ -46,7 +49,7 @@ constexpr int A_STAGE_BYTES = BM * BK * 8;  // 16 KB
 constexpr int B_STAGE_BYTES = BK * BN * 8;  // 8 KB
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int NCONSUMER_WARPS = 8;
-constexpr int NTHREADS = (NCONSUMER_WARPS + 1) * 32;
+constexpr int NTHREADS = NCONSUMER_WARPS * 32;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 }  // namespace
 
@@ -77,29 +80,31 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     __syncthreads();
     if (s_skip) return;  // the call was aborted by an earlier wait
 
-    if (warp == NCONSUMER_WARPS) {
-        // ---------------- producer ----------------
-        if (lane == 0) {
-            prefetch_tmap(&tmA);
-            prefetch_tmap(&tmB);
-            for (int kt = 0; kt < KT; ++kt) {
-                const int s = kt % STAGES;
-                if (kt >= STAGES) {
-                    if (!mbar_wait<false>(&empty[s], ((kt / STAGES) + 1) & 1, ab, 2)) break;
-                }
-                uint8_t *sa = smem + s * STAGE_BYTES;
-                uint8_t *sb = sa + A_STAGE_BYTES;
-                mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
-                tma_load_2d(sa, &tmA, &full[s], kt * BK, m0);
+    auto issue = [&](int kt) {  // thread 0: slab kt into its slot
+        const int s = kt % STAGES;
+        uint8_t *sa = smem + s * STAGE_BYTES;
+        uint8_t *sb = sa + A_STAGE_BYTES;
+        mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
+        tma_load_2d(sa, &tmA, &full[s], kt * BK, m0);
 #pragma unroll
-                for (int g = 0; g < BN / 8; ++g)
-                    tma_load_2d(sb + g * (BK * 8 * 8), &tmB, &full[s], n0 + 8 * g, kt * BK);
-            }
+        for (int g = 0; g < BN / 8; ++g)
+            tma_load_2d(sb + g * (BK * 8 * 8), &tmB, &full[s], n0 + 8 * g, kt * BK);
+    };
+    if (threadIdx.x == 0) {
+        prefetch_tmap(&tmA);
+        prefetch_tmap(&tmB);
+        for (int kt = 0; kt < KT && kt < STAGES; ++kt) issue(kt);
+    }
+    {
+        // the C tile towards L2: two 128-byte lines a thread (rows of 512 bytes)
+        const int r = m0 + (int)(threadIdx.x >> 1), c = n0 + (int)(threadIdx.x & 1) * 32;
+        if (r < M) {
+            const double *p = C + (i64)r * ldc + c;
+            if (c < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+            if (c + 16 < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 16));
         }
-        return;
     }
 
-    // ---------------- consumers ----------------
     const int wm = warp & 3, wn = warp >> 2;  // 4 x 2 warps
     const int gid = lane >> 2, tig = lane & 3;
     double acc[2][4][4];
@@ -147,37 +152,48 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
+        if (threadIdx.x == 0 && kt >= 1 && kt - 1 + STAGES < KT) {  // refill the slab before's slot
+            const int pt = kt - 1;
+            // (on a wait that gave up nothing is issued: every warp's next wait gives up too)
+            if (mbar_wait<false>(&empty[pt % STAGES], (pt / STAGES) & 1, ab, 2)) issue(pt + STAGES);
+        }
+        __syncwarp();
     }
 
-    // epilogue: C -= acc.  The eight C pairs of a row are loaded before any is
+    // epilogue: C -= acc.  The C pairs of two rows are loaded before any is
     // used so their round trips overlap (16-byte accesses when aligned).  A
     // symmetric update's tile that crosses the diagonal writes only the
     // elements on and above it (the other triangle stays as it was).
     const bool vec2 = ((ldc & 1) == 0) && ((((uintptr_t)C) & 15) == 0) && !(upper_only && m0 + BM - 1 > n0);
     const int cmin_row = upper_only ? 1 : 0;  // 1: column c is written only when c >= r
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int mt = 0; mt < 2; ++mt) {
+        double2 cv[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = m0 + wm * 32 + mt * 16 + gid + 8 * h;
+            const double *crow = C + (i64)r * ldc;
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const int c = n0 + wn * 32 + nt * 8 + 2 * tig;
+                if (r < M && c + 1 < N && vec2) cv[h][nt] = __ldcs((const double2 *)(crow + c));
+                else {
+                    cv[h][nt].x = (r < M && c < N && (!cmin_row || c >= r)) ? crow[c] : 0.0;
+                    cv[h][nt].y = (r < M && c + 1 < N && (!cmin_row || c + 1 >= r)) ? crow[c + 1] : 0.0;
+                }
+            }
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int r = m0 + wm * 32 + mt * 16 + gid + 8 * h;
             if (r >= M) continue;
             double *crow = C + (i64)r * ldc;
-            double2 cv[4];
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int c = n0 + wn * 32 + nt * 8 + 2 * tig;
-                if (c + 1 < N && vec2) cv[nt] = __ldcs((const double2 *)(crow + c));
-                else {
-                    cv[nt].x = (c < N && (!cmin_row || c >= r)) ? crow[c] : 0.0;
-                    cv[nt].y = (c + 1 < N && (!cmin_row || c + 1 >= r)) ? crow[c + 1] : 0.0;
-                }
-            }
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
                 const int c = n0 + wn * 32 + nt * 8 + 2 * tig;
                 double2 v;
-                v.x = cv[nt].x - acc[mt][nt][2 * h];
-                v.y = cv[nt].y - acc[mt][nt][2 * h + 1];
+                v.x = cv[h][nt].x - acc[mt][nt][2 * h];
+                v.y = cv[h][nt].y - acc[mt][nt][2 * h + 1];
                 if (c + 1 < N && vec2) __stcs((double2 *)(crow + c), v);
                 else {
                     if (c < N && (!cmin_row || c >= r)) crow[c] = v.x;
@@ -185,6 +201,7 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 }
             }
         }
+    }
 }
 
 void launch_gemm_dmma(double *C, i64 ldc, const double *A, i64 lda, const double *B, i64 ldb, i64 M,
@@ -255,24 +272,20 @@ k_zgemm_dmma(const __grid_constant__ CUtensorMap tmAr, const __grid_constant__ C
     __syncthreads();
     if (s_skip) return;
 
-    if (warp == NCONSUMER_WARPS) {
-        if (lane == 0) {
-            for (int kt = 0; kt < KT; ++kt) {
-                const int s = kt % ZST;
-                if (kt >= ZST && !mbar_wait<false>(&empty[s], ((kt / ZST) + 1) & 1, ab, 2)) break;
-                uint8_t *sa = smem + s * ZSTAGE;
-                mbar_arrive_expect_tx(&full[s], ZSTAGE);
-                tma_load_2d(sa, &tmAr, &full[s], kt * BK, m0);
-                tma_load_2d(sa + ZPLANE, &tmAi, &full[s], kt * BK, m0);
+    auto issue = [&](int kt) {
+        const int s = kt % ZST;
+        uint8_t *sa = smem + s * ZSTAGE;
+        mbar_arrive_expect_tx(&full[s], ZSTAGE);
+        tma_load_2d(sa, &tmAr, &full[s], kt * BK, m0);
+        tma_load_2d(sa + ZPLANE, &tmAi, &full[s], kt * BK, m0);
 #pragma unroll
-                for (int g = 0; g < ZN / 8; ++g) {
-                    tma_load_2d(sa + 2 * ZPLANE + g * (BK * 64), &tmBr, &full[s], n0 + 8 * g, kt * BK);
-                    tma_load_2d(sa + 3 * ZPLANE + g * (BK * 64), &tmBi, &full[s], n0 + 8 * g, kt * BK);
-                }
-            }
+        for (int g = 0; g < ZN / 8; ++g) {
+            tma_load_2d(sa + 2 * ZPLANE + g * (BK * 64), &tmBr, &full[s], n0 + 8 * g, kt * BK);
+            tma_load_2d(sa + 3 * ZPLANE + g * (BK * 64), &tmBi, &full[s], n0 + 8 * g, kt * BK);
         }
-        return;
-    }
+    };
+    if (threadIdx.x == 0)
+        for (int kt = 0; kt < KT && kt < ZST; ++kt) issue(kt);
 
     const int wm = warp & 3, wn = warp >> 2;  // 4 x 2 warps: 16 rows x 32 columns each
     const int gid = lane >> 2, tig = lane & 3;
@@ -309,6 +322,12 @@ k_zgemm_dmma(const __grid_constant__ CUtensorMap tmAr, const __grid_constant__ C
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
+        if (threadIdx.x == 0 && kt >= 1 && kt - 1 + ZST < KT) {
+            const int pt = kt - 1;
+            // (on a wait that gave up nothing is issued: every warp's next wait gives up too)
+            if (mbar_wait<false>(&empty[pt % ZST], (pt / ZST) & 1, ab, 2)) issue(pt + ZST);
+        }
+        __syncwarp();
     }
 
     const bool vec2 = ((ldc & 1) == 0) && ((((uintptr_t)Cr) & 15) == 0) && ((((uintptr_t)Ci) & 15) == 0);
