@@ -237,21 +237,100 @@ __global__ void k_resid_part(const double *__restrict__ A, i64 lda, int n, const
     }
 }
 
+// The same partial sums for up to 8 NT8 right-hand sides in ONE pass over A, on
+// the FP64 tensor cores: a warp takes 32 rows, a k step four columns, and the
+// products with x and with |x| (of |A|) share each fragment of A, which comes
+// straight from memory (a fragment is eight 64-byte row segments of a
+// column).  Bound: the FP64 pipe (2 n^2 nr FMAs for A x and |A||x|); at n = 8192 and
+// 16 right-hand sides that is 115 us.
+constexpr int RM_ROWS = 128, RM_COLS = 64, RM_PARTS = RS * NRMAX / 16;
+template <int NT8>
+__global__ void __launch_bounds__(128) k_resid_part_mma(const double *__restrict__ A, i64 lda, int n,
+                                                        const double *__restrict__ X, i64 ldx, int nr,
+                                                        double *__restrict__ pax, double *__restrict__ pden) {
+    constexpr int XP = 8 * NT8 + 4;  // 4 or 12 modulo 16: no bank conflicts of a fragment's loads
+    __shared__ double xs[RM_COLS][XP];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, gid = lane >> 2, tig = lane & 3;
+    const int r0 = blockIdx.x * RM_ROWS + warp * 32 + gid, s = blockIdx.y;
+    const int chunk = ((n + RM_PARTS - 1) / RM_PARTS + 3) / 4 * 4;
+    const int j0 = s * chunk, j1 = min(n, j0 + chunk);
+    double ax[2][NT8][4], den[2][NT8][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int q = 0; q < NT8; ++q)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ax[m][q][e] = den[m][q][e] = 0.0;
+    bool in[2][2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) in[m][hh] = r0 + 16 * m + 8 * hh < n;
+    auto mma = [](double (&c)[4], double a0, double a1, double b) {
+        asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                     : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+                     : "d"(a0), "d"(a1), "d"(b));
+    };
+    for (int c0 = j0; c0 < j1; c0 += RM_COLS) {
+        __syncthreads();
+#pragma unroll
+        for (int e = t; e < RM_COLS * 8 * NT8; e += 128) {
+            const int c = e % RM_COLS, k = e / RM_COLS;
+            xs[c][k] = (c0 + c < j1 && k < nr) ? X[c0 + c + (i64)k * ldx] : 0.0;
+        }
+        __syncthreads();
+        const double *a = A + r0 + (i64)(c0 + tig) * lda;
+#pragma unroll 4
+        for (int k = 0; k < RM_COLS; k += 4) {
+            const bool cin = c0 + k + tig < j1;
+            double av[2][2], b[NT8];
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh)
+                    av[m][hh] = (cin && in[m][hh]) ? __ldcs(a + (i64)k * lda + 16 * m + 8 * hh) : 0.0;
+#pragma unroll
+            for (int q = 0; q < NT8; ++q) b[q] = xs[k + tig][8 * q + gid];
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int q = 0; q < NT8; ++q) {
+                    mma(ax[m][q], av[m][0], av[m][1], b[q]);
+                    mma(den[m][q], fabs(av[m][0]), fabs(av[m][1]), fabs(b[q]));
+                }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int q = 0; q < NT8; ++q)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int i = r0 + 16 * m + 8 * (e >> 1), k = 8 * q + 2 * tig + (e & 1);
+                if (i < n && k < nr) {
+                    pax[((i64)s * 16 + k) * n + i] = ax[m][q][e];
+                    pden[((i64)s * 16 + k) * n + i] = den[m][q][e];
+                }
+            }
+}
+
+// The partial sums are `parts` of kp right-hand sides each.
 // mode 0: R = B - sum(pax), errors into scal[k*4 + {0 cw, 1 rmax, 2 xmax, 3 bmax}], scal[64+k] += r^2
 // mode 1: Y = sum(pax)
 __global__ void k_resid_final(const double *__restrict__ B, i64 ldb, double *__restrict__ R, i64 ldr,
                               const double *__restrict__ X, i64 ldx, int n, int nr, int k0,
                               const double *__restrict__ pax, const double *__restrict__ pden, int mode,
-                              double *__restrict__ scal) {
+                              double *__restrict__ scal, int parts, int kp) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int k = blockIdx.y;
     if (k >= nr) return;
     double cw = 0.0, rabs = 0.0, xabs = 0.0, babs = 0.0, r2 = 0.0;
     if (i < n) {
         double ax = 0.0, den = 0.0;
-        for (int s = 0; s < RS; ++s) {
-            ax += pax[((i64)s * NRMAX + k) * n + i];
-            if (mode == 0) den += pden[((i64)s * NRMAX + k) * n + i];
+#pragma unroll 8
+        for (int s = 0; s < parts; ++s) {
+            ax += pax[((i64)s * kp + k) * n + i];
+            if (mode == 0) den += pden[((i64)s * kp + k) * n + i];
         }
         if (mode == 1) {
             R[i + (i64)k * ldr] = ax;
@@ -443,10 +522,17 @@ static void residual(MixedRun &M, const double *Xin, double *Rout, std::vector<d
     const int n = (int)M.n, nrhs = (int)M.nrhs;
     OXI_CUDA(cudaMemsetAsync(M.scal, 0, sizeof(double) * 128, s));
     ProfScope ps(KC_RESIDUAL, s, 2.0 * (double)n * n * nrhs, 8.0 * (double)n * n);
-    for (int k0 = 0; k0 < nrhs; k0 += NRMAX) {
-        const int nr = std::min(NRMAX, nrhs - k0);
+    // more right-hand sides than one pass of the row kernel takes: the tensor-core
+    // pass (measured at n = 8192, 16 right-hand sides: 660 us in four passes)
+    const int step = nrhs > NRMAX ? 16 : NRMAX;
+    for (int k0 = 0; k0 < nrhs; k0 += step) {
+        const int nr = std::min(step, nrhs - k0);
         dim3 g1(blocks_for((n + 1) / 2, 128), RS);
-        if (nr == 1)
+        dim3 gm((unsigned)((n + RM_ROWS - 1) / RM_ROWS), RM_PARTS);
+        const double *Xk = Xin + (i64)k0 * M.ldx;
+        if (step == 16 && nr > 8) k_resid_part_mma<2><<<gm, 128, 0, s>>>(M.A, M.lda, n, Xk, M.ldx, nr, M.pax, M.pden);
+        else if (step == 16) k_resid_part_mma<1><<<gm, 128, 0, s>>>(M.A, M.lda, n, Xk, M.ldx, nr, M.pax, M.pden);
+        else if (nr == 1)
             k_resid_part<1><<<g1, 128, 0, s>>>(M.A, M.lda, n, Xin + (i64)k0 * M.ldx, M.ldx, nr, M.pax, M.pden);
         else
             k_resid_part<NRMAX><<<g1, 128, 0, s>>>(M.A, M.lda, n, Xin + (i64)k0 * M.ldx, M.ldx, nr, M.pax, M.pden);
@@ -454,7 +540,7 @@ static void residual(MixedRun &M, const double *Xin, double *Rout, std::vector<d
         dim3 g2(blocks_for(n), nr);
         k_resid_final<<<g2, 256, 0, s>>>(M.B + (i64)k0 * M.ldb, M.ldb, Rout + (i64)k0 * M.n, M.n,
                                           Xin + (i64)k0 * M.ldx, M.ldx, n, nr, k0, M.pax, M.pden, 0,
-                                          M.scal);
+                                          M.scal, step == 16 ? RM_PARTS : RS, step);
         OXI_LAUNCH_CHECK();
     }
     double *hs = M.hsc;
@@ -481,7 +567,7 @@ static void matvec(MixedRun &M, const double *x, double *y) {
     k_resid_part<1><<<g1, 128, 0, s>>>(M.A, M.lda, n, x, n, 1, M.pax, nullptr);
     OXI_LAUNCH_CHECK();
     k_resid_final<<<dim3(blocks_for(n), 1), 256, 0, s>>>(nullptr, 0, y, n, nullptr, 0, n, 1, 0, M.pax,
-                                                         nullptr, 1, nullptr);
+                                                         nullptr, 1, nullptr, RS, NRMAX);
     OXI_LAUNCH_CHECK();
 }
 
