@@ -1446,23 +1446,76 @@ template void launch_gemm_simt<float>(float *, i64, const float *, i64, const fl
 // moves it into place once no CTA reads A12 any more), and each CTA then
 // updates its 128 x 64 tile of A22 (K = KW).
 // ---------------------------------------------------------------------------
+// Bound: latency of one CTA's stages (operands, U12's chain, products) and the
+// panel's L2 round trip.  The tile of A22 is requested with the operands, before
+// U12's chain; a thread owns 8 rows x 4 adjacent columns, so the products read
+// shared memory 16 bytes at a time (three loads per 32 FMAs).
 template <int KW>
 __global__ void __launch_bounds__(256, 2) k_panel_rl(float *__restrict__ P, i64 ld, int M, int N,
                                                   float *__restrict__ ubuf) {
-    constexpr int BM = 128, BN = 64;
+    constexpr int BM = 128, BN = 64, AP = KW + 4, UP = BN + 4;
     __shared__ float Ls[KW][KW + 1];
-    __shared__ __align__(16) float Us[KW][BN + 4];
-    __shared__ __align__(16) float As[KW][BM + 4];  // the L21 tile, transposed
+    __shared__ __align__(16) float Us[KW][UP];
+    __shared__ __align__(16) float As[BM][AP];  // the L21 tile
     const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
     const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
-    for (int e = t; e < KW * KW; e += 256) Ls[e / KW][e % KW] = P[(i64)(e / KW) * ld + e % KW];
-    for (int e = t; e < KW * BN; e += 256) {
-        const int i = e / BN, j = e % BN;
-        Us[i][j] = (n0 + j < N) ? P[(i64)i * ld + KW + n0 + j] : 0.f;
+    const bool vec = (ld % 4 == 0) && ((uintptr_t)P % 16 == 0);
+    constexpr int KV = KW / 4, AL = BM * KV / 256;
+    float4 av[AL];
+#pragma unroll
+    for (int q = 0; q < AL; ++q) {
+        const int e = t + 256 * q, r = e / KV, k = 4 * (e % KV);
+        av[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (m0 + r < M) {
+            const float *src = P + (i64)(KW + m0 + r) * ld + k;
+            if (vec) av[q] = *(const float4 *)src;
+            else av[q] = make_float4(src[0], src[1], src[2], src[3]);
+        }
     }
-    for (int e = t; e < BM * KW; e += 256) {
-        const int r = e / KW, k = e % KW;
-        As[k][r] = (m0 + r < M) ? P[(i64)(KW + m0 + r) * ld + k] : 0.f;
+    constexpr int UL = KW * BN / 256;
+    float uv[UL];
+#pragma unroll
+    for (int q = 0; q < UL; ++q) {
+        const int e = t + 256 * q, i = e / BN, j = e % BN;
+        uv[q] = (n0 + j < N) ? P[(i64)i * ld + KW + n0 + j] : 0.f;
+    }
+    constexpr int LL = (KW * KW + 255) / 256;
+    float lv[LL];
+#pragma unroll
+    for (int q = 0; q < LL; ++q) {
+        const int e = t + 256 * q;
+        lv[q] = e < KW * KW ? P[(i64)(e / KW) * ld + e % KW] : 0.f;
+    }
+    // this thread's elements of A22: rows ty 8 .., columns tx 4 ..
+    float c[8][4];
+    const int col = n0 + tx * 4;
+    const bool whole = vec && col + 3 < N;
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        const int r = m0 + ty * 8 + x;
+        const float *src = P + (i64)(KW + r) * ld + KW + col;
+        if (r < M && whole) {
+            const float4 v = *(const float4 *)src;
+            c[x][0] = v.x; c[x][1] = v.y; c[x][2] = v.z; c[x][3] = v.w;
+        } else {
+#pragma unroll
+            for (int y = 0; y < 4; ++y) c[x][y] = (r < M && col + y < N) ? src[y] : 0.f;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < LL; ++q) {
+        const int e = t + 256 * q;
+        if (e < KW * KW) Ls[e / KW][e % KW] = lv[q];
+    }
+#pragma unroll
+    for (int q = 0; q < UL; ++q) {
+        const int e = t + 256 * q;
+        Us[e / BN][e % BN] = uv[q];
+    }
+#pragma unroll
+    for (int q = 0; q < AL; ++q) {
+        const int e = t + 256 * q;
+        *(float4 *)&As[e / KV][4 * (e % KV)] = av[q];
     }
     __syncthreads();
     if (t < BN) {
@@ -1481,33 +1534,36 @@ __global__ void __launch_bounds__(256, 2) k_panel_rl(float *__restrict__ P, i64 
         }
     }
     __syncthreads();
-    float c[8][4];
+#pragma unroll 2
+    for (int k = 0; k < KW; k += 4) {
+        float4 a[8];
 #pragma unroll
-    for (int x = 0; x < 8; ++x)
+        for (int x = 0; x < 8; ++x) a[x] = *(const float4 *)&As[ty * 8 + x][k];
 #pragma unroll
-        for (int y = 0; y < 4; ++y) {
-            const int r = m0 + ty + 16 * x, col = n0 + tx + 16 * y;
-            c[x][y] = (r < M && col < N) ? P[(i64)(KW + r) * ld + KW + col] : 0.f;
+        for (int kk = 0; kk < 4; ++kk) {
+            const float4 b = *(const float4 *)&Us[k + kk][tx * 4];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+                const float ak = kk == 0 ? a[x].x : (kk == 1 ? a[x].y : (kk == 2 ? a[x].z : a[x].w));
+                c[x][0] = fmaf(-ak, b.x, c[x][0]);
+                c[x][1] = fmaf(-ak, b.y, c[x][1]);
+                c[x][2] = fmaf(-ak, b.z, c[x][2]);
+                c[x][3] = fmaf(-ak, b.w, c[x][3]);
+            }
         }
-#pragma unroll 8
-    for (int k = 0; k < KW; ++k) {
-        float a[8], b[4];
-#pragma unroll
-        for (int x = 0; x < 8; ++x) a[x] = As[k][ty + 16 * x];
-#pragma unroll
-        for (int y = 0; y < 4; ++y) b[y] = Us[k][tx + 16 * y];
-#pragma unroll
-        for (int x = 0; x < 8; ++x)
-#pragma unroll
-            for (int y = 0; y < 4; ++y) c[x][y] = fmaf(-a[x], b[y], c[x][y]);
     }
 #pragma unroll
-    for (int x = 0; x < 8; ++x)
+    for (int x = 0; x < 8; ++x) {
+        const int r = m0 + ty * 8 + x;
+        float *dst = P + (i64)(KW + r) * ld + KW + col;
+        if (r < M && whole) {
+            *(float4 *)dst = make_float4(c[x][0], c[x][1], c[x][2], c[x][3]);
+        } else {
 #pragma unroll
-        for (int y = 0; y < 4; ++y) {
-            const int r = m0 + ty + 16 * x, col = n0 + tx + 16 * y;
-            if (r < M && col < N) P[(i64)(KW + r) * ld + KW + col] = c[x][y];
+            for (int y = 0; y < 4; ++y)
+                if (r < M && col + y < N) dst[y] = c[x][y];
         }
+    }
 }
 
 void launch_panel_rl(float *P, i64 ld, int kw, i64 M, i64 N, float *ubuf, cudaStream_t s) {
