@@ -1080,11 +1080,118 @@ __global__ void __launch_bounds__(256) k_trsm_fused(const T *__restrict__ L, i64
     }
 }
 
+// The narrow FP32 solve (a panel's U12 in the mixed factor, on the panels'
+// critical path): 8 columns per CTA, the 32 x 32 diagonal blocks inverted
+// first, one warp each, so that a block row's solve is a product of all threads
+// instead of a 32-step chain of shuffles; each block column of L is requested
+// one block ahead.  Bound: latency of the block rows (three barriers and two
+// 32-step chains each).
+constexpr int TI_CW = 8;
+struct TrsmInvSmem {
+    float D[TF_TMAX / TF_TB][TF_TB][TF_TB + 1];
+    float L[TF_TMAX - TF_TB][TF_TB + 1];
+    float X[TF_TMAX][TI_CW];
+};
+__global__ void __launch_bounds__(256) k_trsm_inv(const float *__restrict__ L, i64 ldl, float *__restrict__ B, i64 ldb,
+                                                  int t, i64 N) {
+    extern __shared__ __align__(16) unsigned char tf_smem[];
+    TrsmInvSmem &S = *reinterpret_cast<TrsmInvSmem *>(tf_smem);
+    constexpr int PRE = (TF_TMAX - TF_TB) * TF_TB / 256;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const i64 c0 = (i64)blockIdx.x * TI_CW;
+    const int cols = (int)((N - c0) < TI_CW ? (N - c0) : TI_CW);
+    const int nblk = (t + TF_TB - 1) / TF_TB;
+    float pre[PRE];
+    auto fetch = [&](int J) {  // L below diagonal block J
+        const int rb = (J + 1) * TF_TB;
+#pragma unroll
+        for (int q = 0; q < PRE; ++q) {
+            const int r = warp + 8 * q;
+            pre[q] = rb + r < t ? L[(i64)(rb + r) * ldl + J * TF_TB + lane] : 0.f;
+        }
+    };
+    fetch(0);
+    if (warp < nblk) {
+        float(*D)[TF_TB + 1] = S.D[warp];
+        const int d0 = warp * TF_TB;
+#pragma unroll
+        for (int i = 0; i < TF_TB; ++i)
+            D[i][lane] = (d0 + i < t && lane < i) ? L[(i64)(d0 + i) * ldl + d0 + lane] : 0.f;
+        __syncwarp();
+        float x[TF_TB];
+#pragma unroll
+        for (int i = 0; i < TF_TB; ++i) x[i] = i == lane ? 1.f : 0.f;
+#pragma unroll
+        for (int p = 0; p < TF_TB; ++p)
+#pragma unroll
+            for (int i = p + 1; i < TF_TB; ++i) x[i] = fmaf(-D[i][p], x[p], x[i]);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < TF_TB; ++i) D[i][lane] = x[i];
+    }
+#pragma unroll
+    for (int e = tid; e < TF_TMAX * TI_CW; e += 256) {
+        const int i = e / TI_CW, c = e % TI_CW;
+        S.X[i][c] = (i < t && c < cols) ? B[(i64)i * ldb + c0 + c] : 0.f;
+    }
+    const int pr = tid / TI_CW, pc = tid % TI_CW;
+    for (int J = 0; J < nblk; ++J) {
+        const int j0 = J * TF_TB, rem = t - j0 - TF_TB;  // rows below the block
+#pragma unroll
+        for (int q = 0; q < PRE; ++q) S.L[warp + 8 * q][lane] = pre[q];
+        __syncthreads();
+        if (J + 1 < nblk) fetch(J + 1);
+        float y0 = 0.f, y1 = 0.f;
+#pragma unroll 8
+        for (int k = 0; k < TF_TB; k += 2) {
+            y0 = fmaf(S.D[J][pr][k], S.X[j0 + k][pc], y0);
+            y1 = fmaf(S.D[J][pr][k + 1], S.X[j0 + k + 1][pc], y1);
+        }
+        __syncthreads();
+        S.X[j0 + pr][pc] = y0 + y1;
+        __syncthreads();
+        if (tid < rem) {
+            float acc[TI_CW];
+#pragma unroll
+            for (int c = 0; c < TI_CW; ++c) acc[c] = 0.f;
+#pragma unroll 8
+            for (int k = 0; k < TF_TB; ++k) {
+                const float l = S.L[tid][k];
+                const float4 a = *(const float4 *)&S.X[j0 + k][0], b = *(const float4 *)&S.X[j0 + k][4];
+                acc[0] = fmaf(l, a.x, acc[0]);
+                acc[1] = fmaf(l, a.y, acc[1]);
+                acc[2] = fmaf(l, a.z, acc[2]);
+                acc[3] = fmaf(l, a.w, acc[3]);
+                acc[4] = fmaf(l, b.x, acc[4]);
+                acc[5] = fmaf(l, b.y, acc[5]);
+                acc[6] = fmaf(l, b.z, acc[6]);
+                acc[7] = fmaf(l, b.w, acc[7]);
+            }
+#pragma unroll
+            for (int c = 0; c < TI_CW; ++c) S.X[j0 + TF_TB + tid][c] -= acc[c];
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int e = tid; e < TF_TMAX * TI_CW; e += 256) {
+        const int i = e / TI_CW, c = e % TI_CW;
+        if (i < t && c < cols) B[(i64)i * ldb + c0 + c] = S.X[i][c];
+    }
+}
+
 template <typename T>
 void launch_trsm_fused(const T *L, i64 ldl, T *B, i64 ldb, int t, i64 N, cudaStream_t s) {
     if (t <= 1 || N <= 0) return;
     ProfScope ps(KC_TRSM_LEAF, s, (double)t * t * N, 2.0 * (double)t * N * sizeof(T));
-    if (N <= 2048) {
+    if constexpr (sizeof(T) == 4) {
+        if (N <= 2048) {
+            set_max_dyn_smem((const void *)k_trsm_inv, (int)sizeof(TrsmInvSmem));
+            k_trsm_inv<<<(unsigned)((N + TI_CW - 1) / TI_CW), 256, sizeof(TrsmInvSmem), s>>>(L, ldl, B, ldb, t, N);
+            OXI_LAUNCH_CHECK();
+            return;
+        }
+    }
+    if (sizeof(T) == 8 && N <= 2048) {
         constexpr int CW = 8;
         const size_t smem = sizeof(T) * ((size_t)TF_TMAX * (CW + 1) + (size_t)TF_TMAX * (TF_TB + 1));
         set_max_dyn_smem((const void *)k_trsm_fused<T, CW>, (int)smem);
