@@ -29,6 +29,7 @@
 #include <climits>
 #include <cstring>
 #include <vector>
+#include "leaf.cuh"
 #include "oxi_internal.h"
 #include "scaling.cuh"
 
@@ -40,6 +41,10 @@ constexpr int NMAX = 256;      // largest order
 constexpr int NQ = NMAX / 32;  // rows per lane in the warp solves
 constexpr int NBMAX = 32;      // largest panel width
 constexpr int MAXRHS = 8;
+// pitch of the staged U12 rows and of the staged panel's columns: 4 or 12 modulo
+// 16, which keeps a DMMA fragment's loads free of bank conflicts
+constexpr int UP = NMAX + 4;
+__host__ __device__ constexpr int panel_pitch(int m) { return (m + 11) / 16 * 16 + 4; }  // >= m
 constexpr int NBUCKET = 8;     // bucket b holds orders 32b+1 .. 32b+32
 constexpr int MODE_GETRF = 0, MODE_GESV = 1, MODE_MIXED = 2;
 }  // namespace bt
@@ -77,8 +82,8 @@ static int batch_smem_layout(int esize, int mode, int n_smem, int nbmax, BatchDe
     int off = 0;
     auto take = [&](int bytes) { const int o = off; off += (bytes + 15) & ~15; return o; };
     const bool global_mode = n_smem < NMAX;
-    const int op = take(global_mode ? NMAX * nbmax * esize : 0);
-    const int ou = take(global_mode ? nbmax * NMAX * esize : 0);
+    const int op = take(global_mode ? panel_pitch(NMAX) * nbmax * esize : 0);
+    const int ou = take(global_mode ? nbmax * UP * esize : 0);
     const int ox = take(mode == MODE_MIXED ? NMAX * MAXRHS * 8 : 0);
     const int orr = take(mode == MODE_MIXED ? NMAX * MAXRHS * 8 : 0);
     const int ow = take(n_smem * n_smem * esize);
@@ -107,8 +112,10 @@ struct Misc {
     // reciprocals of the radix row and column scales: powers of two in
     // [2^-1023, 2^1022], so x * rrow[i] is exactly x / (row scale i)
     double rrow[bt::NMAX], rcol[bt::NMAX];
-    double prow[2][bt::NBMAX];  // register panel: the pivot row and the old row j
-    double vjv[2];
+    // register panel: every warp's candidate, by column parity -- {position, value}
+    // and its row from the active column on
+    double2 cand[2][bt::NW];
+    double crow[2][bt::NW][bt::NBMAX];
     int item, info, bad;
 };
 
@@ -224,7 +231,7 @@ __device__ void panel_lu(T *P, int ldp, int m, int jb, int k, Misc &S) {
 
 // One column of U12 = L11^-1 A12 (unit lower L11 in P, ldp): rows k..k+jb of
 // column wc, forward substitution in registers; the result back to wc and,
-// when su is given, to su[i NMAX] (the staged U12 the update reads).  JB is
+// when su is given, to su[i UP] (the staged U12 the update reads).  JB is
 // the panel width at compile time (JB = jb), or NBMAX with jb <= JB checked
 // per step for a narrower last panel.
 template <typename T, int JB>
@@ -245,7 +252,7 @@ __device__ __forceinline__ void u12_column(T *wc, int k, int jb, const T *P, int
     for (int i = 0; i < JB; ++i) {
         if (i < jb) {
             wc[k + i] = x[i];
-            if (su) su[i * bt::NMAX] = x[i];
+            if (su) su[i * bt::UP] = x[i];
         }
     }
 }
@@ -253,138 +260,185 @@ __device__ __forceinline__ void u12_column(T *wc, int k, int jb, const T *P, int
 // C (m2 x m2, column-major, ldc) -= A B, A m2 x jb (column-major, lda), B jb x m2
 // with element (kk, c) at B[kk bsk + c bsc]: each product accumulated from zero
 // in kk order, then subtracted (gemm!(C, A, B, -1, 1)).  One warp, columns
-// c0..c0+3 of rows r0..r0+32 NU: lane l holds rows r0 + l + 32 u, so every A
+// c0..c0+8 of rows r0..r0+32 NU: lane l holds rows r0 + l + 32 u, so every A
 // load and C access covers 32 consecutive rows (no shared-memory bank
-// conflicts, whole sectors in global memory), and two columns' C elements
-// are loaded before any of them is stored.
-template <typename T, int NU>
-__device__ __forceinline__ void update_tile(const T *Ap, int lda, const T *Bp, int bsk, int bsc, T *Cp,
+// conflicts, whole sectors in global memory), four columns' C elements are
+// loaded before any of them is stored, and with VB (B staged by rows) a
+// column quadruple of B is one 16-byte load.
+template <int NU, bool VB>
+__device__ __forceinline__ void update_tile(const float *Ap, int lda, const float *Bp, int bsk, int bsc, float *Cp,
                                             int ldc, int m2, int jb, int r0, int c0, int lane) {
-    T acc[NU][4];
+    float acc[NU][8];
 #pragma unroll
     for (int u = 0; u < NU; ++u)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = T(0);
+        for (int v = 0; v < 8; ++v) acc[u][v] = 0.0f;
     const int r = r0 + lane;
+    bool in[NU];
+#pragma unroll
+    for (int u = 0; u < NU; ++u) in[u] = r + 32 * u < m2;
+    const float *ap = Ap + r;
+    // staged rows of B reach past column m2: what they hold there only enters
+    // columns that are not stored
+    const float *bp = Bp + c0 * bsc;
+#pragma unroll 2
     for (int kk = 0; kk < jb; ++kk) {
-        T a[NU], b[4];
+        float a[NU], b[8];
 #pragma unroll
-        for (int u = 0; u < NU; ++u) a[u] = (r + 32 * u < m2) ? Ap[(r + 32 * u) + (i64)kk * lda] : T(0);
+        for (int u = 0; u < NU; ++u) a[u] = in[u] ? ap[32 * u] : 0.0f;
+        if constexpr (VB) {
+            const float4 b0 = *(const float4 *)bp, b1 = *(const float4 *)(bp + 4);
+            b[0] = b0.x; b[1] = b0.y; b[2] = b0.z; b[3] = b0.w;
+            b[4] = b1.x; b[5] = b1.y; b[6] = b1.z; b[7] = b1.w;
+        } else {
 #pragma unroll
-        for (int v = 0; v < 4; ++v) b[v] = (c0 + v < m2) ? Bp[(i64)kk * bsk + (i64)(c0 + v) * bsc] : T(0);
+            for (int v = 0; v < 8; ++v) b[v] = (c0 + v < m2) ? bp[v * bsc] : 0.0f;
+        }
 #pragma unroll
         for (int u = 0; u < NU; ++u)
 #pragma unroll
-            for (int v = 0; v < 4; ++v) acc[u][v] = fma(a[u], b[v], acc[u][v]);
+            for (int v = 0; v < 8; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
+        ap += lda;
+        bp += bsk;
     }
 #pragma unroll
-    for (int h = 0; h < 4; h += 2) {  // two columns' C elements loaded before any is stored
-        T cv[NU][2];
+    for (int h = 0; h < 8; h += 4) {
+        float *cp = Cp + r + (c0 + h) * ldc;
+        float cv[NU][4];
 #pragma unroll
-        for (int v = 0; v < 2; ++v)
+        for (int v = 0; v < 4; ++v)
+#pragma unroll
+            for (int u = 0; u < NU; ++u) cv[u][v] = (in[u] && c0 + h + v < m2) ? cp[32 * u + v * ldc] : 0.0f;
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
 #pragma unroll
             for (int u = 0; u < NU; ++u)
-                cv[u][v] = (r + 32 * u < m2 && c0 + h + v < m2) ? Cp[(r + 32 * u) + (i64)(c0 + h + v) * ldc] : T(0);
-#pragma unroll
-        for (int v = 0; v < 2; ++v)
-#pragma unroll
-            for (int u = 0; u < NU; ++u)
-                if (r + 32 * u < m2 && c0 + h + v < m2)
-                    Cp[(r + 32 * u) + (i64)(c0 + h + v) * ldc] = cv[u][v] - acc[u][h + v];
+                if (in[u] && c0 + h + v < m2) cp[32 * u + v * ldc] = cv[u][v] - acc[u][h + v];
     }
+}
+template <int NU>
+__device__ __forceinline__ void update_tile(const float *Ap, int lda, const float *Bp, int bsk, int bsc, float *Cp,
+                                            int ldc, int m2, int jb, int r0, int c0, int lane) {
+    if (bsc == 1) update_tile<NU, true>(Ap, lda, Bp, bsk, bsc, Cp, ldc, m2, jb, r0, c0, lane);
+    else update_tile<NU, false>(Ap, lda, Bp, bsk, bsc, Cp, ldc, m2, jb, r0, c0, lane);
 }
 
 // Unblocked LU of a full panel of JB columns (m <= NT rows, P column-major,
-// ldp) with thread i holding row i in registers: per column one reduction for
-// the pivot (the reference's rule, as panel_lu), the pivot row and the old
-// row j exchanged through shared memory, the rank-1 update on registers -- two
-// barriers a column instead of three and no shared-memory round trip per
-// updated element.  Same operations in the same order as panel_lu.
+// ldp) with thread i holding row i in registers and implicit pivoting: the row
+// stays with its thread, which follows the position the interchanges give it
+// and stores it there at the end.  Per column the warps' arg-max (one redux and
+// a ballot, usually) puts each warp's candidate and its row into shared memory,
+// one barrier, the arg-max over the warps, and the rank-1 update on registers.
+// Same operations in the same order as panel_lu.
 template <typename T, int JB>
 __device__ void panel_lu_reg(T *P, int ldp, int m, int k, Misc &S) {
     using namespace bt;
     const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
-    const bool own = i < m;
+    int pos = i < m ? i : -1;
     T row[JB];
 #pragma unroll
-    for (int c = 0; c < JB; ++c) row[c] = own ? P[i + (i64)c * ldp] : T(0);
+    for (int c = 0; c < JB; ++c) row[c] = pos >= 0 ? P[i + (i64)c * ldp] : T(0);
 #pragma unroll
     for (int j = 0; j < JB; ++j) {
         const int par = j & 1;
-        // candidates: rows below j (a NaN never becomes one: NaN > -1 is false)
-        const double ax = fabs((double)row[j]);
-        const bool cand = own && i > j && ax > -1.0;
-        double bv = cand ? ax : -1.0, bx = cand ? (double)row[j] : 0.0;
-        int bi = cand ? i : INT_MAX;
+        const uint32_t wm = warp_winner<T>(step_key(row[j], pos, j), pos >= j ? pos : INT_MAX);
+        if (wm == 0 ? lane == 0 : ((wm >> lane) & 1)) {
+            S.cand[par][warp] = make_double2(__hiloint2double(0, wm ? pos : INT_MAX), (double)row[j]);
+            T *cr = (T *)S.crow[par][warp];
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const double ov = __shfl_xor_sync(0xffffffffu, bv, off);
-            const double ox = __shfl_xor_sync(0xffffffffu, bx, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-            if (ov > bv || (ov == bv && oi < bi)) {
-                bv = ov;
-                bi = oi;
-                bx = ox;
-            }
-        }
-        if (lane == 0) {
-            S.red_v[par][warp] = bv;
-            S.red_i[par][warp] = bi;
-            S.red_x[par][warp] = bx;
-        }
-        if (i == j) S.vjv[par] = (double)row[j];
-        __syncthreads();
-        bv = S.red_v[par][0];
-        bi = S.red_i[par][0];
-        bx = S.red_x[par][0];
-#pragma unroll
-        for (int w = 1; w < NW; ++w) {
-            const double ov = S.red_v[par][w];
-            const int oi = S.red_i[par][w];
-            if (ov > bv || (ov == bv && oi < bi)) {
-                bv = ov;
-                bi = oi;
-                bx = S.red_x[par][w];
-            }
-        }
-        const double vj = S.vjv[par];
-        const bool below = bi != INT_MAX && bv > fabs(vj);
-        const int p = below ? bi : j;
-        const T d = (T)(below ? bx : vj);
-        if (i == 0) S.piv[k + j] = k + p;
-        if (d == T(0)) {  // zero column: info, no interchange, no elimination
-            if (i == 0 && S.info == 0) S.info = k + j + 1;
-            continue;
-        }
-        double *pa = S.prow[0], *pj = S.prow[1];
-        if (i == p) {
-#pragma unroll
-            for (int c = 0; c < JB; ++c) pa[c] = (double)row[c];
-        }
-        if (p != j && i == j) {
-#pragma unroll
-            for (int c = 0; c < JB; ++c) pj[c] = (double)row[c];
+            for (int c = j; c < JB; ++c) cr[c] = row[c];
         }
         __syncthreads();
-        if (i == j) {
-#pragma unroll
-            for (int c = 0; c < JB; ++c) row[c] = (T)pa[c];
-        } else if (p != j && i == p) {
-#pragma unroll
-            for (int c = 0; c < JB; ++c) row[c] = (T)pj[c];
+        int wq;
+        {
+            int cp = INT_MAX;
+            uint64_t ck = 0;
+            if (lane < NW) {
+                const double2 h = S.cand[par][lane];
+                cp = __double2loint(h.x);
+                ck = step_key((T)h.y, cp, j);
+            }
+            const uint32_t w = warp_winner<T>(ck, cp);
+            wq = w ? __ffs(w) - 1 : 0;
         }
-        if (own && i > j) {
+        const double2 h = S.cand[par][wq];
+        const int p = __double2loint(h.x);
+        const T d = (T)h.y;
+        const T *pa = (const T *)S.crow[par][wq];
+        if (i == 0) {
+            S.piv[k + j] = k + p;
+            if (d == T(0) && S.info == 0) S.info = k + j + 1;  // no interchange, no elimination: p is j
+        }
+        const int q = pos;
+        pos = q == p ? j : (q == j ? p : q);
+        if (d != T(0) && q >= j && q != p) {
             const T l = row[j] / d;
             row[j] = l;
 #pragma unroll
-            for (int c = j + 1; c < JB; ++c) row[c] = fma(-l, (T)pa[c], row[c]);
+            for (int c = j + 1; c < JB; ++c) row[c] = fma(-l, pa[c], row[c]);
         }
     }
-    if (own) {
+    // every thread has read its row long before (the first barrier)
+    if (pos >= 0) {
 #pragma unroll
-        for (int c = 0; c < JB; ++c) P[i + (i64)c * ldp] = row[c];
+        for (int c = 0; c < JB; ++c) P[pos + (i64)c * ldp] = row[c];
     }
     __syncthreads();  // the panel, S.piv and S.info visible to all
+}
+
+// C (rows r0.. of 32, columns c0.. of 16) -= A B on the FP64 tensor cores, one
+// warp: the sums of update_tile in the same order (a DMMA accumulates its four
+// products one after the other), the C elements requested before the products
+// so their round trip overlaps them.  A at Ap[r + kk lda], B at
+// Bp[kk bsk + c bsc]; rows and columns from m2 and steps from jb on are zeros.
+__device__ __forceinline__ void update_tile_dmma(const double *Ap, int lda, const double *Bp, int bsk, int bsc,
+                                                 double *Cp, int ldc, int m2, int jb, int r0, int c0, int lane) {
+    const int gid = lane >> 2, tig = lane & 3;
+    double acc[2][2][4], cv[2][2][4];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                acc[mt][nt][e] = 0.0;
+                const int r = r0 + mt * 16 + gid + 8 * (e >> 1), c = c0 + nt * 8 + 2 * tig + (e & 1);
+                cv[mt][nt][e] = (r < m2 && c < m2) ? Cp[r + c * ldc] : 0.0;
+            }
+    for (int kk = 0; kk < jb; kk += 4) {
+        const int kc = kk + tig;
+        const bool kin = kc < jb;
+        double a[2][2], b[2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int r = r0 + mt * 16 + gid + 8 * hh;
+                a[mt][hh] = (kin && r < m2) ? Ap[r + kc * lda] : 0.0;
+            }
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            const int c = c0 + nt * 8 + gid;
+            b[nt] = (kin && c < m2) ? Bp[kc * bsk + c * bsc] : 0.0;
+        }
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+                asm volatile(
+                    "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                    : "+d"(acc[mt][nt][0]), "+d"(acc[mt][nt][1]), "+d"(acc[mt][nt][2]), "+d"(acc[mt][nt][3])
+                    : "d"(a[mt][0]), "d"(a[mt][1]), "d"(b[nt]));
+    }
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int r = r0 + mt * 16 + gid + 8 * (e >> 1), c = c0 + nt * 8 + 2 * tig + (e & 1);
+                if (r < m2 && c < m2) Cp[r + c * ldc] = cv[mt][nt][e] - acc[mt][nt][e];
+            }
 }
 
 // Right-looking blocked LU of W (n x n, column-major, ldw; shared or global).
@@ -400,7 +454,7 @@ __device__ void lu_blocked(T *W, int ldw, int n, int nb, bool in_smem, T *sP, T 
             ldp = ldw;
         } else {
             P = sP;
-            ldp = m;
+            ldp = panel_pitch(m);
             // a warp per column, its lanes down the rows (coalesced, no index division)
             for (int c = (int)(threadIdx.x >> 5); c < jb; c += NW)
                 load_col(sP + c * ldp, W + k + (i64)(k + c) * ldw, m, (int)(threadIdx.x & 31));
@@ -490,69 +544,109 @@ __device__ void lu_blocked(T *W, int ldw, int n, int nb, bool in_smem, T *sP, T 
             }
         }
         __syncthreads();
-        // A22 -= L21 U12: a warp takes up to 128 rows x 4 columns (update_tile)
+        // A22 -= L21 U12: FP64 by warp tiles of 32 x 16 on the tensor cores, FP32 by
+        // up to 128 rows x 8 columns (update_tile)
         const int m2 = n - c2;
         if (m2 > 0) {
             const T *Ap = P + jb;
             T *Cp = W + c2 + (i64)c2 * ldw;
             const T *Bp = in_smem ? W + k + (i64)c2 * ldw : sU;
-            const int bsk = in_smem ? 1 : NMAX;
+            const int bsk = in_smem ? 1 : UP;
             const int bsc = in_smem ? ldw : 1;
-            const int RB = (m2 + 127) >> 7, tasks = RB * ((m2 + 3) >> 2);
             const int lane = (int)(threadIdx.x & 31);
-            for (int t = (int)(threadIdx.x >> 5); t < tasks; t += NW) {
-                const int r0 = (t % RB) * 128, c0 = (t / RB) * 4;
-                const int nu = min(4, (m2 - r0 + 31) >> 5);  // warp-uniform
-                if (nu == 4) update_tile<T, 4>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
-                else if (nu == 3) update_tile<T, 3>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
-                else if (nu == 2) update_tile<T, 2>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
-                else update_tile<T, 1>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
+            if constexpr (sizeof(T) == 8) {
+                const int RB = (m2 + 31) >> 5, tasks = RB * ((m2 + 15) >> 4);
+                for (int t = (int)(threadIdx.x >> 5); t < tasks; t += NW)
+                    update_tile_dmma(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, (t % RB) * 32, (t / RB) * 16, lane);
+            } else {
+                const int RB = (m2 + 127) >> 7, tasks = RB * ((m2 + 7) >> 3);
+                for (int t = (int)(threadIdx.x >> 5); t < tasks; t += NW) {
+                    const int r0 = (t % RB) * 128, c0 = (t / RB) * 8;
+                    const int nu = min(4, (m2 - r0 + 31) >> 5);  // warp-uniform
+                    if (nu == 4) update_tile<4>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
+                    else if (nu == 3) update_tile<3>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
+                    else if (nu == 2) update_tile<2>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
+                    else update_tile<1>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
+                }
             }
         }
         __syncthreads();
     }
 }
 
+// Steps j0..j1 (inside row block Q: rows 32 Q..) of the substitutions by one
+// warp, y distributed as y[q] = row lane + 32 q; column j0 + c of the factor
+// starts at cols + c ldc.  The row block is a compile-time constant, so a step is
+// one shuffle and one product per row block still open.  Backward: the pivots'
+// reciprocals are taken beforehand, one per lane, and a quotient is the product
+// corrected by its exact remainder (a division where that is not finite).
+template <typename T, int Q>
+__device__ __forceinline__ void forward_steps(const T *cols, int ldc, int j0, int j1, int n, T (&y)[bt::NQ], int lane) {
+    using namespace bt;
+#pragma unroll 4
+    for (int j = j0; j < j1; ++j) {
+        const int lj = j & 31;
+        const T *col = cols + (j - j0) * ldc + lane;
+        const T yj = __shfl_sync(0xffffffffu, y[Q], lj);
+#pragma unroll
+        for (int q = Q; q < NQ; ++q)
+            if (lane + 32 * q < n && (q > Q || lane > lj)) y[q] = fma(-col[32 * q], yj, y[q]);
+    }
+}
+template <typename T, int Q>
+__device__ __forceinline__ void backward_steps(const T *cols, int ldc, int j0, int j1, T (&y)[bt::NQ], int lane) {
+    using namespace bt;
+    const T ul = j0 + lane < j1 ? cols[lane * ldc + j0 + lane] : T(1);
+    const T rl = T(1) / ul;
+#pragma unroll 4
+    for (int j = j1 - 1; j >= j0; --j) {
+        const int lj = j & 31;
+        const T *col = cols + (j - j0) * ldc + lane;
+        const T u = __shfl_sync(0xffffffffu, ul, j - j0), r = __shfl_sync(0xffffffffu, rl, j - j0);
+        const T s = __shfl_sync(0xffffffffu, y[Q], lj);
+        T x = s * r;
+        x = fma(fma(-x, u, s), r, x);
+        if (!isfinite(x)) x = s / u;
+        if (lane == lj) y[Q] = x;
+#pragma unroll
+        for (int q = 0; q <= Q; ++q)
+            if (q < Q || lane < lj) y[q] = fma(-col[32 * q], x, y[q]);
+    }
+}
+// the same with the row block of j0 found at run time
+template <typename T>
+__device__ __forceinline__ void forward_chunk(const T *cols, int ldc, int j0, int j1, int n, T (&y)[bt::NQ], int lane) {
+    switch (j0 >> 5) {
+    case 0: forward_steps<T, 0>(cols, ldc, j0, j1, n, y, lane); break;
+    case 1: forward_steps<T, 1>(cols, ldc, j0, j1, n, y, lane); break;
+    case 2: forward_steps<T, 2>(cols, ldc, j0, j1, n, y, lane); break;
+    case 3: forward_steps<T, 3>(cols, ldc, j0, j1, n, y, lane); break;
+    case 4: forward_steps<T, 4>(cols, ldc, j0, j1, n, y, lane); break;
+    case 5: forward_steps<T, 5>(cols, ldc, j0, j1, n, y, lane); break;
+    case 6: forward_steps<T, 6>(cols, ldc, j0, j1, n, y, lane); break;
+    default: forward_steps<T, 7>(cols, ldc, j0, j1, n, y, lane); break;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void backward_chunk(const T *cols, int ldc, int j0, int j1, T (&y)[bt::NQ], int lane) {
+    switch (j0 >> 5) {
+    case 0: backward_steps<T, 0>(cols, ldc, j0, j1, y, lane); break;
+    case 1: backward_steps<T, 1>(cols, ldc, j0, j1, y, lane); break;
+    case 2: backward_steps<T, 2>(cols, ldc, j0, j1, y, lane); break;
+    case 3: backward_steps<T, 3>(cols, ldc, j0, j1, y, lane); break;
+    case 4: backward_steps<T, 4>(cols, ldc, j0, j1, y, lane); break;
+    case 5: backward_steps<T, 5>(cols, ldc, j0, j1, y, lane); break;
+    case 6: backward_steps<T, 6>(cols, ldc, j0, j1, y, lane); break;
+    default: backward_steps<T, 7>(cols, ldc, j0, j1, y, lane); break;
+    }
+}
+
 // One warp solves L U y = z (unit L) with z, y distributed as y[q] = row lane + 32 q.
 template <typename T>
 __device__ void warp_lu_solve(const T *W, int ldw, int n, T (&y)[bt::NQ]) {
-    using namespace bt;
     const int lane = threadIdx.x & 31;
-#pragma unroll 2
-    for (int j = 0; j < n; ++j) {
-        const int qj = j >> 5, lj = j & 31;
-        T src = y[0];
-#pragma unroll
-        for (int q = 1; q < NQ; ++q)
-            if (q == qj) src = y[q];
-        const T yj = __shfl_sync(0xffffffffu, src, lj);
-        const T *col = W + (i64)j * ldw;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const int i = lane + 32 * q;
-            if (i > j && i < n) y[q] = fma(-col[i], yj, y[q]);
-        }
-    }
-#pragma unroll 2
-    for (int j = n - 1; j >= 0; --j) {
-        const int qj = j >> 5, lj = j & 31;
-        T src = y[0];
-#pragma unroll
-        for (int q = 1; q < NQ; ++q)
-            if (q == qj) src = y[q];
-        const T *col = W + (i64)j * ldw;
-        const T xj = __shfl_sync(0xffffffffu, src, lj) / col[j];
-        if (lane == lj) {
-#pragma unroll
-            for (int q = 0; q < NQ; ++q)
-                if (q == qj) y[q] = xj;
-        }
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const int i = lane + 32 * q;
-            if (i < j) y[q] = fma(-col[i], xj, y[q]);
-        }
-    }
+    for (int j0 = 0; j0 < n; j0 += 32) forward_chunk(W + j0 * ldw, ldw, j0, min(j0 + 32, n), n, y, lane);
+    for (int j0 = (n - 1) & ~31; j0 >= 0; j0 -= 32) backward_chunk(W + j0 * ldw, ldw, j0, min(j0 + 32, n), y, lane);
 }
 
 // The whole CTA solves L U y = z for the right-hand sides held by its active
@@ -603,20 +697,7 @@ __device__ void block_lu_solve(const T *W, int ldw, int n, T *stage, int cap, bo
         const bool more = j1 < n;
         if (more) fetch(j1, min(j1 + cs, n));
         if (active) {
-            for (int j = j0; j < j1; ++j) {
-                const int qj = j >> 5, lj = j & 31;
-                T src = y[0];
-#pragma unroll
-                for (int q = 1; q < NQ; ++q)
-                    if (q == qj) src = y[q];
-                const T yj = __shfl_sync(0xffffffffu, src, lj);
-                const T *col = cur + (j - j0) * NMAX;
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    const int i = lane + 32 * q;
-                    if (i > j && i < n) y[q] = fma(-col[i], yj, y[q]);
-                }
-            }
+            forward_chunk(cur, NMAX, j0, j1, n, y, lane);
         }
         if (more) put(nxt, j1, min(j1 + cs, n));
         __syncthreads();
@@ -625,41 +706,24 @@ __device__ void block_lu_solve(const T *W, int ldw, int n, T *stage, int cap, bo
         nxt = t;
     }
     {
-        const int a0 = max(0, n - cs);
+        const int a0 = (n - 1) / cs * cs;  // chunks from multiples of cs: none straddles two row blocks
         fetch(a0, n);
         put(cur, a0, n);
         __syncthreads();
     }
-    for (int b = n; b > 0; b -= cs) {  // backward, upper
-        const int a = max(0, b - cs), na = max(0, a - cs);
+    for (int b = n; b > 0;) {  // backward, upper
+        const int a = (b - 1) / cs * cs, na = max(0, a - cs);
         const bool more = a > 0;
         if (more) fetch(na, a);
         if (active) {
-            for (int j = b - 1; j >= a; --j) {
-                const int qj = j >> 5, lj = j & 31;
-                T src = y[0];
-#pragma unroll
-                for (int q = 1; q < NQ; ++q)
-                    if (q == qj) src = y[q];
-                const T *col = cur + (j - a) * NMAX;
-                const T xj = __shfl_sync(0xffffffffu, src, lj) / col[j];
-                if (lane == lj) {
-#pragma unroll
-                    for (int q = 0; q < NQ; ++q)
-                        if (q == qj) y[q] = xj;
-                }
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    const int i = lane + 32 * q;
-                    if (i < j) y[q] = fma(-col[i], xj, y[q]);
-                }
-            }
+            backward_chunk(cur, NMAX, a, b, y, lane);
         }
         if (more) put(nxt, na, a);
         __syncthreads();
         T *t = cur;
         cur = nxt;
         nxt = t;
+        b = a;
     }
 }
 
