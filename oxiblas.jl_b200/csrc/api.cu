@@ -107,6 +107,7 @@ int oxi_destroy(oxi_handle_t h) {
     h->tc_ws2.release();
     h->xtag_ws.release();
     h->rowmap_ws.release();
+    h->ipiv_ws.release();
     h->tslu_ws.release();
     h->gcache.reset();
     h->bgraph.reset();

@@ -495,7 +495,12 @@ static int getrf_entry(oxi_handle_s *h, i64 m, i64 n, T *dA, i64 lda, int64_t *d
         int *d_moves = (int *)(sc + 128);
         OXI_CUDA(cudaMemsetAsync(d_info, 0, sizeof(int64_t), h->stream));
         launch_cm_to_rm<T, T>(dA, lda, W, ld, m, n, h->stream);
-        getrf_rowmajor_cached<T>(h, W, ld, m, n, d_ipiv, d_info, d_moves, d_nmoves);
+        // the handle's own pivots: a factorization of the same shape replays its
+        // graph whatever arrays the caller brings
+        const i64 q = std::min(m, n);
+        int64_t *piv = (int64_t *)h->ipiv_ws.get(sizeof(int64_t) * (size_t)q);
+        getrf_rowmajor_cached<T>(h, W, ld, m, n, piv, d_info, d_moves, d_nmoves);
+        OXI_CUDA(cudaMemcpyAsync(d_ipiv, piv, sizeof(int64_t) * (size_t)q, cudaMemcpyDeviceToDevice, h->stream));
         launch_rm_to_cm<T, T>(W, ld, dA, lda, m, n, h->stream);
         int64_t *hi = (int64_t *)h->host_ws.get(64);
         OXI_CUDA(cudaMemcpyAsync(hi, d_info, sizeof(int64_t), cudaMemcpyDeviceToHost, h->stream));

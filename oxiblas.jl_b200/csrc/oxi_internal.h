@@ -113,6 +113,7 @@ struct oxi_handle_s {
     oxi::DeviceBuffer solve_ws;  // solve workspace
     oxi::DeviceBuffer mixed_ws;  // mixed-precision workspace
     oxi::DeviceBuffer perm_ws;   // row permutation of the last solve
+    oxi::DeviceBuffer ipiv_ws;   // pivots of the running factorization
     oxi::PinnedBuffer host_ws;   // pinned host staging
     oxi::DeviceBuffer tc_ws;     // 16-bit GEMM operands
     oxi::DeviceBuffer tc_ws2;    // the same for a second, concurrent trailing update
