@@ -99,10 +99,18 @@ struct TriInvSmem {
     T Y[ST][YP];
 };
 
-// out (32 x 32, this thread's four elements of row `row`, columns c4..) =
-// A (32 x K, pitch ap) B (K x 32, pitch bp)
+// a / d from d's reciprocal, corrected by the remainder; the division where that
+// leaves the finite numbers
 template <typename T>
-__device__ __forceinline__ void inv_product(const T *A, int ap, const T *B, int bp, int K, T *out, int op) {
+__device__ __forceinline__ T quotient(T a, T d, T r) {
+    const T q = a * r;
+    const T l = mad(mad(-q, d, a), r, q);
+    return isfinite(l) ? l : a / d;
+}
+
+// out (32 x 32) = +-A (32 x K, pitch ap) B (K x 32, pitch bp), one call by the CTA
+template <typename T>
+__device__ __forceinline__ void inv_product(const T *A, int ap, const T *B, int bp, int K, T *out, int op, bool neg) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     if constexpr (sizeof(T) == 8) {
         const int m0 = (warp & 1) * 16, n0 = (warp >> 1) * 8, gid = lane >> 2, tig = lane & 3;
@@ -120,8 +128,10 @@ __device__ __forceinline__ void inv_product(const T *A, int ap, const T *B, int 
             }
         }
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-            out[(m0 + gid + 8 * (e >> 1)) * op + n0 + 2 * tig + (e & 1)] = c[0][e] + c[1][e];
+        for (int e = 0; e < 4; ++e) {
+            const double v = c[0][e] + c[1][e];
+            out[(m0 + gid + 8 * (e >> 1)) * op + n0 + 2 * tig + (e & 1)] = neg ? -v : v;
+        }
     } else {
         const int row = t >> 3, c4 = (t & 7) * 4;
         T z[4] = {T(0), T(0), T(0), T(0)};
@@ -133,7 +143,7 @@ __device__ __forceinline__ void inv_product(const T *A, int ap, const T *B, int 
             for (int u = 0; u < 4; ++u) z[u] = mad(yv, B[k * bp + c4 + u], z[u]);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) out[row * op + c4 + u] = z[u];
+        for (int u = 0; u < 4; ++u) out[row * op + c4 + u] = neg ? -z[u] : z[u];
     }
 }
 
@@ -172,26 +182,64 @@ __global__ void __launch_bounds__(INV_NT) k_tri_inv(const TriView<T> v0, const T
     if (warp <= s) {
         T(*D)[DP] = S.D[warp];
         const int d0 = warp * ST;
+        // the loads in flight together: into registers before the first one is stored
+        T xd[ST];
+        const int ds = d0 + ST <= nrow ? ST : nrow - d0;  // the block's rows (<= 0: none)
 #pragma unroll
         for (int e = 0; e < ST; ++e) {
             const int i = rowacc ? e : lane, j = rowacc ? lane : e;
-            T x = i == j ? T(1) : T(0);
-            if (d0 + i < nrow && (j < i || (j == i && !v.unit))) x = conj_if(base[(d0 + i) * v.rs + (d0 + j) * v.cs], v.conj);
-            D[i][j] = x;
+            xd[e] = (i < ds && j < ds) ? base[(d0 + i) * v.rs + (d0 + j) * v.cs] : T(0);
+        }
+#pragma unroll
+        for (int e = 0; e < ST; ++e) {
+            const int i = rowacc ? e : lane, j = rowacc ? lane : e;
+            D[i][j] = (i < ds && (j < i || (j == i && !v.unit))) ? conj_if(xd[e], v.conj) : i == j ? T(1) : T(0);
         }
         __syncwarp();
-        T x[ST];
+        // column `lane` of the inverse, eight rows at a time (rolled: unrolled over
+        // the 32 rows the code outgrows the instruction cache it runs through once):
+        // the rows by substitution in registers, their products off the rows below.
+        // The finished rows replace the block's, which no later step reads.
+        const T rd = (v.unit || sizeof(T) == 16) ? T(1) : T(1) / D[lane][lane];
+        T xr[ST / 8][8];
 #pragma unroll
-        for (int i = 0; i < ST; ++i) x[i] = (i == lane) ? T(1) : T(0);
+        for (int b = 0; b < ST / 8; ++b)
 #pragma unroll
-        for (int p = 0; p < ST; ++p) {
-            if (!v.unit) x[p] = x[p] / D[p][p];
+            for (int u = 0; u < 8; ++u) xr[b][u] = (8 * b + u == lane) ? T(1) : T(0);
+#pragma unroll 1
+        for (int b = 0; b < ST / 8; ++b) {
+            T x[8];
 #pragma unroll
-            for (int i = p + 1; i < ST; ++i) x[i] = mad(-D[i][p], x[p], x[i]);
+            for (int u = 0; u < 8; ++u) x[u] = xr[0][u];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const T *row = &D[8 * b + u][8 * b];
+#pragma unroll
+                for (int p = 0; p < u; ++p) x[u] = mad(-row[p], x[p], x[u]);
+                if (!v.unit) {
+                    if constexpr (sizeof(T) == 16) x[u] = x[u] / row[u];
+                    else x[u] = quotient(x[u], row[u], __shfl_sync(0xffffffffu, rd, 8 * b + u));
+                }
+            }
+#pragma unroll
+            for (int q = 1; q < ST / 8; ++q) {
+                if (b + q < ST / 8) {
+#pragma unroll
+                    for (int w = 0; w < 8; ++w) {
+                        const T *row = &D[8 * (b + q) + w][8 * b];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) xr[q][w] = mad(-row[u], x[u], xr[q][w]);
+                    }
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 8; ++u) D[8 * b + u][lane] = x[u];
+#pragma unroll
+            for (int q = 0; q < ST / 8 - 1; ++q)
+#pragma unroll
+                for (int u = 0; u < 8; ++u) xr[q][u] = xr[q + 1][u];
         }
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < ST; ++i) D[i][lane] = x[i];
     }
     __syncthreads();
     for (int e = t; e < ST * SP; e += INV_NT) {
@@ -208,20 +256,18 @@ __global__ void __launch_bounds__(INV_NT) k_tri_inv(const TriView<T> v0, const T
         }
         __syncthreads();
         if (b > 0) fetch(b - 1);
-        inv_product<T>(&S.Y[0][(b + 1) * ST], YP, &S.L[0][0], DP, K, &S.Z[0][0], DP);
+        inv_product<T>(&S.Y[0][(b + 1) * ST], YP, &S.L[0][0], DP, K, &S.Z[0][0], DP, true);
         __syncthreads();
-        inv_product<T>(&S.Z[0][0], DP, &S.D[b][0][0], DP, ST, &S.Y[0][b * ST], YP);
-        __syncthreads();
-        for (int e = t; e < ST * ST; e += INV_NT) {
-            T &y = S.Y[e / ST][b * ST + e % ST];
-            y = -y;
-        }
+        inv_product<T>(&S.Z[0][0], DP, &S.D[b][0][0], DP, ST, &S.Y[0][b * ST], YP, false);
         __syncthreads();
     }
     __syncthreads();
     T *Pg = P + (i64)g * SP * ST;
 #pragma unroll 4
-    for (int e = t; e < SP * ST; e += INV_NT) Pg[e] = S.Y[e % ST][e / ST];
+    for (int e = t; e < SP * ST; e += INV_NT) {  // a warp: eight rows of four columns
+        const int l = e & 31, q = e >> 5, r = (l & 7) + 8 * (q & 3), c = (l >> 3) + 4 * (q >> 2);
+        Pg[c * ST + r] = S.Y[r][c];
+    }
 }
 
 // ---------------------------------------------------------------------------
