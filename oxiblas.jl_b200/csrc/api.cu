@@ -119,6 +119,7 @@ int oxi_destroy(oxi_handle_t h) {
     if (h->la_in) cudaEventDestroy(h->la_in);
     if (h->la_out) cudaEventDestroy(h->la_out);
     if (h->la_fork) cudaEventDestroy(h->la_fork);
+    if (h->la_fork2) cudaEventDestroy(h->la_fork2);
     if (h->la_join) cudaEventDestroy(h->la_join);
     if (h->aux_fork) cudaEventDestroy(h->aux_fork);
     if (h->aux_join) cudaEventDestroy(h->aux_join);

@@ -38,6 +38,7 @@ void ensure_lookahead_streams(oxi_handle_s *h) {
     OXI_CUDA(cudaStreamCreateWithPriority(&h->la_stream, cudaStreamNonBlocking, lo));
     OXI_CUDA(cudaStreamCreateWithPriority(&h->la_main, cudaStreamNonBlocking, hi));
     OXI_CUDA(cudaEventCreateWithFlags(&h->la_fork, cudaEventDisableTiming));
+    OXI_CUDA(cudaEventCreateWithFlags(&h->la_fork2, cudaEventDisableTiming));
     OXI_CUDA(cudaEventCreateWithFlags(&h->la_join, cudaEventDisableTiming));
     OXI_CUDA(cudaEventCreateWithFlags(&h->la_in, cudaEventDisableTiming));
     OXI_CUDA(cudaEventCreateWithFlags(&h->la_out, cudaEventDisableTiming));
@@ -328,6 +329,9 @@ void getrf_rowmajor(oxi_handle_s *h, T *W, i64 ld, i64 m, i64 n, int64_t *d_ipiv
                 launch_rowmap_init(R.map, m - f, listcnt, sA);
                 panel_rec(R, f, l - f);
                 launch_rowmap_extract(R.map, m - f, list, listcnt, sA);
+                // the second stream's row moves and U12 need the panel only: they run
+                // beside this stream's work on the next panel's columns
+                if (split) OXI_CUDA(cudaEventRecord(h->la_fork, sA));
                 if (b_pending) {  // the previous trailing update reads L21 and writes the columns moved now
                     OXI_CUDA(cudaStreamWaitEvent(sA, h->la_join, 0));
                     b_pending = false;
@@ -351,7 +355,8 @@ void getrf_rowmajor(oxi_handle_s *h, T *W, i64 ld, i64 m, i64 n, int64_t *d_ipiv
             launch_rowmoves_big<T>(W, ld, f, list, listcnt, maxcnt, l, l2, sA);
             trsm_lower_unit<T>(h, L11, ld, L11 + (l - f), ld, l - f, l2 - l);
             update(f, l, l, l2);
-            OXI_CUDA(cudaEventRecord(h->la_fork, sA));
+            // (the 16-bit update reuses the operand that the one above converted)
+            if (sizeof(T) == 4) OXI_CUDA(cudaEventRecord(h->la_fork2, sA));
             OXI_CUDA(cudaStreamWaitEvent(h->la_stream, h->la_fork, 0));
             // ... everything else on the second stream: its own operand buffers, and
             // SMs left free for the next panel's cluster
@@ -370,6 +375,7 @@ void getrf_rowmajor(oxi_handle_s *h, T *W, i64 ld, i64 m, i64 n, int64_t *d_ipiv
             launch_rowmoves_big<T>(W, ld, f, list, listcnt, maxcnt, 0, f, h->stream);
             launch_rowmoves_big<T>(W, ld, f, list, listcnt, maxcnt, l2, R.ncols_moved, h->stream);
             trsm_lower_unit<T>(h, L11, ld, W + f * ld + l2, ld, l - f, n - l2);
+            if (sizeof(T) == 4) OXI_CUDA(cudaStreamWaitEvent(h->la_stream, h->la_fork2, 0));
             update(f, l, l2, n);
             h->stream = sA;
             h->tc_slot = 0;

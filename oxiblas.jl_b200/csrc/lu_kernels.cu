@@ -891,6 +891,10 @@ void launch_rowmoves_big(T *W, i64 ld, i64 r0, const int *list, const int *cnt, 
     // slab of 64 columns (FP32) / 32 (FP64): 16 or 8 threads per row, 16 or 32 rows at once
     int cpc = vec ? 16 * V : 64;
     while (cpc > V && (size_t)maxcnt * cpc * sizeof(T) > 160 * 1024) cpc /= 2;
+    // few columns (the next panel's, on the panels' critical path): slabs down to 64
+    // bytes, so that the moves spread over more SMs (n = 16384, 256 columns: 4 CTAs
+    // took 30 us)
+    while (vec && (c_hi - c_lo + cpc - 1) / cpc < 32 && cpc * (int)sizeof(T) > 64) cpc /= 2;
     const size_t smem = (size_t)maxcnt * cpc * sizeof(T);
     constexpr int kMaxSmem = 200 * 1024;  // the kernel's one limit (see set_max_dyn_smem)
     if (smem > (size_t)kMaxSmem) throw CudaError{cudaErrorInvalidValue, "panel too wide for the row moves"};

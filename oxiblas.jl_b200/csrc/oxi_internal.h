@@ -131,7 +131,7 @@ struct oxi_handle_s {
     cudaStream_t la_stream = nullptr;        // lookahead: the trailing update's stream
     cudaStream_t la_main = nullptr;          // lookahead: the panels' stream (highest priority)
     cudaEvent_t la_in = nullptr, la_out = nullptr;  // caller's stream -> la_main -> caller's stream
-    cudaEvent_t la_fork = nullptr, la_join = nullptr;
+    cudaEvent_t la_fork = nullptr, la_fork2 = nullptr, la_join = nullptr;
     oxi::DeviceBuffer xtag_ws;   // tickets and exchange words of the triangular solves
     oxi::DeviceBuffer trsv_ws;   // superblock inverses of getrs / potrs
     oxi::DeviceBuffer rowmap_ws; // per-panel row map and composite move list

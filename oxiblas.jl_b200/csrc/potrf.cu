@@ -432,6 +432,9 @@ void potrf_rowmajor(oxi_handle_s *h, T *U, i64 ld, i64 n, int64_t *d_info, T *wo
                 po_sym_update(h, A22, ld, Tt, t, X, ldx, right, right, s);
                 continue;
             }
+            // the rest of the update needs the block row only (FP32 converts its
+            // operands in the handle's buffers, one update after the other)
+            if (sizeof(T) == 8) OXI_CUDA(cudaEventRecord(h->la_fork, s));
             // the next block's rows, after the rest of the previous update
             if (b_pending) {
                 OXI_CUDA(cudaStreamWaitEvent(s, h->la_join, 0));
@@ -440,7 +443,7 @@ void potrf_rowmajor(oxi_handle_s *h, T *U, i64 ld, i64 n, int64_t *d_info, T *wo
             const i64 t2 = std::min<i64>(PO_NB, right);
             po_sym_update(h, A22, ld, Tt, t, X, ldx, t2, right, s);
             if (right > t2) {  // the rest on the low-priority stream
-                OXI_CUDA(cudaEventRecord(h->la_fork, s));
+                if (sizeof(T) == 4) OXI_CUDA(cudaEventRecord(h->la_fork, s));
                 OXI_CUDA(cudaStreamWaitEvent(h->la_stream, h->la_fork, 0));
                 h->stream = h->la_stream;
                 h->tc_slot = 1;
