@@ -101,23 +101,30 @@ namespace {
 
 
 struct Misc {
-    double red_v[2][bt::NW], red_x[2][bt::NW];
-    int red_i[2][bt::NW];
     double red_m[bt::NW][bt::MAXRHS];
     int piv[bt::NMAX];   // pivot row (0-based, within the matrix) of each column
-    int rowat[bt::NMAX]; // a panel's net permutation: position p holds row rowat[p]
-    int mvpos[2 * bt::NBMAX];
+    // during the factorization: a narrow last panel's net permutation, position p
+    // holds row perm[p]; after it: row i of L U is row perm[i] of A
+    int perm[bt::NMAX];
     int nmv;
-    int perm[bt::NMAX];  // net permutation: row i of L U is row perm[i] of A
     // reciprocals of the radix row and column scales: powers of two in
     // [2^-1023, 2^1022], so x * rrow[i] is exactly x / (row scale i)
     double rrow[bt::NMAX], rcol[bt::NMAX];
+    int item, info, bad;
+};
+
+// What a panel's factorization and interchanges pass through shared memory: in
+// the staged U12's place, which is written after them.
+struct PanelScratch {
+    double red_v[2][bt::NW], red_x[2][bt::NW];
+    int red_i[2][bt::NW];
     // register panel: every warp's candidate, by column parity -- {position, value}
     // and its row from the active column on
     double2 cand[2][bt::NW];
-    double crow[2][bt::NW][bt::NBMAX];
-    int item, info, bad;
+    __align__(16) double crow[2][bt::NW][bt::NBMAX];
+    int2 mv[2 * bt::NBMAX];  // the panel's net row moves: row .y goes to position .x
 };
+static_assert(sizeof(PanelScratch) <= 8 * bt::UP * sizeof(float), "fits the narrowest staged U12");
 
 // Rows [0, m) of a column from global memory into dst (m <= NMAX, one warp):
 // every lane issues its loads before its stores, so the round trips overlap.
@@ -141,7 +148,7 @@ __device__ __forceinline__ void load_col(T *dst, const U *src, int m, int lane) 
 // value, and col[j] -- every value read before the barrier, so no thread can
 // see a row the interchange that follows has already moved.
 template <typename T>
-__device__ int block_argmax(const T *col, int j, int m, Misc &S, int par, double &best, double &val,
+__device__ int block_argmax(const T *col, int j, int m, PanelScratch &S, int par, double &best, double &val,
                             double &vj) {
     using namespace bt;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -194,7 +201,7 @@ __device__ int block_argmax(const T *col, int j, int m, Misc &S, int par, double
 // Unblocked LU of the panel P (m x jb, column-major, ldp) holding columns
 // k..k+jb of rows k..n; records S.piv[k + j] and the first zero pivot.
 template <typename T>
-__device__ void panel_lu(T *P, int ldp, int m, int jb, int k, Misc &S) {
+__device__ void panel_lu(T *P, int ldp, int m, int jb, int k, Misc &S, PanelScratch &Q) {
     using namespace bt;
     for (int j = 0; j < jb; ++j) {
         T *colj = P + (i64)j * ldp;
@@ -202,7 +209,7 @@ __device__ void panel_lu(T *P, int ldp, int m, int jb, int k, Misc &S) {
         // strict '>' -- the first maximum; a NaN at row j keeps row j, a NaN
         // below never wins
         double bv, bx, vj;
-        const int pb = block_argmax(colj, j, m, S, j & 1, bv, bx, vj);
+        const int pb = block_argmax(colj, j, m, Q, j & 1, bv, bx, vj);
         const bool below = pb != INT_MAX && bv > fabs(vj);
         const int p = below ? pb : j;
         const T d = (T)(below ? bx : vj);
@@ -331,7 +338,7 @@ __device__ __forceinline__ void update_tile(const float *Ap, int lda, const floa
 // one barrier, the arg-max over the warps, and the rank-1 update on registers.
 // Same operations in the same order as panel_lu.
 template <typename T, int JB>
-__device__ void panel_lu_reg(T *P, int ldp, int m, int k, Misc &S) {
+__device__ void panel_lu_reg(T *P, int ldp, int m, int k, Misc &S, PanelScratch &Q) {
     using namespace bt;
     const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
     int pos = i < m ? i : -1;
@@ -343,10 +350,12 @@ __device__ void panel_lu_reg(T *P, int ldp, int m, int k, Misc &S) {
         const int par = j & 1;
         const uint32_t wm = warp_winner<T>(step_key(row[j], pos, j), pos >= j ? pos : INT_MAX);
         if (wm == 0 ? lane == 0 : ((wm >> lane) & 1)) {
-            S.cand[par][warp] = make_double2(__hiloint2double(0, wm ? pos : INT_MAX), (double)row[j]);
-            T *cr = (T *)S.crow[par][warp];
+            Q.cand[par][warp] = make_double2(__hiloint2double(0, wm ? pos : INT_MAX), (double)row[j]);
+            T *cr = (T *)Q.crow[par][warp];
+            constexpr int VEC = 16 / (int)sizeof(T);
 #pragma unroll
-            for (int c = j; c < JB; ++c) cr[c] = row[c];
+            for (int c = 0; c < JB; c += VEC)
+                if (c + VEC > j) store_row<T, VEC>(cr + c, row + c);
         }
         __syncthreads();
         int wq;
@@ -354,17 +363,17 @@ __device__ void panel_lu_reg(T *P, int ldp, int m, int k, Misc &S) {
             int cp = INT_MAX;
             uint64_t ck = 0;
             if (lane < NW) {
-                const double2 h = S.cand[par][lane];
+                const double2 h = Q.cand[par][lane];
                 cp = __double2loint(h.x);
                 ck = step_key((T)h.y, cp, j);
             }
             const uint32_t w = warp_winner<T>(ck, cp);
             wq = w ? __ffs(w) - 1 : 0;
         }
-        const double2 h = S.cand[par][wq];
+        const double2 h = Q.cand[par][wq];
         const int p = __double2loint(h.x);
         const T d = (T)h.y;
-        const T *pa = (const T *)S.crow[par][wq];
+        const T *pa = (const T *)Q.crow[par][wq];
         if (i == 0) {
             S.piv[k + j] = k + p;
             if (d == T(0) && S.info == 0) S.info = k + j + 1;  // no interchange, no elimination: p is j
@@ -374,14 +383,24 @@ __device__ void panel_lu_reg(T *P, int ldp, int m, int k, Misc &S) {
         if (d != T(0) && q >= j && q != p) {
             const T l = row[j] / d;
             row[j] = l;
+            constexpr int VEC = 16 / (int)sizeof(T);
 #pragma unroll
-            for (int c = j + 1; c < JB; ++c) row[c] = fma(-l, pa[c], row[c]);
+            for (int c = 0; c < JB; c += VEC) {
+                if (c + VEC > j + 1) {
+                    T u[VEC];
+                    load_row<T, VEC>(u, pa + c);
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e)
+                        if (c + e > j) row[c + e] = fma(-l, u[e], row[c + e]);
+                }
+            }
         }
     }
     // every thread has read its row long before (the first barrier)
     if (pos >= 0) {
 #pragma unroll
-        for (int c = 0; c < JB; ++c) P[pos + (i64)c * ldp] = row[c];
+        for (int c = 0; c < JB; ++c) P[pos + c * ldp] = row[c];
+        if (pos != i) Q.mv[atomicAdd(&S.nmv, 1)] = make_int2(k + pos, k + i);
     }
     __syncthreads();  // the panel, S.piv and S.info visible to all
 }
@@ -445,8 +464,10 @@ __device__ __forceinline__ void update_tile_dmma(const double *Ap, int lda, cons
 template <typename T>
 __device__ void lu_blocked(T *W, int ldw, int n, int nb, bool in_smem, T *sP, T *sU, Misc &S) {
     using namespace bt;
+    PanelScratch &Q = *reinterpret_cast<PanelScratch *>(sU);
     for (int k = 0; k < n; k += nb) {
         const int jb = min(nb, n - k), m = n - k;
+        if (threadIdx.x == 0) S.nmv = 0;
         T *P;
         int ldp;
         if (in_smem) {
@@ -458,90 +479,76 @@ __device__ void lu_blocked(T *W, int ldw, int n, int nb, bool in_smem, T *sP, T 
             // a warp per column, its lanes down the rows (coalesced, no index division)
             for (int c = (int)(threadIdx.x >> 5); c < jb; c += NW)
                 load_col(sP + c * ldp, W + k + (i64)(k + c) * ldw, m, (int)(threadIdx.x & 31));
-            __syncthreads();
         }
-        if (jb == 16) panel_lu_reg<T, 16>(P, ldp, m, k, S);
-        else if (jb == 8) panel_lu_reg<T, 8>(P, ldp, m, k, S);
-        else if (jb == 32) panel_lu_reg<T, 32>(P, ldp, m, k, S);
-        else panel_lu(P, ldp, m, jb, k, S);
+        __syncthreads();
+        if (jb == 16) panel_lu_reg<T, 16>(P, ldp, m, k, S, Q);
+        else if (jb == 8) panel_lu_reg<T, 8>(P, ldp, m, k, S, Q);
+        else if (jb == 32) panel_lu_reg<T, 32>(P, ldp, m, k, S, Q);
+        else panel_lu(P, ldp, m, jb, k, S, Q);
         if (!in_smem) {
             for (int c = (int)(threadIdx.x >> 5); c < jb; c += NW)
                 for (int r = (int)(threadIdx.x & 31); r < m; r += 32) W[(k + r) + (i64)(k + c) * ldw] = sP[r + c * ldp];
         }
-        // interchanges on the other columns, then U12 = L11^-1 A12
         const int c2 = k + jb;
-        if (!in_smem) {
-            // global working matrix: the panel's net permutation once, every moved
-            // row of the other columns staged in shared memory (sU), then written
-            // back -- one round trip instead of jb dependent swaps per column
-            for (int p = k + threadIdx.x; p < n; p += NT) S.rowat[p] = p;
-            if (threadIdx.x == 0) S.nmv = 0;
+        if (jb != 8 && jb != 16 && jb != 32) {
+            // a narrower last panel: its interchanges folded into the net row moves
+            for (int p = k + threadIdx.x; p < n; p += NT) S.perm[p] = p;
             __syncthreads();
             if (threadIdx.x == 0)
                 for (int j = 0; j < jb; ++j) {
                     const int a = k + j, b = S.piv[k + j];
-                    const int t = S.rowat[a];
-                    S.rowat[a] = S.rowat[b];
-                    S.rowat[b] = t;
+                    const int t = S.perm[a];
+                    S.perm[a] = S.perm[b];
+                    S.perm[b] = t;
                 }
             __syncthreads();
             for (int p = k + threadIdx.x; p < n; p += NT)
-                if (S.rowat[p] != p) S.mvpos[atomicAdd(&S.nmv, 1)] = p;
+                if (S.perm[p] != p) Q.mv[atomicAdd(&S.nmv, 1)] = make_int2(p, S.perm[p]);
             __syncthreads();
-            const int nmv = S.nmv;  // <= 2 jb
+        }
+        // interchanges on the other columns: a warp per column, a move per lane (two
+        // with 32-column panels), so reading all of a column's sources before
+        // writing needs no staging; four columns in flight
+        {
+            const int nmv = S.nmv, lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
             if (nmv > 0) {
-                const int ccap = (nb * NMAX) / nmv;  // columns per pass (>= 128)
-                for (int cb = 0; cb < n; cb += ccap) {
-                    const int cn = min(ccap, n - cb);
-                    // a warp per moved row, its lanes across the columns
-                    // cn <= n <= 32 NQ: a lane's columns of a moved row in one batch of loads
-                    for (int mv = (int)(threadIdx.x >> 5); mv < nmv; mv += NW) {
-                        const int src = S.rowat[S.mvpos[mv]];
-                        T v[NQ];
+                const int2 m0 = lane < nmv ? Q.mv[lane] : make_int2(0, 0);
+                const int2 m1 = lane + 32 < nmv ? Q.mv[lane + 32] : make_int2(0, 0);
+                const int others = n - jb;
+                for (int q0 = warp; q0 < others; q0 += 4 * NW) {
+                    T v[4][2];
 #pragma unroll
-                        for (int q = 0; q < NQ; ++q) {
-                            const int cc = (int)(threadIdx.x & 31) + 32 * q, c = cb + cc;
-                            v[q] = (cc < cn && !(c >= k && c < c2)) ? W[src + (i64)c * ldw] : T(0);
-                        }
-#pragma unroll
-                        for (int q = 0; q < NQ; ++q) {
-                            const int cc = (int)(threadIdx.x & 31) + 32 * q, c = cb + cc;
-                            if (cc < cn && !(c >= k && c < c2)) sU[mv * ccap + cc] = v[q];
+                    for (int u = 0; u < 4; ++u) {
+                        const int q = q0 + u * NW;
+                        const T *wc = W + (i64)(q < k ? q : q + jb) * ldw;
+                        v[u][0] = v[u][1] = T(0);
+                        if (q < others) {
+                            if (lane < nmv) v[u][0] = wc[m0.y];
+                            if (lane + 32 < nmv) v[u][1] = wc[m1.y];
                         }
                     }
-                    __syncthreads();
-                    for (int mv = (int)(threadIdx.x >> 5); mv < nmv; mv += NW) {
-                        const int dst = S.mvpos[mv];
-                        for (int cc = (int)(threadIdx.x & 31); cc < cn; cc += 32) {
-                            const int c = cb + cc;
-                            if (c >= k && c < c2) continue;
-                            W[dst + (i64)c * ldw] = sU[mv * ccap + cc];
+                    __syncwarp();
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int q = q0 + u * NW;
+                        T *wc = W + (i64)(q < k ? q : q + jb) * ldw;
+                        if (q < others) {
+                            if (lane < nmv) wc[m0.x] = v[u][0];
+                            if (lane + 32 < nmv) wc[m1.x] = v[u][1];
                         }
                     }
-                    __syncthreads();
                 }
             }
         }
-        for (int c = threadIdx.x; c < n; c += NT) {
-            if (c >= k && c < c2) continue;
+        __syncthreads();
+        // U12 = L11^-1 A12
+        for (int c = c2 + threadIdx.x; c < n; c += NT) {
+            // only full panels have columns to the right: the width is a constant
             T *wc = W + (i64)c * ldw;
-            if (in_smem) {
-                for (int j = 0; j < jb; ++j) {
-                    const int p = S.piv[k + j];
-                    if (p != k + j) {
-                        const T t = wc[k + j];
-                        wc[k + j] = wc[p];
-                        wc[p] = t;
-                    }
-                }
-            }
-            if (c >= c2) {  // full panels at a compile-time width: no predicated steps
-                T *su = in_smem ? nullptr : sU + (c - c2);
-                if (jb == 16) u12_column<T, 16>(wc, k, 16, P, ldp, su);
-                else if (jb == 8) u12_column<T, 8>(wc, k, 8, P, ldp, su);
-                else if (jb == 32) u12_column<T, 32>(wc, k, 32, P, ldp, su);
-                else u12_column<T, NBMAX>(wc, k, jb, P, ldp, su);
-            }
+            T *su = in_smem ? nullptr : sU + (c - c2);
+            if (jb == 16) u12_column<T, 16>(wc, k, 16, P, ldp, su);
+            else if (jb == 8) u12_column<T, 8>(wc, k, 8, P, ldp, su);
+            else u12_column<T, 32>(wc, k, 32, P, ldp, su);
         }
         __syncthreads();
         // A22 -= L21 U12: FP64 by warp tiles of 32 x 16 on the tensor cores, FP32 by

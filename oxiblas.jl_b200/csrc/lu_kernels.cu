@@ -111,31 +111,6 @@ template void launch_rm_to_cm<float, double>(const float *, i64, double *, i64, 
 // per-warp shared memory, 128 contiguous bytes at a time: one row per lane, 16
 // bytes at a time, costs 32 cache lines an instruction.
 // ---------------------------------------------------------------------------
-// N elements between registers and 16-byte-aligned shared memory.
-template <typename T, int N>
-__device__ __forceinline__ void store_row(T *dst, const T *v) {
-    constexpr int VEC = 16 / sizeof(T);
-#pragma unroll
-    for (int c = 0; c < N; c += VEC) {
-        int4 x;
-        T *xx = (T *)&x;
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) xx[e] = v[c + e];
-        *(int4 *)(dst + c) = x;
-    }
-}
-template <typename T, int N>
-__device__ __forceinline__ void load_row(T *v, const T *src) {
-    constexpr int VEC = 16 / sizeof(T);
-#pragma unroll
-    for (int c = 0; c < N; c += VEC) {
-        const int4 x = *(const int4 *)(src + c);
-        const T *xx = (const T *)&x;
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) v[c + e] = xx[e];
-    }
-}
-
 constexpr int LEAF_NT = 512;
 constexpr int LEAF_MAX_CS = 16;
 
