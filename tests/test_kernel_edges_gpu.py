@@ -38,6 +38,16 @@ def test_leaf_heights_bit_identical(pkg, oracle, m):
         assert np.array_equal(_np(F.factors), Fo)
 
 
+def test_repeated_factorization_same_bits(pkg):
+    """Both streams of the lookahead and all pipelines under load: every repetition
+    gives the same factors."""
+    g = torch.Generator(device="cuda").manual_seed(2048)
+    A = torch.randn(2048, 2048, dtype=torch.float64, device="cuda", generator=g)
+    F0 = pkg.lu(A).factors.clone()
+    for _ in range(400):
+        assert torch.equal(pkg.lu(A).factors, F0)
+
+
 def test_leaf_zero_nan_and_extreme_pivots(pkg, oracle):
     rng = np.random.default_rng(7)
     A = rng.standard_normal((300, 64))
