@@ -211,7 +211,12 @@ static void panel_rec(LuRun<T> &R, i64 c0, i64 nc) {
             return;
         }
     }
-    const int leafw = ts ? 32 : leaf_width_for<T>(mrows);
+    int leafw = ts ? 32 : leaf_width_for<T>(mrows);
+    if constexpr (sizeof(T) == 8) {
+        // two leaves of 32 columns and the step between them in one launch (composed
+        // panels: the separate row moves take 64 rows at most)
+        if (nc == 64 && R.map && h->opt.gemm == 0 && mrows >= 64 && mrows <= LEAF_DUAL_ROWS) leafw = 64;
+    }
     if (leafw == 0) throw CudaError{cudaErrorInvalidValue, "panel taller than the leaf capacity"};
     if constexpr (sizeof(T) == 8) {
         if (nc > leafw && nc <= 32 && h->opt.gemm == 0) {

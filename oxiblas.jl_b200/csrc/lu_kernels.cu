@@ -126,7 +126,19 @@ __device__ __forceinline__ float multiplier(float a, float d, float y) {
     return fmaf(fmaf(-q, d, a), y, q);
 }
 
-template <typename T, int W, int R, int NT>
+// DUAL (FP64, 64 columns): the recursion's step from 32 to 64 columns inside the
+// launch, in the reference's order (src/lapack/factorizations.jl:140-150): the
+// first 32 columns as a leaf of their own, then the 32 pivot rows go to every
+// CTA, each solves U12 by the recursive TRSM's steps (8-row leaves), every row
+// below takes C - s with s one fma chain over the 32 columns from zero, and the
+// last 32 columns are the second leaf.  It replaces two leaves, a TRSM and a GEMM.
+// Bound: latency, as the leaf.
+// One B200, launches timed with the profile's events: 256 rows 4 x (31 + 31 + 8
+// + 10) us -> 4 x 64 us; the whole FP64 solve of n = 256 591 -> 575 us, n = 3001
+// 6.29 -> 6.00 ms, the n = 2048 forward and pullback 4.59 -> 4.35 ms.  Sending
+// the pivot rows by 16-byte st.async instead of bulk copies, and the step
+// unrolled over its blocks, cost 6 us a leaf more across CTAs.
+template <typename T, int W, int R, int NT, bool DUAL>
 __global__ void __launch_bounds__(NT, 1)
 k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restrict__ ipiv,
           int64_t *__restrict__ info, int *__restrict__ moves, int *__restrict__ nmoves,
@@ -136,7 +148,7 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
     const int cr = (int)cl.block_rank();
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     constexpr int NW = NT / 32;
-    constexpr int GW = W < 8 ? W : 8, NGR = W / GW;
+    constexpr int GW = W < 8 ? W : 8, NGR = W / GW, HW = DUAL ? W / 2 : W, NGRH = HW / GW;
     constexpr int VEC = 16 / sizeof(T);               // elements per 16-byte vector
     constexpr int CW = (VEC + GW + VEC - 1) / VEC * VEC;  // a candidate: position, live group values
     constexpr bool STAGED = (W * sizeof(T)) % 128 == 0;   // rows of whole 128-byte segments
@@ -151,11 +163,12 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
     extern __shared__ __align__(16) unsigned char leaf_smem[];  // 32 rows x 144 bytes per warp (STAGED)
     __shared__ __align__(16) T s_cand[2][NW][CW];              // this CTA's warps, by column parity
     __shared__ __align__(16) T s_slot[2][LEAF_MAX_CS][CW];     // every CTA's winner (clusters), by column parity
-    __shared__ __align__(16) T s_right[GW][W];  // the group's pivot rows: group values, columns to the right
-    __shared__ __align__(16) T s_stage[GW][W];
-    __shared__ __align__(16) T s_u[GW][W];             // columns to the right after the unit triangle
+    __shared__ __align__(16) T s_right[GW][HW];  // the group's pivot rows: group values, columns to the right
+    __shared__ __align__(16) T s_stage[GW][HW];
+    __shared__ __align__(16) T s_u[GW][HW];            // columns to the right after the unit triangle
     __shared__ __align__(8) uint64_t s_xbar[2];        // exchange barriers, by column parity
     __shared__ __align__(8) uint64_t s_rbar;           // pivot rows of a group
+    __shared__ __align__(8) uint64_t s_mbar;           // DUAL: the first half's pivot rows
     __shared__ int s_piv[W];   // pivots and info stay on chip until the end
     __shared__ int s_info;
     __shared__ int s_skip;     // the call was aborted before this launch
@@ -168,6 +181,7 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
         mbar_init(&s_xbar[0], 1);
         mbar_init(&s_xbar[1], 1);
         mbar_init(&s_rbar, 1);
+        mbar_init(&s_mbar, 1);
         fence_barrier_init();
     }
     constexpr int PERMAX = CW / VEC;   // 16-byte chunks of a candidate
@@ -222,6 +236,7 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
             }
         }
     }
+    if (DUAL) fence_proxy_async();  // the transfer area takes bulk copies later
     // every CTA's barriers exist before any CTA pushes into them, and
     // every row is read before any CTA stores one at its final position
     if (CS > 1) cl.sync();
@@ -253,6 +268,7 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
     // so the active group always sits in slots 0..GW-1, the unfinished columns
     // behind it and the finished ones last; after all groups the row is back in
     // its order.
+    uint32_t rphase = 0;  // exchanges of pivot rows so far
 #pragma unroll 1
     for (int s = 0; s < NGR; ++s) {
         const int j0 = s * GW;
@@ -381,7 +397,7 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
         }
         if constexpr (NGR > 1) {
             const int np = min(GW, q - j0);            // pivots of this group
-            const int nblk = NGR - 1 - s;              // unfinished groups to the right
+            const int nblk = NGRH - 1 - s % NGRH;      // unfinished groups to the right (of this half)
             if (np > 0 && nblk > 0 && j0 + np < wact) {
                 const int rem = nblk * GW, nch = (GW + rem) / VEC;
                 // (f) the pivot rows' multipliers and remaining columns to every CTA
@@ -393,7 +409,7 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
                     if (own) {
                         T *dst = (CS > 1) ? s_stage[kk] : s_right[kk];
 #pragma unroll
-                        for (int b = 0; b < NGR; ++b)
+                        for (int b = 0; b < NGRH; ++b)
                             if (b <= nblk) store_row<T, GW>(dst + b * GW, &r[k][b * GW]);
                     }
                     if (CS > 1) {
@@ -412,7 +428,8 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
                     }
                 }
                 if (CS > 1) {
-                    if (warp == 0 && !dead && !mbar_wait(&s_rbar, (uint32_t)(s & 1), pn.abort, 1)) dead = true;
+                    if (warp == 0 && !dead && !mbar_wait(&s_rbar, rphase & 1u, pn.abort, 1)) dead = true;
+                    ++rphase;
                 } else {
                     __syncthreads();
                 }
@@ -455,7 +472,7 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
                 }
                 const bool warp_any = __any_sync(0xffffffffu, any);
 #pragma unroll
-                for (int b = 0; b < NGR - 1; ++b) {
+                for (int b = 0; b < NGRH - 1; ++b) {
                     if (b < nblk) {
                         if (warp_any) {
                             T nv[R][GW];
@@ -509,6 +526,93 @@ k_leaf_lu(T *__restrict__ P, i64 ld, int m, int wact, i64 gofs, int64_t *__restr
                 for (int c = 0; c < W - GW; ++c) r[k][c] = r[k][c + GW];
 #pragma unroll
                 for (int c = 0; c < GW; ++c) r[k][W - GW + c] = f[c];
+            }
+        }
+        if constexpr (DUAL) {
+            if (s == NGRH - 1) {
+                // slots 0..HW-1 hold the second half's columns, slots HW.. the first's.
+                // The rows' transfer area is free until the end: X (U12, HW x HW), the
+                // pivot rows' multipliers, and the rows on their way out.
+                constexpr int LP = HW + 2;
+                static_assert(!DUAL || (R == 1 && (2 * HW + LP + HW) * HW * (int)sizeof(T) <= NW * 32 * 144), "mid-step area");
+                T *X = (T *)leaf_smem;                 // [HW][HW]
+                T *Ls = X + HW * HW;                   // [HW][LP]
+                T *st = Ls + HW * LP;                  // [HW][W]
+                __syncthreads();
+                if (CS > 1 && t == 0 && !dead) mbar_arrive_expect_tx(&s_mbar, (uint32_t)(HW * W * sizeof(T)));
+                const int kk = pos[0];
+                const bool own = kk >= 0 && kk < HW;
+                if (own) {
+                    store_row<T, HW>(CS > 1 ? st + kk * W : Ls + kk * LP, &r[0][HW]);
+                    store_row<T, HW>(CS > 1 ? st + kk * W + HW : X + kk * HW, &r[0][0]);
+                }
+                if (CS > 1) {
+                    // a row's two halves to every CTA, one bulk copy each
+                    uint32_t om = __ballot_sync(0xffffffffu, own);
+                    if (own) fence_proxy_async();
+                    __syncwarp();
+                    while (om) {
+                        const int src = __ffs(om) - 1;
+                        om &= om - 1;
+                        const int ks = __shfl_sync(0xffffffffu, kk, src);
+                        const bool lo = lane < 16;
+                        if (half < CS && !dead)
+                            bulk_to_cluster(smem_u32(lo ? Ls + ks * LP : X + ks * HW) + to_cta,
+                                            smem_u32(st + ks * W + (lo ? 0 : HW)), HW * sizeof(T),
+                                            smem_u32(&s_mbar) + to_cta);
+                    }
+                    if (!dead && !mbar_wait(&s_mbar, 0u, pn.abort, 1)) dead = true;
+                }
+                __syncthreads();
+                // U12 in the order of the recursive solve: halves down to 8-row leaves
+#pragma unroll 1
+                for (int a = 0; a < HW; a += 8) {
+                    if (t < HW) {
+                        T x[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) x[u] = X[(a + u) * HW + t];
+#pragma unroll
+                        for (int u = 1; u < 8; ++u)
+#pragma unroll
+                            for (int p = 0; p < u; ++p) x[u] = fma(-Ls[(a + u) * LP + a + p], x[p], x[u]);
+#pragma unroll
+                        for (int u = 1; u < 8; ++u) X[(a + u) * HW + t] = x[u];
+                    }
+                    __syncthreads();
+                    // rows [a + 8, hi) -= L[rows, lo:a+8] X[lo:a+8]
+                    const int lo = a == 8 ? 0 : a, hi = a == 8 ? HW : a == 24 ? 0 : a + 16;
+                    for (int i = a + 8 + t / HW; i < hi; i += NT / HW) {
+                        T acc = T(0);
+#pragma unroll 8
+                        for (int p = lo; p < a + 8; ++p) acc = fma(Ls[i * LP + p], X[p * HW + t % HW], acc);
+                        X[i * HW + t % HW] -= acc;
+                    }
+                    __syncthreads();
+                }
+                // the rows below: C - s; the pivot rows' own columns are U12's rows
+                if (own) {
+                    load_row<T, HW>(&r[0][0], X + kk * HW);
+                } else {
+#pragma unroll 1
+                    for (int b = 0; b < NGRH; ++b) {  // rotating, as the groups do
+                        T acc[GW];
+#pragma unroll
+                        for (int c = 0; c < GW; ++c) acc[c] = T(0);
+#pragma unroll
+                        for (int p = 0; p < HW; ++p) {
+                            T u[GW];
+                            load_row<T, GW>(u, X + p * HW + b * GW);
+#pragma unroll
+                            for (int c = 0; c < GW; ++c) acc[c] = fma(r[0][HW + p], u[c], acc[c]);
+                        }
+#pragma unroll
+                        for (int c = 0; c < GW; ++c) acc[c] = r[0][c] - acc[c];
+#pragma unroll
+                        for (int c = 0; c < HW - GW; ++c) r[0][c] = r[0][c + GW];
+#pragma unroll
+                        for (int c = 0; c < GW; ++c) r[0][HW - GW + c] = acc[c];
+                    }
+                }
             }
         }
     }
@@ -667,13 +771,13 @@ template <> int leaf_width_for<float>(i64 m) {
     return 0;
 }
 
-template <typename T, int W, int R, int NT = LEAF_NT>
+template <typename T, int W, int R, int NT = LEAF_NT, bool DUAL = false>
 static void launch_leaf_wr(T *P, i64 ld, i64 m, int w, i64 gofs, int64_t *ipiv, int64_t *info,
                            int *moves, int *nmoves, cudaStream_t s, LeafPanel pn) {
     const i64 per_cta = (i64)NT * R;
     int need = (int)((m + per_cta - 1) / per_cta);
     const int cs = need;
-    auto kern = k_leaf_lu<T, W, R, NT>;
+    auto kern = k_leaf_lu<T, W, R, NT, DUAL>;
     if (cs > 8) OXI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cs);
@@ -697,11 +801,20 @@ static void launch_leaf_wr(T *P, i64 ld, i64 m, int w, i64 gofs, int64_t *ipiv, 
     count_launch();
 }
 
+// Threads and rows a thread by height.  256 threads of one row while 16 CTAs hold
+// the rows (4096): fewer warps to reduce over and twice the registers a thread;
+// above, 512 threads (FP32 one row to 8192, then two).  FP64, 32 columns, kernel
+// alone, 256 against 512 threads: 1024 rows 44 against 46 us, 4096 rows 47
+// against 47 (16 CTAs against 8).  FP32: 4096 rows 41 us with 256 threads, 8192
+// rows 44 with 512 (54 with two rows in 256).  The cluster has as many CTAs as the
+// rows need, not the next power of two: the exchange takes 413 cycles among 2 CTAs
+// and 746 among 16.
 template <typename T>
 void launch_leaf(T *P, i64 ld, i64 m, int w, i64 gofs, int64_t *ipiv, int64_t *info, int *moves,
                  int *nmoves, int leafw, cudaStream_t s, LeafPanel pn) {
     if constexpr (sizeof(T) == 8) {
-        if (leafw == 32 && m <= LEAF_MAX_CS * 256) launch_leaf_wr<T, 32, 1, 256>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
+        if (leafw == 64) launch_leaf_wr<T, 64, 1, 256, true>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
+        else if (leafw == 32 && m <= LEAF_MAX_CS * 256) launch_leaf_wr<T, 32, 1, 256>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
         else if (leafw == 32) launch_leaf_wr<T, 32, 1>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
         else if (leafw == 16) launch_leaf_wr<T, 16, 2>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);
         else if (leafw == 8) launch_leaf_wr<T, 8, 4>(P, ld, m, w, gofs, ipiv, info, moves, nmoves, s, pn);

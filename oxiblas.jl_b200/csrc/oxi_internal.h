@@ -242,6 +242,9 @@ void launch_rm_to_cm(const TS *W, i64 ldw, TD *A, i64 lda, i64 m, i64 n, cudaStr
 // map = null switch it off.
 // Other panel columns (panel width minus the leaf's) that the in-leaf row moves
 // reach; wider panels apply each leaf's interchanges with separate row moves.
+// Rows up to which an FP64 leaf may have 64 columns (two halves of 32): 16 CTAs of 256
+// threads, whose 255 registers hold a row; 512 threads have 128.
+constexpr int LEAF_DUAL_ROWS = 16 * 256;
 constexpr int LEAF_MAX_OTHER = 256;
 
 // gemm_ctas = -k asks the persistent tensor-core GEMM for at most k clusters of

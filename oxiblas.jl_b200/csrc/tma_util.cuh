@@ -117,6 +117,14 @@ __device__ __forceinline__ void st_async_v4(uint32_t raddr, uint4 v, uint32_t rb
         : "memory");
 }
 
+// Bulk copy from this CTA's shared memory to another CTA's of the cluster,
+// completing on that CTA's mbarrier; addresses and size multiples of 16 bytes.
+__device__ __forceinline__ void bulk_to_cluster(uint32_t rdst, uint32_t src, uint32_t bytes, uint32_t rbar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(rdst),
+                 "r"(src), "r"(bytes), "r"(rbar)
+                 : "memory");
+}
+
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *tm, uint64_t *bar, int x,
                                             int y) {
     asm volatile(

@@ -38,6 +38,24 @@ def test_leaf_heights_bit_identical(pkg, oracle, m):
         assert np.array_equal(_np(F.factors), Fo)
 
 
+@pytest.mark.parametrize("m", [129, 191, 192, 193, 257, 513, 1111, 4096, 4097, 4161])
+def test_wide_leaf_bit_identical(pkg, oracle, m):
+    """A panel of 128 columns takes two FP64 leaves of 64 columns (the recursion's
+    step from 32 to 64 inside the launch) where 64 <= rows <= 4096; the 32 columns
+    behind the panel take the narrow one."""
+    rng = np.random.default_rng(m)
+    Z = rng.standard_normal((m, 160))
+    Z[:, 9] = 0.0                        # zero pivots in both halves of a leaf
+    Z[:, 45] = 0.0
+    Z[m // 2:, 70] = np.nan
+    for A in (rng.standard_normal((m, 160)), rng.integers(-2, 3, (m, 160)).astype(float), Z):
+        F = pkg.lu(A, check=False)
+        Fo, ipo, info = oracle.getrf(A, check=False)
+        assert F.info == info
+        assert np.array_equal(_np(F.ipiv), ipo)
+        assert np.array_equal(_np(F.factors), Fo, equal_nan=True)
+
+
 def test_repeated_factorization_same_bits(pkg):
     """Both streams of the lookahead and all pipelines under load: every repetition
     gives the same factors."""
