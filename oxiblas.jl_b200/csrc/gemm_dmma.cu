@@ -2,8 +2,8 @@
 //
 // sm_100a has no FP64 kind for tcgen05.mma; the FP64 tensor path is DMMA
 // (mma.sync.aligned.m16n8k4 .f64), which this kernel feeds from TMA.
-// CTA tile 128 x 64, k slab 16, 4-stage mbarrier pipeline, 8 warps in a 4 x 2 grid,
-// 32 x 32 per warp (2 x 4 MMAs per k4).  Thread 0 issues the TMA loads: a slot is
+// CTA tile 128 x 64 (64 x 32 where those are few), k slab 16, 4-stage mbarrier pipeline, 8 warps in a 4 x 2 grid,
+// 32 x 32 per warp (2 x 4 MMAs per k4; 16 x 16 and 1 x 2).  Thread 0 issues the TMA loads: a slot is
 // refilled one slab after its own, when every warp has left it.  (A producer warp
 // of its own costs the others registers: nine warps a CTA, two CTAs an SM,
 // leave 96 a thread, eight leave 128, which the epilogue's loads in flight need.)
@@ -44,13 +44,11 @@ void make_tmap_2d(CUtensorMap *tm, CUtensorMapDataType dt, int esize, const void
 }
 
 namespace {
-constexpr int BM = 128, BN = 64, BK = 16, STAGES = 4;
-constexpr int A_STAGE_BYTES = BM * BK * 8;  // 16 KB
-constexpr int B_STAGE_BYTES = BK * BN * 8;  // 8 KB
-constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+constexpr int BK = 16, STAGES = 4;
 constexpr int NCONSUMER_WARPS = 8;
 constexpr int NTHREADS = NCONSUMER_WARPS * 32;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+constexpr i64 DMMA_SMALL_MAX = 104;  // large tiles up to which small ones are taken
+constexpr int smem_bytes(int bm, int bn) { return STAGES * (bm + bn) * BK * 8 + 1024 /*align*/ + 256 /*barriers*/; }
 }  // namespace
 
 // A warp leaves a slab: its arrival lets thread 0 order the slot's refill.  The
@@ -65,9 +63,12 @@ __device__ __forceinline__ void leave_slab(uint64_t *bar, uint32_t seen, int lan
     if (lane == 0 || (v & (uint32_t)(m >> 31))) mbar_arrive(bar);  // m >= 0: lane 0 only
 }
 
+template <int BM, int BN>
 __global__ void __launch_bounds__(NTHREADS, 2)
 k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             double *__restrict__ C, i64 ldc, int M, int N, int K, int *__restrict__ ab, int upper_only) {
+    constexpr int A_STAGE_BYTES = BM * BK * 8, STAGE_BYTES = (BM + BN) * BK * 8;
+    constexpr int WM = BM / 4, WN = BN / 2, MT = WM / 16, NT = WN / 8;  // a warp's rows, columns, MMA tiles
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~uintptr_t(1023));
     uint64_t *full = (uint64_t *)(smem + STAGES * STAGE_BYTES);
@@ -108,22 +109,21 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         for (int kt = 0; kt < KT && kt < STAGES; ++kt) issue(kt);
     }
     {
-        // the C tile towards L2: two 128-byte lines a thread (rows of 512 bytes)
-        const int r = m0 + (int)(threadIdx.x >> 1), c = n0 + (int)(threadIdx.x & 1) * 32;
-        if (r < M) {
-            const double *p = C + (i64)r * ldc + c;
-            if (c < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-            if (c + 16 < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 16));
+        // the C tile towards L2, 128-byte lines
+#pragma unroll
+        for (int e = threadIdx.x; e < BM * BN / 16; e += NTHREADS) {
+            const int r = m0 + e / (BN / 16), c = n0 + e % (BN / 16) * 16;
+            if (r < M && c < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (i64)r * ldc + c));
         }
     }
 
     const int wm = warp & 3, wn = warp >> 2;  // 4 x 2 warps
     const int gid = lane >> 2, tig = lane & 3;
-    double acc[2][4][4];
+    double acc[MT][NT][4];
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < MT; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
+        for (int b = 0; b < NT; ++b)
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[a][b][c] = 0.0;
 
@@ -135,31 +135,31 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const uint8_t *sb = sa + A_STAGE_BYTES;
 #pragma unroll
         for (int k4 = 0; k4 < BK / 4; ++k4) {
-            double af[2][2], bf[4];
+            double af[MT][2], bf[NT];
             const int kc = k4 * 4 + tig;  // k column within the slab
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
+            for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const int r = wm * 32 + mt * 16 + gid + 8 * h;
+                    const int r = wm * WM + mt * 16 + gid + 8 * h;
                     // 128B swizzle: 16-byte chunk index XOR (row mod 8)
                     const int off = r * 128 + ((((kc * 8) >> 4) ^ (r & 7)) << 4) + ((kc * 8) & 15);
                     af[mt][h] = *(const double *)(sa + off);
                 }
             }
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int g = (wn * 32 + nt * 8) >> 3;
+            for (int nt = 0; nt < NT; ++nt) {
+                const int g = (wn * WN + nt * 8) >> 3;
                 bf[nt] = *(const double *)(sb + g * (BK * 64) + kc * 64 + gid * 8);
             }
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt) seen ^= __double2loint(af[mt][0]) ^ __double2loint(af[mt][1]);
+            for (int mt = 0; mt < MT; ++mt) seen ^= __double2loint(af[mt][0]) ^ __double2loint(af[mt][1]);
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) seen ^= __double2loint(bf[nt]);
+            for (int nt = 0; nt < NT; ++nt) seen ^= __double2loint(bf[nt]);
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
+            for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt)
+                for (int nt = 0; nt < NT; ++nt)
                     asm volatile(
                         "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, "
                         "{%6}, {%0,%1,%2,%3};"
@@ -183,15 +183,15 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const bool vec2 = ((ldc & 1) == 0) && ((((uintptr_t)C) & 15) == 0) && !(upper_only && m0 + BM - 1 > n0);
     const int cmin_row = upper_only ? 1 : 0;  // 1: column c is written only when c >= r
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-        double2 cv[2][4];
+    for (int mt = 0; mt < MT; ++mt) {
+        double2 cv[2][NT];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int r = m0 + wm * 32 + mt * 16 + gid + 8 * h;
+            const int r = m0 + wm * WM + mt * 16 + gid + 8 * h;
             const double *crow = C + (i64)r * ldc;
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int c = n0 + wn * 32 + nt * 8 + 2 * tig;
+            for (int nt = 0; nt < NT; ++nt) {
+                const int c = n0 + wn * WN + nt * 8 + 2 * tig;
                 if (r < M && c + 1 < N && vec2) cv[h][nt] = __ldcs((const double2 *)(crow + c));
                 else {
                     cv[h][nt].x = (r < M && c < N && (!cmin_row || c >= r)) ? crow[c] : 0.0;
@@ -201,12 +201,12 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int r = m0 + wm * 32 + mt * 16 + gid + 8 * h;
+            const int r = m0 + wm * WM + mt * 16 + gid + 8 * h;
             if (r >= M) continue;
             double *crow = C + (i64)r * ldc;
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int c = n0 + wn * 32 + nt * 8 + 2 * tig;
+            for (int nt = 0; nt < NT; ++nt) {
+                const int c = n0 + wn * WN + nt * 8 + 2 * tig;
                 double2 v;
                 v.x = cv[h][nt].x - acc[mt][nt][2 * h];
                 v.y = cv[h][nt].y - acc[mt][nt][2 * h + 1];
@@ -220,6 +220,21 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
 }
 
+template <int BM, int BN>
+static void launch_dmma_tile(double *C, i64 ldc, const double *A, i64 lda, const double *B, i64 ldb, i64 M, i64 N,
+                             i64 K, cudaStream_t s, bool upper_only) {
+    CUtensorMap tmA, tmB;
+    make_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, K, M, lda, BK, BM,
+                 CU_TENSOR_MAP_SWIZZLE_128B);
+    make_tmap_2d(&tmB, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, B, N, K, ldb, 8, BK,
+                 CU_TENSOR_MAP_SWIZZLE_NONE);
+    set_max_dyn_smem((const void *)k_gemm_dmma<BM, BN>, smem_bytes(BM, BN));
+    dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM));
+    k_gemm_dmma<BM, BN><<<grid, NTHREADS, smem_bytes(BM, BN), s>>>(tmA, tmB, C, ldc, (int)M, (int)N, (int)K, cur_abort(),
+                                                                   upper_only ? 1 : 0);
+    OXI_LAUNCH_CHECK();
+}
+
 void launch_gemm_dmma(double *C, i64 ldc, const double *A, i64 lda, const double *B, i64 ldb, i64 M,
                       i64 N, i64 K, cudaStream_t s, bool upper_only) {
     if (M <= 0 || N <= 0 || K <= 0) return;
@@ -231,17 +246,15 @@ void launch_gemm_dmma(double *C, i64 ldc, const double *A, i64 lda, const double
         launch_gemm_ref<double>(C, ldc, A, lda, B, ldb, M, N, K, s);
         return;
     }
-    CUtensorMap tmA, tmB;
-    make_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, K, M, lda, BK, BM,
-                 CU_TENSOR_MAP_SWIZZLE_128B);
-    make_tmap_2d(&tmB, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, B, N, K, ldb, 8, BK,
-                 CU_TENSOR_MAP_SWIZZLE_NONE);
-    set_max_dyn_smem((const void *)k_gemm_dmma, SMEM_BYTES);
-    dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM));
     ProfScope ps(KC_GEMM_DMMA, s, (upper_only ? 1.0 : 2.0) * M * N * K, 8.0 * (2.0 * M * N + M * K + K * N));
-    k_gemm_dmma<<<grid, NTHREADS, SMEM_BYTES, s>>>(tmA, tmB, C, ldc, (int)M, (int)N, (int)K, cur_abort(),
-                                                   upper_only ? 1 : 0);
-    OXI_LAUNCH_CHECK();
+    // Small tiles while the large ones leave SMs without one: a tile's time is its
+    // chain of products on one SM, whatever the other SMs do.  Large against small,
+    // us, by number of large tiles: 8 (960 x 64 x 64) 14.2, 10.3; 48 (3000 x 128 x
+    // 128) 19.4, 15.3; 96 (6144 x 128 x 128) 19.6, 18.4; 98 (896 x 896 x 128) 20.3,
+    // 17.8; 126 (8064 x 128 x 128) 19.2, 21.5; 148: 20.1, 23.1.
+    const i64 large = ((M + 127) / 128) * ((N + 63) / 64);
+    if (large <= DMMA_SMALL_MAX) launch_dmma_tile<64, 32>(C, ldc, A, lda, B, ldb, M, N, K, s, upper_only);
+    else launch_dmma_tile<128, 64>(C, ldc, A, lda, B, ldb, M, N, K, s, upper_only);
 }
 
 // ---------------------------------------------------------------------------

@@ -56,6 +56,21 @@ def test_wide_leaf_bit_identical(pkg, oracle, m):
         assert np.array_equal(_np(F.factors), Fo, equal_nan=True)
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 2, 2), (63, 30, 16), (64, 32, 18), (65, 34, 64), (130, 66, 128), (569, 128, 128)])
+def test_gemm_tiles_same_bits(pkg, m, n, k):
+    """Few 128 x 64 tiles: the update runs on 64 x 32 ones.  Every element is one
+    chain over k, so the rows of a taller update, which takes the large tiles, are
+    the same bits; and they are within k eps of the exact product."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    rows = 128 * 105
+    C, A = (torch.randn(rows, c, dtype=torch.float64, device="cuda", generator=g) for c in (n, k))
+    B = torch.randn(k, n, dtype=torch.float64, device="cuda", generator=g)
+    small = pkg.gemm_update(C[:m].clone(), A[:m].contiguous(), B)
+    assert torch.equal(small, pkg.gemm_update(C.clone(), A, B)[:m])
+    err = (small - (C[:m] - A[:m] @ B)).abs()
+    assert bool((err <= 2 * (k + 1) * EPS * (C[:m].abs() + A[:m].abs() @ B.abs())).all())
+
+
 def test_repeated_factorization_same_bits(pkg):
     """Both streams of the lookahead and all pipelines under load: every repetition
     gives the same factors."""
