@@ -38,40 +38,94 @@ namespace {
 constexpr int PO_NB = 128;          // block rows per step
 constexpr int PO_SB = 32;           // blocks inside a diagonal block
 constexpr int PO_NT = 256;
+constexpr int PO_FW = 4;             // diagonal block: warps that factor, the others update
+constexpr int PO_DT = 32 * PO_FW + 256;
 constexpr int PO_GB = 8;            // rows factored between two updates of the block
 // row pitches in shared memory: 4 modulo 16, no conflicts of a DMMA fragment's loads
 constexpr int PO_LP = PO_NB + 4, PO_CP = PO_SB + 4;
 }  // namespace
 
-// d = sqrt(a) and y = 1 / d for a finite a > 0: the approximate reciprocal
-// root, one cubic Newton step, and a fused correction of each result (the
-// latency of one chain instead of a square root followed by a division); the
-// library functions where an exponent could over- or underflow on the way.
-__device__ __forceinline__ void root_recip(double a, double &d, double &y) {
-    if (a > 0x1p-900 && a < 0x1p900) {
-        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-        const double e = fma(-(a * y), y, 1.0);
-        y = fma(y * e, fma(0.375, e, 0.5), y);
-        const double g = a * y;
-        d = fma(fma(-g, g, a), 0.5 * y, g);
-        y = fma(fma(-d, y, 1.0), y, y);
-    } else {
-        d = sqrt(a);
-        y = 1.0 / d;
-    }
+// d = sqrt(a), y = 1 / d and z, an approximation of 1 / d that is ready earlier,
+// for 2^-900 < a < 2^900: the approximate reciprocal root, one cubic Newton step
+// (z), and a fused correction of each result (the latency of one chain instead
+// of a square root followed by a division).
+__device__ __forceinline__ void root_recip(double a, double &d, double &y, double &z) {
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double e = fma(-(a * y), y, 1.0);
+    z = fma(y * e, fma(0.375, e, 0.5), y);
+    const double g = a * z;
+    d = fma(fma(-g, g, a), 0.5 * z, g);
+    y = fma(fma(-d, z, 1.0), z, z);
 }
-__device__ __forceinline__ void root_recip(float a, float &d, float &y) {
+__device__ __forceinline__ void root_recip(float a, float &d, float &y, float &z) {
     d = sqrtf(a);
-    y = 1.0f / d;
+    z = y = 1.0f / d;
 }
+__device__ __forceinline__ bool root_range(double a) { return a > 0x1p-900 && a < 0x1p900; }
+__device__ __forceinline__ bool root_range(float a) { return a > 0.0f && a <= 3.402823466e38f; }
 __device__ __forceinline__ bool exp_all_ones(double a) { return (__double2hiint(a) & 0x7ff00000) == 0x7ff00000; }
 __device__ __forceinline__ bool exp_all_ones(float a) { return (__float_as_uint(a) & 0x7f800000u) == 0x7f800000u; }
-// a / d with the reciprocal's rounding corrected by the remainder
+
+// Rows of an N x N diagonal block (upper, u) with one column x beside it:
+// u_cc = sqrt(u_cc), u_cj /= u_cc, x_c /= u_cc, then the rows below take the
+// products; sy, if not null, takes the reciprocals of the roots.  FAST has no branch: roots and quotients are products with the
+// reciprocal corrected by the remainder, and false is returned where a pivot or
+// a result leaves the range in which that holds (the caller starts again without
+// FAST, which divides).  Returns true with bad = the first pivot that is not
+// finite and positive (N: none) otherwise.
+template <bool FAST, int N, typename T>
+__device__ __forceinline__ bool chol_rows(T (&u)[N][N], T (&x)[N], T *sy, int &bad) {
+    bool ok = true;
+    bad = N;
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+        const T a = u[c][c];
+        T d, y, z;
+        if constexpr (FAST) {
+            ok = ok && root_range(a);
+            root_recip(a, d, y, z);
+        } else {
+            if (bad < N) continue;
+            if (!(a > T(0)) || exp_all_ones(a)) {
+                bad = c;
+                continue;
+            }
+            d = sqrt(a);
+            y = T(1) / d;
+        }
+        if (sy) sy[c] = y;
+        u[c][c] = d;
+#pragma unroll
+        for (int j = c; j < N; ++j) {  // j = c: the column beside the block
+            T &v = j == c ? x[c] : u[c][j];
+            if constexpr (FAST) {
+                const T q = v * z;
+                v = fma(fma(-q, d, v), z, q);
+            } else {
+                v = v / d;
+            }
+        }
+#pragma unroll
+        for (int i = c + 1; i < N; ++i) {
+#pragma unroll
+            for (int k = i; k < N; ++k) u[i][k] = fma(-u[c][i], u[c][k], u[i][k]);
+            x[i] = fma(-u[c][i], x[c], x[i]);
+        }
+    }
+    if constexpr (FAST) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            ok = ok && !exp_all_ones(x[i]);
+#pragma unroll
+            for (int k = i; k < N; ++k) ok = ok && !exp_all_ones(u[i][k]);
+        }
+    }
+    return ok;
+}
+
 template <typename T>
-__device__ __forceinline__ T scaled(T a, T d, T y) {
-    const T q = a * y;
-    const T r = fma(fma(-q, d, a), y, q);
-    return exp_all_ones(r) ? a / d : r;
+__device__ __forceinline__ void copy_async(T *dst, const T *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"((int)sizeof(T)) : "memory");
 }
 
 // four neighbours in shared memory, 16-byte aligned
@@ -90,94 +144,56 @@ __device__ __forceinline__ void store4(double *p, const double (&v)[4]) {
 __device__ __forceinline__ void store4(float *p, const float (&v)[4]) { *(float4 *)p = make_float4(v[0], v[1], v[2], v[3]); }
 
 // Cholesky of the t x t diagonal block (row-major upper, ld) in shared memory, by
-// groups of 8 rows: warp 0 factors the group's 8 x 8 diagonal block in
-// registers, the columns to the right are solved by substitution, one per
-// thread, and the rest takes the rank-8 update in 4 x 4 tiles.  Element for
-// element these are the operations of the reference leaf's column updates
+// groups of 8 rows.  Each of the factoring warps that has columns to the right factors
+// the group's 8 x 8 diagonal block in registers, each lane the whole of it (no
+// exchange between lanes, no barrier before the rows to the right), and takes
+// its own column along.  The updating warps then take the rank-8 product for the
+// next group's rows, and for the rest while the next group is factored.  These
+// are the operations of the reference leaf's column updates
 // (src/lapack/factorizations.jl:266-282), read through the transposition.
 // Winv: the inverses of a full block's 32 x 32 diagonal blocks, PO_SB x PO_SB
 // row-major each (upper), one warp each at the end.
-// Bound: latency of the 16 groups (eight dependent roots, reciprocals and scaled
-// rows in one warp, then two phases of the CTA).
+// Bound: latency of the 16 groups, each a chain of eight roots, quotients and
+// products (3200 cycles), the next rows' update (250) and two barriers.  Alone on
+// one B200: 80000 cycles; 472000 with one warp passing the block's rows by shuffles
+// (380000 of them), loads each waiting for the store of the one before (36000)
+// and the update between the groups (1500 each).  In the n = 4999 factorization,
+// beside the trailing update, 88 -> 53 us; the whole, with small tiles for the next
+// block's rows, 5.76 -> 4.06 ms.
 template <typename T>
-__global__ void __launch_bounds__(PO_NT) k_potrf_diag(T *__restrict__ U, i64 ld, int t, i64 g0,
+__global__ void __launch_bounds__(PO_DT) k_potrf_diag(T *__restrict__ U, i64 ld, int t, i64 g0,
                                                       int64_t *__restrict__ info, T *__restrict__ Winv) {
     extern __shared__ __align__(16) unsigned char po_smem_raw[];
     T *S = (T *)po_smem_raw;
     __shared__ T s_y[PO_NB];  // 1 / u_ii
-    __shared__ int s_fail;
+    __shared__ __align__(16) T s_d[PO_GB][PO_GB];  // a group's factored diagonal block
+    __shared__ int s_fail;            // 1 + the first column of the failing group
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_fail = (*(volatile int64_t *)info != 0) ? 1 : 0;
     __syncthreads();
     if (s_fail) return;  // an earlier block failed
-#pragma unroll 16
-    for (int e = tid; e < PO_NB * PO_NB; e += PO_NT) {
+    // the upper triangle, every element's copy in flight at once; identity past t
+    for (int e = tid; e < PO_NB * PO_NB; e += PO_DT) {
         const int i = e / PO_NB, j = e % PO_NB;
-        S[i * PO_LP + j] = (i < t && j < t) ? ((j >= i) ? U[(i64)i * ld + j] : T(0)) : (i == j ? T(1) : T(0));
+        if (j < i) continue;
+        if (j < t) copy_async(&S[i * PO_LP + j], U + (i64)i * ld + j);
+        else S[i * PO_LP + j] = i == j ? T(1) : T(0);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-#pragma unroll 1
-    for (int b0 = 0; b0 < t; b0 += PO_GB) {
-        if (warp == 0) {
-            const int col = lane & (PO_GB - 1);  // lanes 0..7 hold the columns (the others repeat them)
-            T x[PO_GB];
-#pragma unroll
-            for (int i = 0; i < PO_GB; ++i) x[i] = S[(b0 + i) * PO_LP + b0 + col];
-            bool fail = false;
-#pragma unroll
-            for (int c = 0; c < PO_GB; ++c) {
-                const T a = __shfl_sync(0xffffffffu, x[c], c);
-                if (!(a > T(0)) || exp_all_ones(a)) {  // not positive definite at global column g0 + b0 + c + 1
-                    if (!fail && lane == 0) {
-                        s_fail = 1;
-                        if (*info == 0) *info = g0 + b0 + c + 1;
-                    }
-                    fail = true;
-                }
-                if (!fail) {
-                    T d, y;
-                    root_recip(a, d, y);
-                    x[c] = (col == c) ? d : scaled(x[c], d, y);
-                    if (lane == c) s_y[b0 + c] = y;
-#pragma unroll
-                    for (int i = c + 1; i < PO_GB; ++i) x[i] = fma(-__shfl_sync(0xffffffffu, x[c], i), x[c], x[i]);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < PO_GB; ++i)
-                if (lane < PO_GB && i <= col) S[(b0 + i) * PO_LP + b0 + col] = x[i];
-        }
-        __syncthreads();
-        if (s_fail) break;
-        const int r0 = b0 + PO_GB;  // the columns to the right
-        if (tid < PO_NB - r0) {
-            // x_i = (a_i - sum_{p<i} u_pi x_p) / u_ii
-            const int j = r0 + tid;
-            T x[PO_GB];
-#pragma unroll
-            for (int i = 0; i < PO_GB; ++i) x[i] = S[(b0 + i) * PO_LP + j];
-#pragma unroll
-            for (int p = 0; p < PO_GB; ++p) {
-                const T *row = S + (b0 + p) * PO_LP + b0;
-                x[p] = scaled(x[p], row[p], s_y[b0 + p]);
-#pragma unroll
-                for (int i = p + 1; i < PO_GB; ++i) x[i] = fma(-row[i], x[p], x[i]);
-            }
-#pragma unroll
-            for (int i = 0; i < PO_GB; ++i) S[(b0 + i) * PO_LP + j] = x[i];
-        }
-        __syncthreads();
-        // a_ij -= sum_p u_pi u_pj (r0 <= i <= j), 4 x 4 tiles of the upper triangle
+    // FP32: the whole of it by 4 x 4 tiles of the upper triangle
+    auto update32 = [&](int b0) {
+        const int r0 = b0 + PO_GB;
         const int nt4 = (PO_NB - r0) / 4, tasks = nt4 * (nt4 + 1) / 2;
-        for (int q = tid; q < tasks; q += PO_NT) {
+        for (int q = tid; q < tasks; q += PO_DT) {
             int bj = (int)((sqrtf(8.0f * q + 1.0f) - 1.0f) * 0.5f);
             while ((bj + 1) * (bj + 2) / 2 <= q) ++bj;
             while (bj * (bj + 1) / 2 > q) --bj;
             const int bi = q - bj * (bj + 1) / 2;
             const int i = r0 + 4 * bi, j = r0 + 4 * bj;
-            T acc[4][4];
+            T v[4][4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) load4(acc[u], S + (i + u) * PO_LP + j);
+            for (int u = 0; u < 4; ++u) load4(v[u], S + (i + u) * PO_LP + j);
 #pragma unroll
             for (int p = 0; p < PO_GB; ++p) {
                 const T *row = S + (b0 + p) * PO_LP;
@@ -187,12 +203,158 @@ __global__ void __launch_bounds__(PO_NT) k_potrf_diag(T *__restrict__ U, i64 ld,
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) acc[u][w] = fma(-ui[u], uj[w], acc[u][w]);
+                    for (int w = 0; w < 4; ++w) v[u][w] = fma(-ui[u], uj[w], v[u][w]);
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) store4(S + (i + u) * PO_LP + j, acc[u]);
+            for (int u = 0; u < 4; ++u) store4(S + (i + u) * PO_LP + j, v[u]);
         }
-        __syncthreads();
+    };
+    auto bar = [] { asm volatile("bar.sync 1, %0;" ::"n"(PO_DT) : "memory"); };
+    // The two roles meet at two barriers a group: the group's rows are factored;
+    // the next group's rows are up to date.
+    if (warp < PO_FW) {
+#pragma unroll 1
+        for (int b0 = 0; b0 < t; b0 += PO_GB) {
+            const int r0 = b0 + PO_GB;  // the columns to the right
+            if (warp == 0 || r0 + 32 * warp < PO_NB) {
+                // u: the diagonal block; x: this thread's column,
+                // x_i = (a_i - sum_{p<i} u_pi x_p) / u_ii
+                const int j = r0 + tid, jc = min(j, PO_NB - 1);
+                T u[PO_GB][PO_GB], x[PO_GB];
+                int bad;
+                auto load = [&]() {
+#pragma unroll
+                    for (int i = 0; i < PO_GB; ++i) {
+                        const T *row = S + (b0 + i) * PO_LP;
+#pragma unroll
+                        for (int h = 0; h < PO_GB; h += 4)
+                            if (h + 3 >= i) {
+                                T v[4];
+                                load4(v, row + b0 + h);
+#pragma unroll
+                                for (int c = 0; c < 4; ++c) u[i][h + c] = v[c];
+                            }
+                        x[i] = row[jc];
+                    }
+                };
+                load();
+                if (!__all_sync(0xffffffffu, chol_rows<true>(u, x, tid == 0 ? s_y + b0 : nullptr, bad))) {
+                    load();
+                    chol_rows<false>(u, x, tid == 0 ? s_y + b0 : nullptr, bad);
+                    if (bad < PO_GB && tid == 0) {  // not positive definite at global column g0 + b0 + bad + 1
+                        s_fail = b0 + 1;
+                        if (*info == 0) *info = g0 + b0 + bad + 1;
+                    }
+                }
+                if (tid == 0) {  // not over the block itself: other warps may still read it
+#pragma unroll
+                    for (int i = 0; i < PO_GB; ++i) {
+#pragma unroll
+                        for (int h = 0; h < PO_GB; h += 4)
+                            if (h + 3 >= i) {
+                                const T v[4] = {u[i][h], u[i][h + 1], u[i][h + 2], u[i][h + 3]};
+                                store4(&s_d[i][h], v);
+                            }
+                    }
+                }
+                if (j < PO_NB && bad == PO_GB) {
+#pragma unroll
+                    for (int i = 0; i < PO_GB; ++i) S[(b0 + i) * PO_LP + j] = x[i];
+                }
+            }
+            bar();
+            if (s_fail) break;
+            if (tid < PO_GB * PO_GB && (tid & 7) >= (tid >> 3))
+                S[(b0 + (tid >> 3)) * PO_LP + b0 + (tid & 7)] = s_d[tid >> 3][tid & 7];
+            if (sizeof(T) == 4) update32(b0);
+            bar();
+        }
+        if (s_fail && tid < PO_GB * PO_GB && (tid & 7) >= (tid >> 3))  // the failing group's block as far as it got
+            S[(s_fail - 1 + (tid >> 3)) * PO_LP + s_fail - 1 + (tid & 7)] = s_d[tid >> 3][tid & 7];
+    } else {
+        // a_ij -= sum_p u_pi u_pj (r0 <= i <= j).  FP64: the block's 72 tiles of
+        // 16 x 8 on and above the diagonal stay in registers as the tensor cores'
+        // accumulators, nine a warp of the eight: slot e of warp w is row tile e of
+        // column tile w, then row tile e - w / 2 - 1 of column tile 15 - w.
+        constexpr int SLOTS = sizeof(T) == 8 ? 9 : 1;
+        const int uw = warp - PO_FW;
+        const int gid = lane >> 2, tig = lane & 3;
+        const int first = uw / 2 + 1;  // slots of the first column tile
+        auto tile_row = [&](int e) { return 16 * (e < first ? e : e - first); };
+        auto tile_col = [&](int e) { return 8 * (e < first ? uw : 15 - uw); };
+        T acc[SLOTS][4];
+        // the tiles of row tile lo (rest: below it) take the products of group b0's rows
+        // (what a tile holds below the diagonal or of finished rows is never read)
+        auto update = [&](int b0, bool rest) {
+            if constexpr (sizeof(T) == 8) {
+                const int r0 = b0 + PO_GB, lo = r0 & ~15;
+                double bf[2][2];
+#pragma unroll
+                for (int w = 0; w < 2; ++w)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) bf[w][h] = S[(b0 + 4 * h + tig) * PO_LP + 8 * (w == 0 ? uw : 15 - uw) + gid];
+#pragma unroll
+                for (int e = 0; e < SLOTS; ++e) {
+                    const int i = tile_row(e);
+                    if (tile_col(e) >= r0 && (rest ? i > lo : i == lo)) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const double *row = S + (b0 + 4 * h + tig) * PO_LP + i + gid;
+                            asm volatile(
+                                "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                                : "+d"(acc[e][0]), "+d"(acc[e][1]), "+d"(acc[e][2]), "+d"(acc[e][3])
+                                : "d"(-row[0]), "d"(-row[8]), "d"(e < first ? bf[0][h] : bf[1][h]));
+                        }
+                    }
+                }
+            }
+        };
+        if (sizeof(T) == 8) {
+#pragma unroll
+            for (int e = 0; e < SLOTS; ++e) {
+                const int i = tile_row(e), j = tile_col(e);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const T *p = S + (i + 8 * h + gid) * PO_LP + j + 2 * tig;
+                    acc[e][2 * h] = p[0];
+                    acc[e][2 * h + 1] = p[1];
+                }
+            }
+        }
+#pragma unroll 1
+        for (int b0 = 0; b0 < t; b0 += PO_GB) {
+            if (b0 > 0) update(b0 - PO_GB, true);  // beside this group's factorization
+            bar();
+            if (s_fail) {  // the rows below as far as they got
+                if constexpr (sizeof(T) == 8) {
+#pragma unroll
+                    for (int e = 0; e < SLOTS; ++e)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int i = tile_row(e) + 8 * h + gid;
+                            if (i >= b0 + PO_GB)
+                                *(double2 *)(S + i * PO_LP + tile_col(e) + 2 * tig) =
+                                    make_double2(acc[e][2 * h], acc[e][2 * h + 1]);
+                        }
+                }
+                break;
+            }
+            if constexpr (sizeof(T) == 8) {
+                // as far as the next group's rows, which go back to shared memory
+                const int r0 = b0 + PO_GB;
+                update(b0, false);
+#pragma unroll
+                for (int e = 0; e < SLOTS; ++e)
+                    if (tile_row(e) == (r0 & ~15) && tile_col(e) >= r0) {
+                        const int h = (r0 >> 3) & 1;
+                        *(double2 *)(S + (r0 + gid) * PO_LP + tile_col(e) + 2 * tig) =
+                            h ? make_double2(acc[e][2], acc[e][3]) : make_double2(acc[e][0], acc[e][1]);
+                    }
+            } else {
+                update32(b0);
+            }
+            bar();
+        }
     }
     __syncthreads();
     if (warp < PO_NB / PO_SB && t == PO_NB && !s_fail) {
@@ -211,7 +373,7 @@ __global__ void __launch_bounds__(PO_NT) k_potrf_diag(T *__restrict__ U, i64 ld,
         for (int i = 0; i < PO_SB; ++i) Winv[(b0 + i) * PO_SB + lane] = w[i];
     }
 #pragma unroll 16
-    for (int e = tid; e < PO_NB * PO_NB; e += PO_NT) {
+    for (int e = tid; e < PO_NB * PO_NB; e += PO_DT) {
         const int i = e / PO_NB, j = e % PO_NB;
         if (j >= i && j < t) U[(i64)i * ld + j] = S[i * PO_LP + j];
     }
@@ -252,9 +414,6 @@ __global__ void __launch_bounds__(PO_NT) k_potrf_row(const T *__restrict__ Ukk, 
         }
         return;
     }
-auto copy_async = [](T *dst, const T *src) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"((int)sizeof(T)) : "memory");
-    };
     for (int e = tid; e < PO_NB * PO_NB; e += PO_NT) {
         const int i = e / PO_NB, j = e % PO_NB;
         if (j / PO_SB > i / PO_SB) copy_async(&S.U[i][j], Ukk + (i64)i * ld + j);
@@ -414,7 +573,7 @@ void potrf_rowmajor(oxi_handle_s *h, T *U, i64 ld, i64 n, int64_t *d_info, T *wo
                 const int smem = (int)(sizeof(T) * PO_NB * PO_LP);
                 set_max_dyn_smem((const void *)k_potrf_diag<T>, smem);
                 ProfScope ps(KC_LEAF, s, (double)t * t * t * (2.0 / 3.0), 2.0 * sizeof(T) * t * t);
-                k_potrf_diag<T><<<1, PO_NT, smem, s>>>(Ukk, ld, t, k0, d_info, Winv);
+                k_potrf_diag<T><<<1, PO_DT, smem, s>>>(Ukk, ld, t, k0, d_info, Winv);
                 OXI_LAUNCH_CHECK();
             }
             const i64 right = n - k0 - t;

@@ -88,6 +88,9 @@ TriView<T> tri_view(const T *A, i64 lda, i64 n, bool lower, bool unit, bool rowa
 // right of the diagonal; rows past n are those of the identity.  Bound: latency
 // of the block columns' steps (up to seven, each two barriers and a chain of
 // up to 64 DMMAs); both triangles of a factor are one launch.
+// 62000 cycles for the longest strip (32000 of them DMMAs and their loads, 21000
+// the fetches, 12000 the diagonal inverses), 71000 before a diagonal block's
+// loads were issued together.
 // ---------------------------------------------------------------------------
 template <typename T>
 struct TriInvSmem {
@@ -650,7 +653,11 @@ static void tri_inv_launch(const TriView<T> &v0, const TriView<T> &v1, T *P0, T 
 }
 
 // First triangle, then the second, on X (n x nrhs, in place), by chunks of right-hand
-// sides.  Measured on one B200 (us for the pair of solves, before -> now):
+// sides.  Measured on one B200 (before: 64-row blocks, then -> now), us: inverses
+// and pair of FP64 solves, n = 256, one right-hand side 330 -> 66; n = 4096,
+// transposed, 8 right-hand sides 2090 -> 250 (178 the solves); FP32 pairs of the
+// refinement at n = 8192 with 16 right-hand sides 15400 -> 2130 in all; complex n =
+// 2048 about 8000 (a column at a time) -> 224.
 template <typename T, bool ROWACC0, bool ROWACC1>
 static void trsv_pair(oxi_handle_s *h, const TriView<T> &v0, const TriView<T> &v1, const T *P0, const T *P1, T *X,
                       i64 ldx, i64 nrhs, int *err) {

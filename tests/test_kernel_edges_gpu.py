@@ -153,6 +153,19 @@ def test_cholesky_blocks_and_first_failing_column(pkg, oracle, n):
         assert pkg.cholesky(M, check=False).info == oracle.potrf(M)[1] == bad + 1
 
 
+@pytest.mark.parametrize("n", [8, 127, 300])
+def test_cholesky_pivots_out_of_the_fast_range(pkg, n):
+    """Scaling by 2^-960 (exact) brings the pivots under 2^-900, where roots and
+    quotients are computed by the library functions.  |L L' - A| <= (n + 1) eps
+    |L||L'| elementwise, whose diagonal is that of A; twice that for the products
+    with inverted blocks."""
+    rng = np.random.default_rng(n)
+    G = rng.standard_normal((n, n))
+    A = G @ G.T + n * np.eye(n)
+    L = _np(pkg.cholesky(A * 2.0 ** -960).L) * 2.0 ** 480
+    assert np.abs(L @ L.T - A).max() <= 2 * (n + 1) * EPS * A.diagonal().max()
+
+
 @pytest.mark.parametrize("nrhs", [4, 5, 8, 9, 16])
 @pytest.mark.parametrize("n", [130, 300, 1027])
 def test_mixed_solve_right_hand_sides(pkg, n, nrhs):
