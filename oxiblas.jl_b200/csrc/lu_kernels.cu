@@ -801,14 +801,16 @@ static void launch_leaf_wr(T *P, i64 ld, i64 m, int w, i64 gofs, int64_t *ipiv, 
     count_launch();
 }
 
-// Threads and rows a thread by height.  256 threads of one row while 16 CTAs hold
-// the rows (4096): fewer warps to reduce over and twice the registers a thread;
-// above, 512 threads (FP32 one row to 8192, then two).  FP64, 32 columns, kernel
-// alone, 256 against 512 threads: 1024 rows 44 against 46 us, 4096 rows 47
-// against 47 (16 CTAs against 8).  FP32: 4096 rows 41 us with 256 threads, 8192
-// rows 44 with 512 (54 with two rows in 256).  The cluster has as many CTAs as the
-// rows need, not the next power of two: the exchange takes 413 cycles among 2 CTAs
-// and 746 among 16.
+// Threads and rows a thread by height, kernel alone, us on one B200: 256 threads of
+// one row while 16 CTAs hold the rows (FP64 1024 rows 44 against 52 with 512 threads, 4096 rows 47
+// against 54; FP32 256 rows 27 against 33, 4096 rows 41 against 43, with two rows a
+// thread 47): fewer warps to reduce over, twice the registers.  Above 4096 rows 512
+// threads (8192 rows: FP64 56 against 60 with 256 threads of two rows, FP32 45
+// against 50), from 8193 FP32 rows two a thread (16384: 55, 70 with four in 256).
+// (257 to 512 rows in one CTA of 512 threads: FP64 39 against 44, FP32 31 against
+// 40, and no difference to a whole solve, so no rule of their own.)
+// The cluster has as many CTAs as the rows need, not the next power of two: the
+// exchange takes 413 cycles among 2 CTAs and 746 among 16.
 template <typename T>
 void launch_leaf(T *P, i64 ld, i64 m, int w, i64 gofs, int64_t *ipiv, int64_t *info, int *moves,
                  int *nmoves, int leafw, cudaStream_t s, LeafPanel pn) {

@@ -47,10 +47,19 @@ __device__ __forceinline__ double2 zmsub2(double2 c, double2 a, double2 b) {
     return make_double2(fma(a.y, b.y, fma(-a.x, b.x, c.x)), fma(-a.y, b.x, fma(-a.x, b.y, c.y)));
 }
 
-// 1 / b, scaled by the larger of |b.r|, |b.i| (no spurious overflow)
+// 1 / b = conj(b) / |b|^2, b scaled by the power of two of the larger of |b.r|,
+// |b.i| (exact, and |b|^2 stays far from over- and underflow): one division instead of
+// the four of scaling by the component itself, which a column step waits for.
 __device__ __forceinline__ zd zrecip(zd b) {
-    double s = fmax(fabs(b.r), fabs(b.i));
-    if (s == 0.0) s = 1.0;
+    const double m = fmax(fabs(b.r), fabs(b.i));
+    if (m > 0x1p-1000 && m < 0x1p1000) {
+        const int e = (__double2hiint(m) >> 20) - 1023;
+        const double s = __hiloint2double((1023 - e) << 20, 0);  // 2^-e
+        const double br = b.r * s, bi = b.i * s;                 // the larger in [1, 2)
+        const double y = 1.0 / fma(br, br, bi * bi);
+        return {br * y * s, -(bi * y) * s};
+    }
+    const double s = m == 0.0 ? 1.0 : m;
     const double br = b.r / s, bi = b.i / s;
     const double den = (br * br + bi * bi) * s;
     return {br / den, -bi / den};
