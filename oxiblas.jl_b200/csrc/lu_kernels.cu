@@ -843,7 +843,6 @@ template void launch_leaf<float>(float *, i64, i64, int, i64, int64_t *, int64_t
 // touches 32 contiguous elements of each row (coalesced).
 // ---------------------------------------------------------------------------
 constexpr int MAX_MOVES = 64;
-constexpr int MAX_MOVES_LEAF = 64;  // a leaf of <= 32 columns moves at most 64 rows
 
 template <typename T>
 __global__ void k_rowmoves(T *__restrict__ W, i64 ld, i64 r0, const int *__restrict__ moves,
@@ -888,15 +887,6 @@ __global__ void k_rowmap_init(int *__restrict__ map, int len, int *__restrict__ 
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p < len) map[p] = p;
     if (p == 0) *listcnt = 0;
-}
-__global__ void k_rowmap_apply(int *__restrict__ map, int offset, const int *__restrict__ moves,
-                               const int *__restrict__ nmoves) {
-    const int e = threadIdx.x;
-    const int cnt = min(*nmoves, MAX_MOVES_LEAF);
-    int v = 0;
-    if (e < cnt) v = map[offset + moves[2 * e + 1]];
-    __syncthreads();
-    if (e < cnt) map[offset + moves[2 * e]] = v;
 }
 __global__ void k_rowmap_extract(const int *__restrict__ map, int len, int *__restrict__ list,
                                  int *__restrict__ cnt) {
@@ -961,10 +951,6 @@ __global__ void __launch_bounds__(256) k_rowmoves_big(T *__restrict__ W, i64 ld,
 void launch_rowmap_init(int *map, i64 len, int *listcnt, cudaStream_t s) {
     if (len <= 0) return;
     k_rowmap_init<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(map, (int)len, listcnt);
-    OXI_LAUNCH_CHECK();
-}
-void launch_rowmap_apply(int *map, i64 offset, const int *moves, const int *nmoves, cudaStream_t s) {
-    k_rowmap_apply<<<1, MAX_MOVES_LEAF, 0, s>>>(map, (int)offset, moves, nmoves);
     OXI_LAUNCH_CHECK();
 }
 void launch_rowmap_extract(const int *map, i64 len, int *list, int *cnt, cudaStream_t s) {

@@ -288,7 +288,6 @@ void launch_rowmoves(T *W, i64 ld, i64 r0, const int *moves, const int *nmoves, 
 
 // Per-panel composition of the leaves' row permutations (see lu_kernels.cu).
 void launch_rowmap_init(int *map, i64 len, int *listcnt, cudaStream_t s);
-void launch_rowmap_apply(int *map, i64 offset, const int *moves, const int *nmoves, cudaStream_t s);
 void launch_rowmap_extract(const int *map, i64 len, int *list, int *cnt, cudaStream_t s);
 template <typename T>
 void launch_rowmoves_big(T *W, i64 ld, i64 r0, const int *list, const int *cnt, int maxcnt, i64 c_lo,
