@@ -410,8 +410,9 @@ __device__ void panel_lu_reg(T *P, int ldp, int m, int k, Misc &S, PanelScratch 
 // products one after the other), the C elements requested before the products
 // so their round trip overlaps them.  A at Ap[r + kk lda], B at
 // Bp[kk bsk + c bsc]; rows and columns from m2 and steps from jb on are zeros.
+// (ldc may be the caller's leading dimension: column offsets need 64 bits.)
 __device__ __forceinline__ void update_tile_dmma(const double *Ap, int lda, const double *Bp, int bsk, int bsc,
-                                                 double *Cp, int ldc, int m2, int jb, int r0, int c0, int lane) {
+                                                 double *Cp, i64 ldc, int m2, int jb, int r0, int c0, int lane) {
     const int gid = lane >> 2, tig = lane & 3;
     double acc[2][2][4], cv[2][2][4];
 #pragma unroll
@@ -422,7 +423,7 @@ __device__ __forceinline__ void update_tile_dmma(const double *Ap, int lda, cons
             for (int e = 0; e < 4; ++e) {
                 acc[mt][nt][e] = 0.0;
                 const int r = r0 + mt * 16 + gid + 8 * (e >> 1), c = c0 + nt * 8 + 2 * tig + (e & 1);
-                cv[mt][nt][e] = (r < m2 && c < m2) ? Cp[r + c * ldc] : 0.0;
+                cv[mt][nt][e] = (r < m2 && c < m2) ? Cp[r + (i64)c * ldc] : 0.0;
             }
     for (int kk = 0; kk < jb; kk += 4) {
         const int kc = kk + tig;
@@ -456,13 +457,14 @@ __device__ __forceinline__ void update_tile_dmma(const double *Ap, int lda, cons
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int r = r0 + mt * 16 + gid + 8 * (e >> 1), c = c0 + nt * 8 + 2 * tig + (e & 1);
-                if (r < m2 && c < m2) Cp[r + c * ldc] = cv[mt][nt][e] - acc[mt][nt][e];
+                if (r < m2 && c < m2) Cp[r + (i64)c * ldc] = cv[mt][nt][e] - acc[mt][nt][e];
             }
 }
 
-// Right-looking blocked LU of W (n x n, column-major, ldw; shared or global).
+// Right-looking blocked LU of W (n x n, column-major, ldw; shared, or global
+// with any leading dimension).
 template <typename T>
-__device__ void lu_blocked(T *W, int ldw, int n, int nb, bool in_smem, T *sP, T *sU, Misc &S) {
+__device__ void lu_blocked(T *W, i64 ldw, int n, int nb, bool in_smem, T *sP, T *sU, Misc &S) {
     using namespace bt;
     PanelScratch &Q = *reinterpret_cast<PanelScratch *>(sU);
     for (int k = 0; k < n; k += nb) {
@@ -471,8 +473,8 @@ __device__ void lu_blocked(T *W, int ldw, int n, int nb, bool in_smem, T *sP, T 
         T *P;
         int ldp;
         if (in_smem) {
-            P = W + k + (i64)k * ldw;
-            ldp = ldw;
+            P = W + k + k * ldw;
+            ldp = (int)ldw;
         } else {
             P = sP;
             ldp = panel_pitch(m);
@@ -559,21 +561,22 @@ __device__ void lu_blocked(T *W, int ldw, int n, int nb, bool in_smem, T *sP, T 
             T *Cp = W + c2 + (i64)c2 * ldw;
             const T *Bp = in_smem ? W + k + (i64)c2 * ldw : sU;
             const int bsk = in_smem ? 1 : UP;
-            const int bsc = in_smem ? ldw : 1;
+            const int bsc = in_smem ? (int)ldw : 1;
             const int lane = (int)(threadIdx.x & 31);
             if constexpr (sizeof(T) == 8) {
                 const int RB = (m2 + 31) >> 5, tasks = RB * ((m2 + 15) >> 4);
                 for (int t = (int)(threadIdx.x >> 5); t < tasks; t += NW)
                     update_tile_dmma(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, (t % RB) * 32, (t / RB) * 16, lane);
             } else {
+                const int ldc = (int)ldw;  // FP32: shared memory or the CTA's own working matrix
                 const int RB = (m2 + 127) >> 7, tasks = RB * ((m2 + 7) >> 3);
                 for (int t = (int)(threadIdx.x >> 5); t < tasks; t += NW) {
                     const int r0 = (t % RB) * 128, c0 = (t / RB) * 8;
                     const int nu = min(4, (m2 - r0 + 31) >> 5);  // warp-uniform
-                    if (nu == 4) update_tile<4>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
-                    else if (nu == 3) update_tile<3>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
-                    else if (nu == 2) update_tile<2>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
-                    else update_tile<1>(Ap, ldp, Bp, bsk, bsc, Cp, ldw, m2, jb, r0, c0, lane);
+                    if (nu == 4) update_tile<4>(Ap, ldp, Bp, bsk, bsc, Cp, ldc, m2, jb, r0, c0, lane);
+                    else if (nu == 3) update_tile<3>(Ap, ldp, Bp, bsk, bsc, Cp, ldc, m2, jb, r0, c0, lane);
+                    else if (nu == 2) update_tile<2>(Ap, ldp, Bp, bsk, bsc, Cp, ldc, m2, jb, r0, c0, lane);
+                    else update_tile<1>(Ap, ldp, Bp, bsk, bsc, Cp, ldc, m2, jb, r0, c0, lane);
                 }
             }
         }
@@ -664,7 +667,7 @@ __device__ void warp_lu_solve(const T *W, int ldw, int n, T (&y)[bt::NQ]) {
 // are in flight (two columns a warp), so each step reads shared memory and the
 // L2 round trips overlap the steps.  Every thread calls it.
 template <typename T>
-__device__ void block_lu_solve(const T *W, int ldw, int n, T *stage, int cap, bool active, T (&y)[bt::NQ]) {
+__device__ void block_lu_solve(const T *W, i64 ldw, int n, T *stage, int cap, bool active, T (&y)[bt::NQ]) {
     using namespace bt;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int cs = min(2 * NW, cap / 2);
@@ -822,7 +825,7 @@ __global__ void __launch_bounds__(bt::NT, 2) k_lu_batched(const __grid_constant_
             S.bad = 0;
         }
         T *W;
-        int ldw;
+        i64 ldw;
         if constexpr (sizeof(T) == 8) {
             // plain FP64: the caller's matrix is the working matrix (in place)
             if (in_smem) {
@@ -831,7 +834,7 @@ __global__ void __launch_bounds__(bt::NT, 2) k_lu_batched(const __grid_constant_
                 for (int c = warp; c < n; c += NW) load_col(W + c * ldw, A + (i64)c * lda, n, lane);
             } else {
                 W = (T *)A;
-                ldw = (int)lda;
+                ldw = lda;
             }
             __syncthreads();
         } else {
@@ -937,7 +940,7 @@ __global__ void __launch_bounds__(bt::NT, 2) k_lu_batched(const __grid_constant_
                 }
                 __syncwarp();
                 if (in_smem) {
-                    if (active) warp_lu_solve<T>(W, ldw, n, y);
+                    if (active) warp_lu_solve<T>(W, (int)ldw, n, y);
                 } else {
                     block_lu_solve<T>(W, ldw, n, sP, 2 * d.nbmax, active, y);
                 }
@@ -975,7 +978,7 @@ __global__ void __launch_bounds__(bt::NT, 2) k_lu_batched(const __grid_constant_
                     }
                 }
                 if (in_smem) {
-                    if (active) warp_lu_solve<T>(W, ldw, n, y);
+                    if (active) warp_lu_solve<T>(W, (int)ldw, n, y);
                 } else {
                     block_lu_solve<T>(W, ldw, n, sP, 2 * d.nbmax, active, y);
                 }

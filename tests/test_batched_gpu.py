@@ -170,3 +170,34 @@ def test_getrf_batched_nan_pivot_rule(pkg, oracle, n_smem):
         assert _np(P.ipiv(0))[3] == 4
     finally:
         pkg.batched_set_tuning("fp64", 64, [8, 8, 16, 16, 16, 16, 16, 16])
+
+
+def test_batched_fp64_leading_dimension_beyond_32_bit_offsets(pkg, oracle):
+    """Blocks of tall matrices, factored in place: with lda = 9,000,000 an element
+    of column 240 is more than 2^31 elements from its matrix's start.  The rows
+    around the block keep what they hold."""
+    n, lda, pad = 256, 9_000_000, 64
+    assert (n - 16) * lda > 2 ** 31
+    rng = np.random.default_rng(35)
+    A, b = rng.standard_normal((n, n)) + 0.5 * n * np.eye(n), rng.standard_normal(n)
+    pool = torch.empty(n * lda, dtype=torch.float64, device="cuda")
+    around = pool.as_strided((n + pad, n), (1, lda))  # the block and the rows below it
+    around[n:] = 7.0
+    around[:n] = torch.from_numpy(A).cuda()
+    P = pkg.BatchedLU([n, 65], [1, 1])
+    P.load([A, A[:65, :65]], [b, b[:65]])
+    P.d_A[0], P.d_ld = pool.data_ptr(), P.d_ld.clone()
+    ldb = P.d_ld.clone()
+    P.d_ld[0] = lda
+    h = pkg.Handle.get()
+    v = lambda t: t.data_ptr()
+    st = h.lib.oxi_dgesv_batched_uneven(h.ptr, 3, 2, v(P.d_n), v(P.d_nrhs), v(P.d_A), v(P.d_ld), v(P.d_P), v(P.d_B),
+                                        v(ldb), v(P.d_X), v(ldb), v(P.d_info), v(P.d_iters), v(P.d_berr), 0, 0.0)
+    h.check(st)
+    Fo, ipo, _ = oracle.getrf(A)
+    assert np.array_equal(_np(P.ipiv(0)), ipo)
+    F = _np(around)
+    assert np.abs(F[:n] - Fo).max() <= 1e-12 * np.abs(Fo).max()
+    assert np.all(F[n:] == 7.0)
+    x = _np(P.B(0))[:, 0]
+    assert np.abs(A @ x - b).max() <= 30 * n * 2.3e-16 * np.abs(A).sum(1).max() * np.abs(x).max()
