@@ -51,16 +51,19 @@ constexpr i64 DMMA_SMALL_MAX = 104;  // large tiles up to which small ones are t
 constexpr int smem_bytes(int bm, int bn) { return STAGES * (bm + bn) * BK * 8 + 1024 /*align*/ + 256 /*barriers*/; }
 }  // namespace
 
-// A warp leaves a slab: its arrival lets thread 0 order the slot's refill.  The
-// arrival is made to depend on the values of all the slab's fragment loads (seen:
-// their low words combined): a load that is only issued may be overtaken by the
-// refill, whose writes come through the asynchronous proxy.  With 64 x 32 tiles
-// a few elements of one n = 2048 factorization in 350 took the last k4 step's
-// operands from the slab four further on.  The comparison costs a vote a slab
-// (6144 x 128 x 128: 18.2 us without, 18.1 to 19.5 us with it).
-__device__ __forceinline__ void leave_slab(uint64_t *bar, uint32_t seen, int lane, int m) {
-    const uint32_t v = __ballot_sync(0xffffffffu, seen == 0x9e3779b9u);
-    if (lane == 0 || (v & (uint32_t)(m >> 31))) mbar_arrive(bar);  // m >= 0: lane 0 only
+// A warp leaves a slab; thread 0 refills the slot when every warp has.  The slab
+// was read through the generic proxy and the refill writes through the
+// asynchronous one: an arrival releases the reads to other generic accesses only,
+// so each lane orders its own reads before later asynchronous writes with the
+// proxy fence, and lane 0 arrives for the warp.  Without the fence a refill could
+// overtake a load that was issued but not done: with 64 x 32 tiles one n = 2048
+// factorization in 350 (one in 64 with an arrival by every lane, which releases no
+// more and adds traffic to the barrier) took a few operands of the slab four
+// further on.
+__device__ __forceinline__ void leave_slab(uint64_t *bar, int lane) {
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
 }
 
 template <int BM, int BN>
@@ -129,7 +132,6 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
     for (int kt = 0; kt < KT; ++kt) {
         const int s = kt % STAGES;
-        uint32_t seen = 0;
         if (!mbar_wait<false>(&full[s], (kt / STAGES) & 1, ab, 2)) return;
         const uint8_t *sa = smem + s * STAGE_BYTES;
         const uint8_t *sb = sa + A_STAGE_BYTES;
@@ -153,10 +155,6 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 bf[nt] = *(const double *)(sb + g * (BK * 64) + kc * 64 + gid * 8);
             }
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) seen ^= __double2loint(af[mt][0]) ^ __double2loint(af[mt][1]);
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) seen ^= __double2loint(bf[nt]);
-#pragma unroll
             for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt)
@@ -167,7 +165,7 @@ k_gemm_dmma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                           "+d"(acc[mt][nt][3])
                         : "d"(af[mt][0]), "d"(af[mt][1]), "d"(bf[nt]));
         }
-        leave_slab(&empty[s], seen, lane, M);
+        leave_slab(&empty[s], lane);
         if (threadIdx.x == 0 && kt >= 1 && kt - 1 + STAGES < KT) {  // refill the slab before's slot
             const int pt = kt - 1;
             // (on a wait that gave up nothing is issued: every warp's next wait gives up too)
@@ -325,7 +323,6 @@ k_zgemm_dmma(const __grid_constant__ CUtensorMap tmAr, const __grid_constant__ C
         for (int c = 0; c < 4; ++c) cr[b][c] = ci[b][c] = 0.0;
     for (int kt = 0; kt < KT; ++kt) {
         const int s = kt % ZST;
-        uint32_t seen = 0;
         if (!mbar_wait<false>(&full[s], (kt / ZST) & 1, ab, 2)) return;
         const uint8_t *sa = smem + s * ZSTAGE;
 #pragma unroll
@@ -338,21 +335,19 @@ k_zgemm_dmma(const __grid_constant__ CUtensorMap tmAr, const __grid_constant__ C
                 const int off = r * 128 + ((((kc * 8) >> 4) ^ (r & 7)) << 4) + ((kc * 8) & 15);
                 ar[hh] = *(const double *)(sa + off);
                 ai[hh] = *(const double *)(sa + ZPLANE + off);
-                seen ^= __double2loint(ar[hh]) ^ __double2loint(ai[hh]);
             }
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
                 const int off = (wn * 4 + nt) * (BK * 64) + kc * 64 + gid * 8;
                 const double br = *(const double *)(sa + 2 * ZPLANE + off);
                 const double bi = *(const double *)(sa + 3 * ZPLANE + off);
-                seen ^= __double2loint(br) ^ __double2loint(bi);
                 dmma_16x8x4(cr[nt], ar[0], ar[1], br);
                 dmma_16x8x4(ci[nt], ar[0], ar[1], bi);
                 dmma_16x8x4(cr[nt], -ai[0], -ai[1], bi);
                 dmma_16x8x4(ci[nt], ai[0], ai[1], br);
             }
         }
-        leave_slab(&empty[s], seen, lane, M);
+        leave_slab(&empty[s], lane);
         if (threadIdx.x == 0 && kt >= 1 && kt - 1 + ZST < KT) {
             const int pt = kt - 1;
             // (on a wait that gave up nothing is issued: every warp's next wait gives up too)

@@ -81,6 +81,21 @@ def test_repeated_factorization_same_bits(pkg):
         assert torch.equal(pkg.lu(A).factors, F0)
 
 
+def test_repeated_products_same_bits(pkg):
+    """The slabs' refills of the complex product and of both tile sizes."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+
+    def randn(*shape, dtype=torch.float64):
+        return torch.randn(*shape, dtype=dtype, device="cuda", generator=g)
+    Z, S = randn(1500, 1500, dtype=torch.complex128), randn(1500, 1500)
+    S = S @ S.T + 1500 * torch.eye(1500, dtype=S.dtype, device="cuda")
+    C, A, B = randn(3000, 128), randn(3000, 128), randn(128, 128)
+    for count, f in ((150, lambda: pkg.lu(Z).factors), (300, lambda: pkg.cholesky(S).factors),
+                     (4000, lambda: pkg.gemm_update(C.clone(), A, B))):
+        first = f().clone()
+        assert all(torch.equal(f(), first) for _ in range(count))
+
+
 def test_leaf_zero_nan_and_extreme_pivots(pkg, oracle):
     rng = np.random.default_rng(7)
     A = rng.standard_normal((300, 64))
