@@ -14,9 +14,33 @@
 // right-hand sides through distributed shared memory, and each multiplies by
 // its strip of Inv_B and publishes its 32 rows.
 //
+// A product with an inverse is not backward stable: its error grows with the
+// condition of the block, that of substitution does not.  k_tri_inv therefore
+// leaves an estimate E of the inverse's quality with each strip, the largest row
+// sum of |Inv||M| times that of the 32 x 32 diagonal blocks (whose explicit
+// inverses the strip's rows are made with), and a superblock is solved by its
+// largest E:
+//   E <= kTriPlain: the product as it is (errors within a few roundings of
+//     substitution's);
+//   E <= tri_limit: one correction with the triangle itself, x += Inv (r - M x);
+//   beyond, and where a right-hand side or the product is not finite:
+//     substitution, the strips in turn.
+// Backward errors max|b - A x| / (|A||x| + |b|) of a solve by this rule's three forms,
+// in units of n eps (substitution / product / corrected), b = A * ones, kernels
+// exp(-((i-j)/w)^2) of order 512 restated in NumPy with these kernels' association:
+//   FP64 w = 1.4 (E = 60): 3e-3 / 5e-3 / 1e-3;  w = 2.2 (4e7): 2e-3 / 3e1 / 1e-3;
+//   w = 2.6 (2e11): 3e-3 / 1e5 / 2e-3;  w = 2.8 (6e13): 3e-3 / 5e7 / 2e1, and beyond
+//   that the correction fails altogether: the limit lies at 2^38 = 3e11;
+//   FP32 w = 2 (1e6): 3e-3 / 3 / 2e-3;  w = 2.1 (1e7): 3e-3 / 2e1 / 2e-3;  w = 2.2 (4e7):
+//   2e-3 / 1e1 / 5e-3;  w = 2.4 (6e9): 3e-3 / 4e2 / 3e1: 2^25 = 3e7.
+// Factors of random matrices have E of 4e5 to 4e7 and are corrected: 1e-2 / 5e-2 /
+// 1e-2 at order 1024.
+//
 // Bound: for one right-hand side of a large system the single pass over the
-// factor, otherwise the chain of superblocks: one hop through L2, one cluster
-// barrier and two 32 x SP products per SP rows.  Measured on one B200 against
+// factor, otherwise the chain of superblocks: one hop through L2, the 32 x SP product
+// with the last superblock solved, then three 32 x SP products (with 8 FP64 right-hand
+// sides 2300 cycles each, 750 of them the other strips' values) and three cluster
+// barriers (950 each) per SP rows.  Measured on one B200 against
 // the form it replaces (64-row blocks, a hop through L2 per block): see the
 // figures at trsv_pair.
 //
@@ -25,6 +49,7 @@
 // equals, and a reader polls the data itself.
 #include <cooperative_groups.h>
 #include <algorithm>
+#include <type_traits>
 #include "oxi_internal.h"
 #include "tma_util.cuh"
 
@@ -38,6 +63,10 @@ constexpr int ST = 32;
 // would not fit shared memory otherwise
 template <typename T> constexpr int SP_ = sizeof(T) == 16 ? 128 : 256;
 constexpr int INV_NT = 256;
+// The estimates up to which a superblock's product stands as it is, and with one
+// correction (see above).
+constexpr double kTriPlain = 64.0;
+template <typename T> constexpr double tri_limit = sizeof(T) == 4 ? 0x1p25 : 0x1p38;
 
 // One effective triangle in solve order.
 template <typename T>
@@ -61,6 +90,22 @@ __device__ __forceinline__ double shfl_xor(double v, int o) { return __shfl_xor_
 __device__ __forceinline__ zc64 shfl_xor(zc64 v, int o) {
     return zc64(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
 }
+__device__ __forceinline__ float shfl(float v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+__device__ __forceinline__ double shfl(double v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+__device__ __forceinline__ zc64 shfl(zc64 v, int l) {
+    return zc64(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
+}
+// size of an element (complex: within sqrt(2)), and whether it is finite
+__device__ __forceinline__ float mag(float v) { return fabsf(v); }
+__device__ __forceinline__ double mag(double v) { return fabs(v); }
+__device__ __forceinline__ double mag(zc64 v) { return fabs(v.x) + fabs(v.y); }
+__device__ __forceinline__ bool is_finite(float v) { return isfinite(v); }
+__device__ __forceinline__ bool is_finite(double v) { return isfinite(v); }
+__device__ __forceinline__ bool is_finite(zc64 v) { return isfinite(v.x) && isfinite(v.y); }
+// the estimate beside the inverses, stored as an element
+__device__ __forceinline__ double est_value(float v) { return v; }
+__device__ __forceinline__ double est_value(double v) { return v; }
+__device__ __forceinline__ double est_value(zc64 v) { return v.x; }
 __device__ __forceinline__ float conj_if(float v, int) { return v; }
 __device__ __forceinline__ double conj_if(double v, int) { return v; }
 __device__ __forceinline__ zc64 conj_if(zc64 v, int c) { return zc64(v.x, c ? -v.y : v.y); }
@@ -85,12 +130,13 @@ TriView<T> tri_view(const T *A, i64 lda, i64 n, bool lower, bool unit, bool rowa
 // registers.  Each block column's elements are requested before the products
 // of the one before it.  FP64 products run on the tensor cores, a 16 x 8 tile
 // per warp.  Written column by column, P[(strip * SP + c) * ST + r], zero to the
-// right of the diagonal; rows past n are those of the identity.  Bound: latency
+// right of the diagonal; rows past n are those of the identity; behind them the
+// strips' estimates (see the head of the file).  Bound: latency
 // of the block columns' steps (up to seven, each two barriers and a chain of
 // up to 64 DMMAs); both triangles of a factor are one launch.
 // 62000 cycles for the longest strip (32000 of them DMMAs and their loads, 21000
 // the fetches, 12000 the diagonal inverses), 71000 before a diagonal block's
-// loads were issued together.
+// loads were issued together, and about 5000 for the estimate.
 // ---------------------------------------------------------------------------
 template <typename T>
 struct TriInvSmem {
@@ -151,7 +197,7 @@ __device__ __forceinline__ void inv_product(const T *A, int ap, const T *B, int 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(INV_NT) k_tri_inv(const TriView<T> v0, const TriView<T> v1, T *__restrict__ P0,
+__global__ void __launch_bounds__(INV_NT, 1) k_tri_inv(const TriView<T> v0, const TriView<T> v1, T *__restrict__ P0,
                                                     T *__restrict__ P1) {
     constexpr int SP = SP_<T>, NS = SP / ST, DP = TriInvSmem<T>::DP, YP = TriInvSmem<T>::YP;
     constexpr int PRE = (NS - 1) * ST * ST / INV_NT;
@@ -159,8 +205,20 @@ __global__ void __launch_bounds__(INV_NT) k_tri_inv(const TriView<T> v0, const T
     TriInvSmem<T> &S = *reinterpret_cast<TriInvSmem<T> *>(tri_smem);
     const TriView<T> &v = blockIdx.y ? v1 : v0;
     T *P = blockIdx.y ? P1 : P0;
+    using R = decltype(mag(T()));
+    __shared__ R s_w[SP];          // row sums of |M|, rows up to this strip's
+    __shared__ R s_k[NS], s_e[INV_NT / 32];  // |D^-1||D| of the diagonal blocks, |Y||M| of a warp's rows
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int g = blockIdx.x, s = g % NS;
+    auto larger = [](R a, R b) { return (a >= b || a != a) ? a : b; };  // keeps a NaN
+    // sum of |row| over ST columns, from the lane's own on (no bank conflicts), four
+    // chains of additions
+    auto row_sum = [&](const T *row) {
+        R a[4] = {R(0), R(0), R(0), R(0)};
+#pragma unroll
+        for (int e = 0; e < ST; ++e) a[e & 3] += mag(row[(e + lane) & 31]);
+        return (a[0] + a[1]) + (a[2] + a[3]);
+    };
     const i64 r0 = (i64)(g / NS) * SP;  // the superblock's first row
     const bool rowacc = v.cs == 1 || v.cs == -1;
     const T *base = v.a + r0 * (v.rs + v.cs);
@@ -199,6 +257,8 @@ __global__ void __launch_bounds__(INV_NT) k_tri_inv(const TriView<T> v0, const T
             D[i][j] = (i < ds && (j < i || (j == i && !v.unit))) ? conj_if(xd[e], v.conj) : i == j ? T(1) : T(0);
         }
         __syncwarp();
+        const R wsum = row_sum(D[lane]);
+        s_w[d0 + lane] = wsum;
         // column `lane` of the inverse, eight rows at a time (rolled: unrolled over
         // the 32 rows the code outgrows the instruction cache it runs through once):
         // the rows by substitution in registers, their products off the rows below.
@@ -243,6 +303,17 @@ __global__ void __launch_bounds__(INV_NT) k_tri_inv(const TriView<T> v0, const T
 #pragma unroll
                 for (int u = 0; u < 8; ++u) xr[q][u] = xr[q + 1][u];
         }
+        __syncwarp();
+        R k4[4] = {R(0), R(0), R(0), R(0)};
+#pragma unroll
+        for (int e = 0; e < ST; ++e) k4[e & 3] += mag(D[lane][(e + lane) & 31]) * s_w[d0 + ((e + lane) & 31)];
+        R k = (k4[0] + k4[1]) + (k4[2] + k4[3]);
+        // an inverse near or among the subnormal numbers has lost digits
+        constexpr R tiny = sizeof(R) == 4 ? R(0x1p-102) : R(0x1p-969);
+        if (!(mag(D[lane][lane]) >= tiny)) k = R(INFINITY);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) k = larger(k, shfl_xor(k, o));
+        if (lane == 0) s_k[warp] = k;
     }
     __syncthreads();
     for (int e = t; e < ST * SP; e += INV_NT) {
@@ -259,6 +330,7 @@ __global__ void __launch_bounds__(INV_NT) k_tri_inv(const TriView<T> v0, const T
         }
         __syncthreads();
         if (b > 0) fetch(b - 1);
+        if (t < K) s_w[(b + 1) * ST + t] += row_sum(S.L[t]);
         inv_product<T>(&S.Y[0][(b + 1) * ST], YP, &S.L[0][0], DP, K, &S.Z[0][0], DP, true);
         __syncthreads();
         inv_product<T>(&S.Z[0][0], DP, &S.D[b][0][0], DP, ST, &S.Y[0][b * ST], YP, false);
@@ -270,6 +342,26 @@ __global__ void __launch_bounds__(INV_NT) k_tri_inv(const TriView<T> v0, const T
     for (int e = t; e < SP * ST; e += INV_NT) {  // a warp: eight rows of four columns
         const int l = e & 31, q = e >> 5, r = (l & 7) + 8 * (q & 3), c = (l >> 3) + 4 * (q >> 2);
         Pg[c * ST + r] = S.Y[r][c];
+    }
+    // the strip's estimate, behind the inverses: eight lanes a row
+    R e4[4] = {R(0), R(0), R(0), R(0)};
+    for (int c = t & 7; c < (s + 1) * ST; c += 32)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) e4[u] += mag(S.Y[t >> 3][c + 8 * u]) * s_w[c + 8 * u];
+    R e = (e4[0] + e4[1]) + (e4[2] + e4[3]);
+    e += shfl_xor(e, 1);
+    e += shfl_xor(e, 2);
+    e += shfl_xor(e, 4);
+    e = larger(e, shfl_xor(e, 8));
+    e = larger(e, shfl_xor(e, 16));
+    if (lane == 0) s_e[warp] = e;
+    __syncthreads();
+    if (t == 0) {
+        R k = s_k[0];
+        for (int q = 1; q < INV_NT / 32; ++q) e = larger(e, s_e[q]);
+        for (int q = 1; q <= s; ++q) k = larger(k, s_k[q]);
+        const R est = e * k;
+        P[(i64)((v.n + SP - 1) / SP) * SP * SP + g] = T(est == est ? est : R(INFINITY));
     }
 }
 
@@ -395,12 +487,18 @@ template <typename T, int NR>
 struct TriSolveSmem {
     static constexpr int SP = SP_<T>, NS = SP / ST;
     // pitch of a row's values: 16 bytes more keep eight lanes' 16-byte reads of
-    // eight rows free of bank conflicts
-    static constexpr int XP = NR * (int)sizeof(T) >= 32 ? NR + 16 / (int)sizeof(T) : NR;
-    T inv[SP][ST];       // this strip of the superblock's inverse, by columns
+    // eight rows free of bank conflicts, 32 bytes a DMMA fragment's loads
+    static constexpr int XP = NR * (int)sizeof(T) >= 32 ? NR + (sizeof(T) == 8 && NR == 8 ? 32 : 16) / (int)sizeof(T) : NR;
+    // a column's pitch: 16-byte rows, and 4 modulo 16 for the DMMA fragments
+    static constexpr int MP = ST + 4;
+    T inv[SP][MP];       // this strip of the superblock's inverse, by columns
+    T m[SP][MP];         // this strip of the superblock's triangle, by columns
     T xs[2][SP * XP];    // solved values being multiplied, double-buffered
-    T part[NS][NR][ST];  // per-warp partial sums
-    T r[ST][NR];         // the strip's right-hand side, read by the other strips
+    T part[NS][NR][MP];  // per-warp partial sums (the sums read rows of all right-hand sides)
+    // read by the other strips: the strip's right-hand side, its product with the
+    // inverse (or its solution), the residual of that
+    T r[ST][NR], x[ST][NR], d[ST][NR];
+    int bad[2];          // values of r, of x, that are not finite
 };
 
 template <typename T, bool ROWACC, int NR>
@@ -413,7 +511,7 @@ k_tri_solve(const TriView<T> v, const T *__restrict__ P, T *__restrict__ X, i64 
     constexpr int RPW = ST / NS, CPL = SP / 32;  // ROWACC: rows per warp, columns per lane
     // the next tile is loaded ahead where two fit the registers
     constexpr bool AHEAD = sizeof(T) <= 8;
-    constexpr int XP = TriSolveSmem<T, NR>::XP;
+    constexpr int XP = TriSolveSmem<T, NR>::XP, MP = TriSolveSmem<T, NR>::MP;
     extern __shared__ __align__(16) unsigned char tri_smem[];
     TriSolveSmem<T, NR> &S = *reinterpret_cast<TriSolveSmem<T, NR> *>(tri_smem);
     __shared__ int s_blk;
@@ -423,6 +521,7 @@ k_tri_solve(const TriView<T> v, const T *__restrict__ P, T *__restrict__ X, i64 
     const int n = v.n, nsb = (n + SP - 1) / SP;
     // the ticket counts from -1 (cleared with the exchange words); an aborted call takes no block
     if (s == 0 && t == 0) s_blk = aborted(err) ? nsb : atomicAdd(ticket, 1) + 1;
+    if (t < 2) S.bad[t] = 0;
     cl.sync();
     const int B = *cl.map_shared_rank(&s_blk, 0);
     if (B >= nsb) {
@@ -439,6 +538,32 @@ k_tri_solve(const TriView<T> v, const T *__restrict__ P, T *__restrict__ X, i64 
 #pragma unroll
         for (int c = 0; c < ST; ++c) S.inv[warp * ST + c][lane] = Pg[(warp * ST + c) * ST + lane];
     }
+    // how the superblock is solved (the same in all its strips): 0 the product, 1
+    // with a correction, 2 substitution
+    int mode;
+    {
+        double est = 0.0;
+        if (lane < NS && (i64)B * SP + lane * ST < n) est = est_value(P[(i64)nsb * SP * SP + B * NS + lane]);
+#pragma unroll
+        for (int o = NS / 2; o > 0; o >>= 1) est = fmax(est, shfl_xor(est, o));
+        est = shfl(est, 0);
+        mode = est <= kTriPlain ? 0 : (est <= tri_limit<T> ? 1 : 2);
+    }
+    // the strip of the triangle: warp w its block of columns w
+    auto load_triangle = [&]() {
+        if (warp > s || rows <= 0) return;
+        const T *p = v.a + r0 * v.rs + ((i64)B * SP + warp * ST) * v.cs;
+        T a[ST];
+#pragma unroll
+        for (int e = 0; e < ST; ++e) {
+            const int i = ROWACC ? e : lane, j = ROWACC ? lane : e;
+            a[e] = (i < rows && (warp < s || j < i || (j == i && !v.unit))) ? conj_if(p[i * v.rs + j * v.cs], v.conj)
+                                                                            : T(warp == s && i == j ? 1 : 0);
+        }
+#pragma unroll
+        for (int e = 0; e < ST; ++e) S.m[warp * ST + (ROWACC ? lane : e)][ROWACC ? e : lane] = a[e];
+    };
+    if (mode > 0) load_triangle();
     constexpr int V = ROWACC ? RPW * NR : NR;             // accumulators per lane
     constexpr int OUT = (ST * NR + TRI_NT - 1) / TRI_NT;  // outputs per thread
     // outputs of the first product: (row, rhs) of thread t's q-th value
@@ -583,52 +708,185 @@ k_tri_solve(const TriView<T> v, const T *__restrict__ P, T *__restrict__ X, i64 
 #pragma unroll
                 for (int w = 0; w < NS; ++w) sum += S.part[w][k][row];
             }
-            S.r[row][k] = bv[q] - sum;
+            const T v0 = bv[q] - sum;
+            S.r[row][k] = v0;
+            if (!is_finite(v0)) S.bad[0] = 1;
         }
     }
     cl.sync();
 
-    // ---- x = Inv r: warp w takes strip w's 32 columns, a lane one row ----
-    T o[NR];
-#pragma unroll
-    for (int k = 0; k < NR; ++k) o[k] = T(0);
-    if (warp <= s && rows > 0) {
-        const T *rr = cl.map_shared_rank(&S.r[0][0], warp) + lane * NR;
-        T *xs = S.xs[0];
-        {
-            T x[NR];
-            get_row<T, NR>(x, rr);
-            put_row<T, NR>(xs + t * XP, x);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int c = 0; c < ST; ++c) {
-            const T iv = S.inv[warp * ST + c][lane];
-            T x[NR];
-            get_row<T, NR>(x, xs + (warp * ST + c) * XP);
-#pragma unroll
-            for (int k = 0; k < NR; ++k) o[k] = mad(iv, x[k], o[k]);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < NR; ++k) S.part[warp][k][lane] = o[k];
-    __syncthreads();
-    for (int e = t; e < ST * NR; e += TRI_NT) {
-        const int row = e / NR, k = e % NR;
-        T x = T(0);
-#pragma unroll
-        for (int w = 0; w < NS; ++w) x += S.part[w][k][row];
+    // ---- the superblock's own triangle ----
+    auto any_bad = [&](int i) -> bool {
+        const int b = lane < NS ? *cl.map_shared_rank(&S.bad[i], lane) : 0;
+        return __any_sync(0xffffffffu, b != 0);
+    };
+    auto publish = [&](int row, int k, T x) {
         if (row < rows) {
             EW::publish(exch + ((r0 + row) * NR + k) * TW, x);
             X[xrow(r0 + row) + (i64)k * ldx] = x;
         }
+    };
+    // the strips' values of src, strip w to warp w: 16 contiguous bytes a lane at a time
+    // (of a row each, 64-byte strides, 16 KB take 1700 cycles)
+    constexpr int XB = NR * (int)sizeof(T), CPR = XB >= 16 ? XB / 16 : NR;  // a row's bytes, its chunks
+    using Chunk = typename std::conditional<(XB >= 16), int4, T>::type;
+    struct Chunks {
+        Chunk c[CPR];
+    } xv;
+    auto fetch = [&](T *src) {
+        if (warp <= s && rows > 0) {
+            const Chunk *p = reinterpret_cast<const Chunk *>(cl.map_shared_rank(src, warp));
+#pragma unroll
+            for (int i = 0; i < CPR; ++i) xv.c[i] = p[i * 32 + lane];
+        }
+    };
+    auto keep = [&]() {  // into the warp's rows of xs
+#pragma unroll
+        for (int i = 0; i < CPR; ++i) {
+            const int c = i * 32 + lane;
+            *reinterpret_cast<Chunk *>(S.xs[0] + (warp * ST + c / CPR) * XP + c % CPR * (NR / CPR)) = xv.c[i];
+        }
+    };
+    // The strip's rows of Mat times those values, warp w strip w's 32 columns, then
+    // sink(row, rhs, sum).  With a lane per row, 16-byte loads of a row's values (the
+    // same for all lanes, and yet four passes of the shared memory each) bound the
+    // product: 5200 cycles with 8 FP64 values, 6000 with 16 FP32 ones.  So FP64 runs
+    // on the tensor cores from 4 right-hand sides on, and FP32 by tiles of 4 rows from
+    // 8 on.
+    auto multiply = [&](const T *Mat, auto &&sink) {
+        const bool mine = warp <= s && rows > 0;
+        __syncwarp();
+        if (mine) keep();
+        __syncwarp();
+        const T *A = Mat + warp * ST * MP, *xs = S.xs[0] + warp * ST * XP;
+        if constexpr (sizeof(T) == 8 && NR >= 4) {
+            const int gid = lane >> 2, tig = lane & 3;
+            double c[2][4] = {};
+            if (mine)
+#pragma unroll
+                for (int kk = 0; kk < ST; kk += 4) {
+                    const double xb = gid < NR ? xs[(kk + tig) * XP + (gid < NR ? gid : 0)] : 0.0;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        asm volatile(
+                            "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                            : "+d"(c[h][0]), "+d"(c[h][1]), "+d"(c[h][2]), "+d"(c[h][3])
+                            : "d"(A[(kk + tig) * MP + 16 * h + gid]), "d"(A[(kk + tig) * MP + 16 * h + gid + 8]), "d"(xb));
+                }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (2 * tig + (e & 1) < NR) S.part[warp][2 * tig + (e & 1)][16 * h + gid + 8 * (e >> 1)] = c[h][e];
+        } else if constexpr (sizeof(T) == 4 && NR >= 8) {
+            constexpr int KW = NR / 4;
+            const int r4 = (lane & 7) * 4, k0 = (lane >> 3) * KW;
+            T o[KW][4];
+#pragma unroll
+            for (int k = 0; k < KW; ++k)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) o[k][i] = T(0);
+            if (mine)
+#pragma unroll 8
+                for (int c = 0; c < ST; ++c) {
+                    T m[4], x[KW];
+                    get_row<T, 4>(m, A + c * MP + r4);
+                    if constexpr (KW == 4) get_row<T, 4>(x, xs + c * XP + k0);
+                    else *(float2 *)x = *(const float2 *)(xs + c * XP + k0);
+#pragma unroll
+                    for (int k = 0; k < KW; ++k)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) o[k][i] = mad(m[i], x[k], o[k][i]);
+                }
+#pragma unroll
+            for (int k = 0; k < KW; ++k) put_row<T, 4>(&S.part[warp][k0 + k][r4], o[k]);
+        } else {
+            T o[NR];
+#pragma unroll
+            for (int k = 0; k < NR; ++k) o[k] = T(0);
+            if (mine)
+#pragma unroll
+                for (int c = 0; c < ST; ++c) {
+                    const T mv = A[c * MP + lane];
+                    T x[NR];
+                    get_row<T, NR>(x, xs + c * XP);
+#pragma unroll
+                    for (int k = 0; k < NR; ++k) o[k] = mad(mv, x[k], o[k]);
+                }
+#pragma unroll
+            for (int k = 0; k < NR; ++k) S.part[warp][k][lane] = o[k];
+        }
+        __syncthreads();
+        for (int e = t; e < ST * NR; e += TRI_NT) {
+            const int row = e / NR, k = e % NR;
+            T x = T(0);
+#pragma unroll
+            for (int w = 0; w < NS; ++w) x += S.part[w][k][row];
+            sink(row, k, x);
+        }
+    };
+    const int planned = mode;
+    fetch(&S.r[0][0]);
+    if (any_bad(0)) mode = 2;
+    if (mode == 0) {
+        multiply(&S.inv[0][0], publish);
+    } else if (mode == 1) {
+        multiply(&S.inv[0][0], [&](int row, int k, T x) {
+            S.x[row][k] = x;
+            if (!is_finite(x)) S.bad[1] = 1;
+        });
+        cl.sync();
+        fetch(&S.x[0][0]);
+        if (any_bad(1)) {
+            mode = 2;
+        } else {
+            multiply(&S.m[0][0], [&](int row, int k, T x) { S.d[row][k] = S.r[row][k] - x; });
+            cl.sync();
+            fetch(&S.d[0][0]);
+            multiply(&S.inv[0][0], [&](int row, int k, T x) { publish(row, k, S.x[row][k] + x); });
+        }
     }
-    cl.sync();  // the other strips have read this one's right-hand side
+    if (mode == 2) {
+        // the strips in turn, a right-hand side per warp
+        if (planned == 0) load_triangle();
+        __syncthreads();
+        for (int q = 0; q < NS; ++q) {
+            if (s == q) {
+                for (int k = warp; k < NR; k += NS) {
+                    T y = S.r[lane][k];
+                    for (int p = 0; p < rows; ++p) {
+                        T xp = shfl(y, p);
+                        if (!v.unit) xp = xp / S.m[s * ST + p][p];
+                        if (lane > p) y = mad(-S.m[s * ST + p][lane], xp, y);
+                        else if (lane == p) y = xp;
+                    }
+                    S.x[lane][k] = y;
+                    publish(lane, k, y);
+                }
+            }
+            cl.sync();
+            if (s > q && rows > 0) {
+                T *xq = S.xs[0];
+                const T *src = cl.map_shared_rank(&S.x[0][0], q);
+                for (int e = t; e < ST * NR; e += TRI_NT) xq[e] = src[e];
+                __syncthreads();
+                for (int e = t; e < ST * NR; e += TRI_NT) {
+                    const int row = e % ST, k = e / ST;
+                    T y = S.r[row][k];
+#pragma unroll 8
+                    for (int p = 0; p < ST; ++p) y = mad(-S.m[q * ST + p][row], xq[p * NR + k], y);
+                    S.r[row][k] = y;
+                }
+                __syncthreads();
+            }
+        }
+    }
+    cl.sync();  // the other strips have read this one's values
 }
 
 template <typename T>
 i64 tri_inverse_elems(i64 n) {
-    return (n + SP_<T> - 1) / SP_<T> * SP_<T> * (i64)SP_<T>;
+    return (n + SP_<T> - 1) / SP_<T> * (SP_<T> * (i64)SP_<T> + SP_<T> / ST);  // the inverses, an estimate a strip
 }
 template i64 tri_inverse_elems<float>(i64);
 template i64 tri_inverse_elems<double>(i64);
@@ -653,11 +911,13 @@ static void tri_inv_launch(const TriView<T> &v0, const TriView<T> &v1, T *P0, T 
 }
 
 // First triangle, then the second, on X (n x nrhs, in place), by chunks of right-hand
-// sides.  Measured on one B200 (before: 64-row blocks, then -> now), us: inverses
-// and pair of FP64 solves, n = 256, one right-hand side 330 -> 66; n = 4096,
-// transposed, 8 right-hand sides 2090 -> 250 (178 the solves); FP32 pairs of the
-// refinement at n = 8192 with 16 right-hand sides 15400 -> 2130 in all; complex n =
-// 2048 about 8000 (a column at a time) -> 224.
+// sides.  Measured on one B200, us, in 64-row blocks -> superblocks by the product
+// alone -> by the rule at the head of the file (all of these corrected): inverses and
+// pair of FP64 solves, n = 256, one right-hand side 330 -> 66 -> 80; n = 4096, transposed,
+// 8 right-hand sides 2090 -> 250 -> 321 (243 the solves); FP32 pairs of the refinement at
+// n = 8192 with 16 right-hand sides 15400 -> 2130 -> 3090 in all; complex n = 2048 about
+// 8000 (substitution, a column at a time) -> 224 -> 290.  By substitution, n = 2048, one
+// right-hand side: 406, complex 1290 (130 and 290 by corrected products).
 template <typename T, bool ROWACC0, bool ROWACC1>
 static void trsv_pair(oxi_handle_s *h, const TriView<T> &v0, const TriView<T> &v1, const T *P0, const T *P1, T *X,
                       i64 ldx, i64 nrhs, int *err) {
