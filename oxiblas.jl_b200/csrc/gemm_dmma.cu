@@ -396,6 +396,9 @@ bool zgemm_dmma_applicable(const double *Ar, const double *Ai, const double *Br,
 void launch_zgemm_dmma(double *Cr, double *Ci, const double *Ar, const double *Ai, const double *Br, const double *Bi,
                        i64 ld, i64 M, i64 N, i64 K, cudaStream_t s) {
     if (M <= 0 || N <= 0 || K <= 0) return;
+    constexpr i64 rows_max = 65535ll * ZM;  // a grid's rows of tiles (a tall matrix may have more)
+    for (; M > rows_max; M -= rows_max, Ar += rows_max * ld, Ai += rows_max * ld, Cr += rows_max * ld, Ci += rows_max * ld)
+        launch_zgemm_dmma(Cr, Ci, Ar, Ai, Br, Bi, ld, rows_max, N, K, s);
     CUtensorMap tm[4];
     make_tmap_2d(&tm[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, Ar, K, M, ld, BK, ZM, CU_TENSOR_MAP_SWIZZLE_128B);
     make_tmap_2d(&tm[1], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, Ai, K, M, ld, BK, ZM, CU_TENSOR_MAP_SWIZZLE_128B);

@@ -174,3 +174,18 @@ def test_complex_singular_info_and_empty(pkg, oracle):
     assert F.info == info == 38
     E = pkg.lu(np.zeros((0, 0), dtype=np.complex128))
     assert E.shape == (0, 0) and E.issuccess()
+
+
+def test_complex_matrix_taller_than_a_grid_of_tiles(pkg):
+    """The trailing update of 65535 x 64 rows and more takes several launches."""
+    m, n = 65535 * 64 + 100, 4
+    g = torch.Generator(device="cuda").manual_seed(3)
+    A = torch.randn(n, m, dtype=torch.complex128, device="cuda", generator=g).t()  # column-major
+    F = pkg.lu(A, blocksize=2)
+    PA = A.clone()
+    for j, p in enumerate(F.ipiv.cpu().tolist()):
+        PA[[j, p - 1]] = PA[[p - 1, j]]
+    L = torch.tril(F.factors, -1)
+    L[range(n), range(n)] = 1.0
+    assert float((PA - L @ torch.triu(F.factors[:n])).abs().max()) <= 1e-13 * float(A.abs().max())
+    assert float(L.abs().max()) <= 1 + 1e-15
