@@ -1163,25 +1163,28 @@ __global__ void __launch_bounds__(256) k_trsm_fused(const T *__restrict__ L, i64
 }
 
 // The narrow FP32 solve (a panel's U12 in the mixed factor, on the panels'
-// critical path): 8 columns per CTA, the 32 x 32 diagonal blocks inverted
-// first, one warp each, so that a block row's solve is a product of all threads
-// instead of a 32-step chain of shuffles; each block column of L is requested
-// one block ahead.  Bound: latency of the block rows (three barriers and two
-// 32-step chains each).
-constexpr int TI_CW = 8;
-struct TrsmInvSmem {
+// critical path): 8 columns per CTA, all diagonal blocks in shared memory from the
+// start, each block column of L requested one block ahead; a block row's solve is
+// a substitution, a warp per column with its row of the block in registers.
+// Bound: latency of the block rows (a 31-step chain of shuffles, a 32-step one of
+// products, three barriers each).  By products with inverted diagonal blocks the
+// chain is shorter (the 125 solves of the n = 16384 mixed factor 7.4 ms instead of
+// 7.65), but the residual reached 258 roundings where substitution leaves 2
+// (restated in NumPy, fourth difference matrix of order 1024).
+constexpr int TN_CW = 8;
+struct TrsmNarrowSmem {
     float D[TF_TMAX / TF_TB][TF_TB][TF_TB + 1];
     float L[TF_TMAX - TF_TB][TF_TB + 1];
-    float X[TF_TMAX][TI_CW];
+    float X[TF_TMAX][TN_CW];
 };
-__global__ void __launch_bounds__(256) k_trsm_inv(const float *__restrict__ L, i64 ldl, float *__restrict__ B, i64 ldb,
+__global__ void __launch_bounds__(256) k_trsm_narrow(const float *__restrict__ L, i64 ldl, float *__restrict__ B, i64 ldb,
                                                   int t, i64 N) {
     extern __shared__ __align__(16) unsigned char tf_smem[];
-    TrsmInvSmem &S = *reinterpret_cast<TrsmInvSmem *>(tf_smem);
+    TrsmNarrowSmem &S = *reinterpret_cast<TrsmNarrowSmem *>(tf_smem);
     constexpr int PRE = (TF_TMAX - TF_TB) * TF_TB / 256;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const i64 c0 = (i64)blockIdx.x * TI_CW;
-    const int cols = (int)((N - c0) < TI_CW ? (N - c0) : TI_CW);
+    const i64 c0 = (i64)blockIdx.x * TN_CW;
+    const int cols = (int)((N - c0) < TN_CW ? (N - c0) : TN_CW);
     const int nblk = (t + TF_TB - 1) / TF_TB;
     float pre[PRE];
     auto fetch = [&](int J) {  // L below diagonal block J
@@ -1199,43 +1202,34 @@ __global__ void __launch_bounds__(256) k_trsm_inv(const float *__restrict__ L, i
 #pragma unroll
         for (int i = 0; i < TF_TB; ++i)
             D[i][lane] = (d0 + i < t && lane < i) ? L[(i64)(d0 + i) * ldl + d0 + lane] : 0.f;
-        __syncwarp();
-        float x[TF_TB];
-#pragma unroll
-        for (int i = 0; i < TF_TB; ++i) x[i] = i == lane ? 1.f : 0.f;
-#pragma unroll
-        for (int p = 0; p < TF_TB; ++p)
-#pragma unroll
-            for (int i = p + 1; i < TF_TB; ++i) x[i] = fmaf(-D[i][p], x[p], x[i]);
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < TF_TB; ++i) D[i][lane] = x[i];
     }
 #pragma unroll
-    for (int e = tid; e < TF_TMAX * TI_CW; e += 256) {
-        const int i = e / TI_CW, c = e % TI_CW;
+    for (int e = tid; e < TF_TMAX * TN_CW; e += 256) {
+        const int i = e / TN_CW, c = e % TN_CW;
         S.X[i][c] = (i < t && c < cols) ? B[(i64)i * ldb + c0 + c] : 0.f;
     }
-    const int pr = tid / TI_CW, pc = tid % TI_CW;
     for (int J = 0; J < nblk; ++J) {
         const int j0 = J * TF_TB, rem = t - j0 - TF_TB;  // rows below the block
 #pragma unroll
         for (int q = 0; q < PRE; ++q) S.L[warp + 8 * q][lane] = pre[q];
         __syncthreads();
         if (J + 1 < nblk) fetch(J + 1);
-        float y0 = 0.f, y1 = 0.f;
-#pragma unroll 8
-        for (int k = 0; k < TF_TB; k += 2) {
-            y0 = fmaf(S.D[J][pr][k], S.X[j0 + k][pc], y0);
-            y1 = fmaf(S.D[J][pr][k + 1], S.X[j0 + k + 1][pc], y1);
+        {
+            float x = S.X[j0 + lane][warp], d[TF_TB];
+#pragma unroll
+            for (int p = 0; p < TF_TB; ++p) d[p] = S.D[J][lane][p];
+#pragma unroll
+            for (int p = 0; p < TF_TB - 1; ++p) {
+                const float xp = __shfl_sync(0xffffffffu, x, p);
+                if (lane > p) x = fmaf(-d[p], xp, x);
+            }
+            S.X[j0 + lane][warp] = x;
         }
         __syncthreads();
-        S.X[j0 + pr][pc] = y0 + y1;
-        __syncthreads();
         if (tid < rem) {
-            float acc[TI_CW];
+            float acc[TN_CW];
 #pragma unroll
-            for (int c = 0; c < TI_CW; ++c) acc[c] = 0.f;
+            for (int c = 0; c < TN_CW; ++c) acc[c] = 0.f;
 #pragma unroll 8
             for (int k = 0; k < TF_TB; ++k) {
                 const float l = S.L[tid][k];
@@ -1250,13 +1244,13 @@ __global__ void __launch_bounds__(256) k_trsm_inv(const float *__restrict__ L, i
                 acc[7] = fmaf(l, b.w, acc[7]);
             }
 #pragma unroll
-            for (int c = 0; c < TI_CW; ++c) S.X[j0 + TF_TB + tid][c] -= acc[c];
+            for (int c = 0; c < TN_CW; ++c) S.X[j0 + TF_TB + tid][c] -= acc[c];
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int e = tid; e < TF_TMAX * TI_CW; e += 256) {
-        const int i = e / TI_CW, c = e % TI_CW;
+    for (int e = tid; e < TF_TMAX * TN_CW; e += 256) {
+        const int i = e / TN_CW, c = e % TN_CW;
         if (i < t && c < cols) B[(i64)i * ldb + c0 + c] = S.X[i][c];
     }
 }
@@ -1267,8 +1261,8 @@ void launch_trsm_fused(const T *L, i64 ldl, T *B, i64 ldb, int t, i64 N, cudaStr
     ProfScope ps(KC_TRSM_LEAF, s, (double)t * t * N, 2.0 * (double)t * N * sizeof(T));
     if constexpr (sizeof(T) == 4) {
         if (N <= 2048) {
-            set_max_dyn_smem((const void *)k_trsm_inv, (int)sizeof(TrsmInvSmem));
-            k_trsm_inv<<<(unsigned)((N + TI_CW - 1) / TI_CW), 256, sizeof(TrsmInvSmem), s>>>(L, ldl, B, ldb, t, N);
+            set_max_dyn_smem((const void *)k_trsm_narrow, (int)sizeof(TrsmNarrowSmem));
+            k_trsm_narrow<<<(unsigned)((N + TN_CW - 1) / TN_CW), 256, sizeof(TrsmNarrowSmem), s>>>(L, ldl, B, ldb, t, N);
             OXI_LAUNCH_CHECK();
             return;
         }

@@ -71,6 +71,25 @@ def test_gemm_tiles_same_bits(pkg, m, n, k):
     assert bool((err <= 2 * (k + 1) * EPS * (C[:m].abs() + A[:m].abs() @ B.abs())).all())
 
 
+@pytest.mark.parametrize("power", [2, 3])
+def test_float32_block_row_by_substitution(pkg, power):
+    """U12 of an FP32 panel whose triangle's 32 x 32 blocks are ill-conditioned, its
+    columns the products of L with random ones: |P A - L U| <= k u |L||U| with k
+    terms an element, which substitution keeps (a product with the blocks'
+    inverses left 2.3 and 2.9 times that)."""
+    rng = np.random.default_rng(power)
+    m, w = 600, 128
+    T = np.linalg.matrix_power(2 * np.eye(m) - np.eye(m, k=1) - np.eye(m, k=-1), power)[:, :w].astype(np.float32)
+    P, L, _ = sl.lu(T)
+    A = np.hstack([T, (P @ L @ rng.standard_normal((w, 64))).astype(np.float32)])
+    F = pkg.lu(torch.from_numpy(A), check=False)  # the rows below have nothing left to factor
+    LU, PA = _np(F.factors).astype(float), A[F.p].astype(float)
+    n = A.shape[1]
+    Lf, U = np.tril(LU, -1) + np.eye(m, n), np.triu(LU[:n])
+    k = np.minimum(np.arange(m)[:, None], np.arange(n)) + 1
+    assert (np.abs(PA - Lf @ U) <= (k + 1) * 2.0 ** -24 * (np.abs(Lf) @ np.abs(U))).all()
+
+
 def test_repeated_factorization_same_bits(pkg):
     """Both streams of the lookahead and all pipelines under load: every repetition
     gives the same factors."""
