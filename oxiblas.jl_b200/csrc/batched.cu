@@ -589,7 +589,9 @@ __device__ void lu_blocked(T *W, i64 ldw, int n, int nb, bool in_smem, T *sP, T 
 // starts at cols + c ldc.  The row block is a compile-time constant, so a step is
 // one shuffle and one product per row block still open.  Backward: the pivots'
 // reciprocals are taken beforehand, one per lane, and a quotient is the product
-// corrected by its exact remainder (a division where that is not finite).
+// corrected by its exact remainder (Markstein's quotient, see potrf.cu; of 2e8 FP64
+// and 4e8 FP32 random ones none differed from the division; a division where that
+// is not finite).
 template <typename T, int Q>
 __device__ __forceinline__ void forward_steps(const T *cols, int ldc, int j0, int j1, int n, T (&y)[bt::NQ], int lane) {
     using namespace bt;

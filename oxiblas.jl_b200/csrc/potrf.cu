@@ -46,9 +46,15 @@ constexpr int PO_LP = PO_NB + 4, PO_CP = PO_SB + 4;
 }  // namespace
 
 // d = sqrt(a), y = 1 / d and z, an approximation of 1 / d that is ready earlier,
-// for 2^-900 < a < 2^900: the approximate reciprocal root, one cubic Newton step
-// (z), and a fused correction of each result (the latency of one chain instead
-// of a square root followed by a division).
+// for 2^-900 < a < 2^900: the approximate reciprocal root y0, one step of the
+// binomial series of (1 - e)^(-1/2) with e = 1 - a y0^2 (z = y0 (1 + e / 2 + 3 e^2 / 8),
+// within an ulp), and each result corrected once by its fused remainder
+// (P. Markstein, Computation of elementary functions on the IBM RISC System/6000
+// processor, IBM J. Res. Dev. 34, 1990): the latency of one chain instead of a
+// square root followed by a division.  What is left before the last rounding is of
+// the order of 2^-103 of the result, so it is the rounded root (quotient) but where
+// the exact one lies that close to the middle of two numbers; test_kernel_edges_gpu.py
+// compares both with sqrt and the division bit for bit.
 __device__ __forceinline__ void root_recip(double a, double &d, double &y, double &z) {
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
     const double e = fma(-(a * y), y, 1.0);
@@ -68,8 +74,9 @@ __device__ __forceinline__ bool exp_all_ones(float a) { return (__float_as_uint(
 
 // Rows of an N x N diagonal block (upper, u) with one column x beside it:
 // u_cc = sqrt(u_cc), u_cj /= u_cc, x_c /= u_cc, then the rows below take the
-// products; sy, if not null, takes the reciprocals of the roots.  FAST has no branch: roots and quotients are products with the
-// reciprocal corrected by the remainder, and false is returned where a pivot or
+// products; sy, if not null, takes the reciprocals of the roots.  FAST has no
+// branch: roots and quotients are products with the reciprocal corrected by the
+// remainder (see root_recip), and false is returned where a pivot or
 // a result leaves the range in which that holds (the caller starts again without
 // FAST, which divides).  Returns true with bad = the first pivot that is not
 // finite and positive (N: none) otherwise.
@@ -640,8 +647,8 @@ template void potrf_rowmajor<float>(oxi_handle_s *, float *, i64, i64, int64_t *
 // ---------------------------------------------------------------------------
 // Solves with the factor: L y = b, then L^T x = y (the reference's two
 // triangular solves, src/lapack/factorizations.jl:293-305).  L is the caller's
-// column-major lower factor: the non-unit lower block-operator solve and its
-// transpose (solve.cu).
+// column-major lower factor: the superblock solve of a non-unit lower triangle and its
+// transpose (solve.cu, trsv.cu).
 // ---------------------------------------------------------------------------
 template <typename T>
 void potrs_colmajor(oxi_handle_s *h, i64 n, i64 nrhs, const T *L, i64 ldl, T *B, i64 ldb, int *d_err);

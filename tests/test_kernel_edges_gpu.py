@@ -187,6 +187,25 @@ def test_cholesky_blocks_and_first_failing_column(pkg, oracle, n):
         assert pkg.cholesky(M, check=False).info == oracle.potrf(M)[1] == bad + 1
 
 
+def test_cholesky_roots_and_quotients_are_the_rounded_ones(pkg):
+    """The diagonal block forms roots and quotients from an approximate reciprocal
+    root by fused corrections: the values of sqrt and of the division, over the
+    exponents where that form is taken.  (It could miss one in 2^50: a result
+    whose exact value lies within 2^-103 of the middle of two numbers.)"""
+    rng = np.random.default_rng(11)
+    for _ in range(10):
+        a = rng.uniform(1, 2, 1024) * 2.0 ** rng.integers(-899, 899, 1024)
+        assert np.array_equal(_np(pkg.cholesky(np.diag(a)).L).diagonal(), np.sqrt(a))
+    for _ in range(40):
+        a = rng.uniform(1, 4) * 2.0 ** rng.integers(-200, 200)
+        v = np.sqrt(a) * rng.uniform(-1, 1, 127) * 2.0 ** rng.integers(-60, 60, 127)
+        A = np.diag(np.concatenate([[a], 256 * (v / np.sqrt(a)) ** 2]))
+        A[0, 1:] = A[1:, 0] = v
+        # the other columns see u_0i u_0j of both signs and sizes: only the first row is exact
+        A[1:, 1:] += np.outer(v, v) / a
+        assert np.array_equal(_np(pkg.cholesky(A).L)[1:, 0], v / np.sqrt(a))
+
+
 @pytest.mark.parametrize("n", [8, 127, 300])
 def test_cholesky_pivots_out_of_the_fast_range(pkg, n):
     """Scaling by 2^-960 (exact) brings the pivots under 2^-900, where roots and

@@ -224,9 +224,9 @@ def test_lookahead_gives_identical_factors(pkg, oracle, dtype):
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 def test_many_rhs_solves_every_chunk_width(pkg, dtype):
-    """ldiv! with 23 right-hand sides runs the block-operator triangular solve
-    in chunks of 16 (FP32), 8, 4, 2 and 1 columns; n = 777 gives a partial last
-    64-row block and more blocks than the three the chain couples.  Each column
+    """ldiv! with 23 right-hand sides runs the superblock triangular solve
+    in chunks of 16 (FP32), 8, 4, 2 and 1 columns; n = 777 gives three full
+    superblocks of 256 rows and a last one of nine.  Each column
     must equal the one-column solve of the same factor (relative 1e-13 FP64,
     1e-5 FP32: the per-column arithmetic does not depend on the chunk width),
     and the whole solve must have a normwise backward error <= 30 n eps, for N
