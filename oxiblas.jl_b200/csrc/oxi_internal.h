@@ -351,7 +351,8 @@ void ensure_lookahead_streams(oxi_handle_s *h);
 template <typename T>
 void potrf_rowmajor(oxi_handle_s *h, T *U, i64 ld, i64 n, int64_t *d_info, T *work);
 // Triangular solves in superblocks (trsv.cu).  tri_inverses: the superblock
-// inverses of both triangles of a factor, tri_inverse_elems(n) elements each;
+// inverses of both triangles of a factor and the estimates of their quality,
+// tri_inverse_elems(n) elements each;
 // tri_solves: the two solves in the form's order, X (column-major n x nrhs) in
 // place.  *err is the call's abort block.
 enum class TriForm {
