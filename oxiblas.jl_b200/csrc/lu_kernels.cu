@@ -1268,18 +1268,19 @@ void launch_trsm_fused(const T *L, i64 ldl, T *B, i64 ldb, int t, i64 N, cudaStr
             return;
         }
     }
-    if (sizeof(T) == 8 && N <= 2048) {
-        constexpr int CW = 8;
-        const size_t smem = sizeof(T) * ((size_t)TF_TMAX * (CW + 1) + (size_t)TF_TMAX * (TF_TB + 1));
-        set_max_dyn_smem((const void *)k_trsm_fused<T, CW>, (int)smem);
-        k_trsm_fused<T, CW><<<(unsigned)((N + CW - 1) / CW), 256, smem, s>>>(L, ldl, B, ldb, t, N);
-    } else {
-        constexpr int CW = 32;
-        const size_t smem = sizeof(T) * ((size_t)TF_TMAX * (CW + 1) + (size_t)TF_TMAX * (TF_TB + 1));
-        set_max_dyn_smem((const void *)k_trsm_fused<T, CW>, (int)smem);
-        k_trsm_fused<T, CW><<<(unsigned)((N + CW - 1) / CW), 256, smem, s>>>(L, ldl, B, ldb, t, N);
+    auto go = [&](auto kern, int cw) {
+        const size_t smem = sizeof(T) * ((size_t)TF_TMAX * (cw + 1) + (size_t)TF_TMAX * (TF_TB + 1));
+        set_max_dyn_smem((const void *)kern, (int)smem);
+        kern<<<(unsigned)((N + cw - 1) / cw), 256, smem, s>>>(L, ldl, B, ldb, t, N);
+        OXI_LAUNCH_CHECK();
+    };
+    if constexpr (sizeof(T) == 8) {
+        if (N <= 2048) {
+            go(k_trsm_fused<T, 8>, 8);
+            return;
+        }
     }
-    OXI_LAUNCH_CHECK();
+    go(k_trsm_fused<T, 32>, 32);
 }
 // ---------------------------------------------------------------------------
 // Reference-order TRSM (FP64, t <= 128): B (t x N) <- L^-1 B for a unit lower
