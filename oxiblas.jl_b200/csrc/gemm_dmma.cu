@@ -247,9 +247,9 @@ void launch_gemm_dmma(double *C, i64 ldc, const double *A, i64 lda, const double
     ProfScope ps(KC_GEMM_DMMA, s, (upper_only ? 1.0 : 2.0) * M * N * K, 8.0 * (2.0 * M * N + M * K + K * N));
     // Small tiles while the large ones leave SMs without one: a tile's time is its
     // chain of products on one SM, whatever the other SMs do.  Large against small,
-    // us, by number of large tiles: 8 (960 x 64 x 64) 14.2, 10.3; 48 (3000 x 128 x
-    // 128) 19.4, 15.3; 96 (6144 x 128 x 128) 19.6, 18.4; 98 (896 x 896 x 128) 20.3,
-    // 17.8; 126 (8064 x 128 x 128) 19.2, 21.5; 148: 20.1, 23.1.
+    // us, by number of large tiles: 8 (960 x 64 x 64) 13.0, 10.1; 48 (3000 x 128 x
+    // 128) 18.7, 14.5; 96 (6144 x 128 x 128) 19.1, 18.5; 98 (896 x 896 x 128) 18.9,
+    // 18.7; 126 (8064 x 128 x 128) 19.7, 21.5; 148: 20.1, 23.1.
     const i64 large = ((M + 127) / 128) * ((N + 63) / 64);
     if (large <= DMMA_SMALL_MAX) launch_dmma_tile<64, 32>(C, ldc, A, lda, B, ldb, M, N, K, s, upper_only);
     else launch_dmma_tile<128, 64>(C, ldc, A, lda, B, ldb, M, N, K, s, upper_only);
